@@ -6,8 +6,8 @@
 //   hetrd    k_hetrd_warp (n <= 65) or k_hetrd: Householder tridiagonalisation of C,
 //            reflectors and (d, e, tau) into the workspace; the mixed form (n <= 56) runs it
 //            in complex64 (k_hetrd_warp_c64).
-//   eig      FP64, n <= 63 (and 85..128, launched from bigsolve.cu): k_ql_values (the
-//            implicit-QL recurrence, one thread per pair, eigenvalues only) and
+//   eig      FP64, n <= 63 (and 85..128, launched from bigsolve.cu): k_tridiag_values
+//            (tridiag.cu: bisection on Sturm counts, a thread per one or two eigenvalues) and
 //            k_tridiag_invit (eigenvectors by inverse iteration, one warp per pair).
 //            Otherwise k_ql_chain logs the recurrence's rotations and k_ql_apply /
 //            k_ql_apply_reg replay the log onto Z (W ascending).  The mixed form refines
@@ -785,31 +785,8 @@ __global__ void k_ql_apply_reg(int n, int batch, Workspace ws, double* __restric
     }
 }
 
-// ----------------------------------------------------------------------------- k_ql_values
-// The QL chain of k_ql_chain (one thread per pair) for the eigenvalues only: no rotation log,
-// no permutation; W ascending.  Feeds k_tridiag_invit.
-__global__ void k_ql_values(int n, int batch, Workspace ws, double* __restrict__ W, int* __restrict__ info) {
-    const int tid = threadIdx.x, T = blockDim.x;
-    const int b = blockIdx.x * T + tid;
-    extern __shared__ __align__(16) unsigned char smem[];
-    double* d = reinterpret_cast<double*>(smem) + tid;
-    double* e = reinterpret_cast<double*>(smem) + static_cast<size_t>(n) * T + tid;
-    if (b >= batch || !pair_selected(ws, b)) return;
-    double* Wb = W + static_cast<size_t>(n) * b;
-    if (info[b] != 0) {
-        for (int i = 0; i < n; ++i) Wb[i] = __longlong_as_double(0x7ff8000000000000ll);
-        return;
-    }
-    for (int i = 0; i < n; ++i) {
-        d[i * T] = ws.d[static_cast<size_t>(n) * b + i];
-        e[i * T] = ws.e[static_cast<size_t>(n) * b + i];
-    }
-    const int r = ql_chain<double, false>(n, d, e, T, nullptr, 0, nullptr, Wb);
-    if (r > 0) info[b] = r;
-}
-
 // ----------------------------------------------------------------------------- k_tridiag_invit
-// Eigenvectors of the tridiagonal T (d, e) from its FP64 eigenvalues (k_ql_values) by inverse
+// Eigenvectors of the tridiagonal T (d, e) from its FP64 eigenvalues (k_tridiag_values) by inverse
 // iteration, one warp per pair, one lane per eigenvector at a time (LAPACK dstein's method):
 // T - lambda_j I = L U without pivoting, a pivot below eps ||T|| replaced by that size, two
 // solves from a fixed pseudo-random start, each followed by normalisation.  That is O(n) work
@@ -819,7 +796,7 @@ __global__ void k_ql_values(int n, int batch, Workspace ws, double* __restrict__
 // (modified Gram-Schmidt); the other vectors' orthogonality is ~eps ||T|| / gap.  Every
 // vector must pass ||T z - lambda z|| <= kInvitTol ||T||; a pair with a failed vector, a
 // cluster of more than kInvitMaxCluster eigenvalues (a spectrum dominated by one huge
-// eigenvalue), or a QL chain that did not converge is recomputed by the warp QL instead.
+// eigenvalue), or a T that is not finite is recomputed by the warp QL instead.
 // Per-lane scratch (1/u and the vector) is interleaved [i * 33 + lane]: lane-parallel
 // recurrences read consecutive words, and the warp's column-by-column copy to the caller's X
 // buffer (Z, column k = vector k) reads it across lanes without bank conflicts.
@@ -1405,14 +1382,12 @@ cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, d
                              int chain_threads, bool flag_redo, cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (!W || !X || !info || !ws.d || !ws.e || !ws.flag) return cudaErrorInvalidValue;
-    const size_t vs = ql_chain_smem_bytes(n, chain_threads, false);
     const size_t is = InvitSmem(n, !flag_redo).per_warp;
-    if (vs > static_cast<size_t>(max_smem_optin()) || is > static_cast<size_t>(max_smem_optin()))
-        return cudaErrorInvalidValue;
-    static SmemOptIn fv, fi;
-    set_max_smem_once(k_ql_values, fv);
+    if (is > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
+    static SmemOptIn fi;
     set_max_smem_once(k_tridiag_invit, fi);
-    k_ql_values<<<(batch + chain_threads - 1) / chain_threads, chain_threads, vs, stream>>>(n, batch, ws, W, info);
+    const cudaError_t err = launch_tridiag_values(n, batch, ws, W, info, stream);
+    if (err != cudaSuccess) return err;
     k_tridiag_invit<<<batch, 32, is, stream>>>(n, batch, ws, W, X, info, flag_redo ? 1 : 0);
     return cudaGetLastError();
 }

@@ -254,7 +254,7 @@ cudaError_t launch_ql_chain(int n, int batch, const Workspace& ws, double* W, in
 // and the Householder kernel; one kernel otherwise.
 inline int reduce_kernel_count(int n, bool tc = false) { return n <= 56 || (n > kSmallMaxN && tc) ? 2 : 1; }
 // (57 <= n <= 84 with tc: k_reduce_tc alone, the Householder being its own stage there.)
-// FP64 eigenvectors by inverse iteration (k_ql_values + k_tridiag_invit) for n <= kInvitMaxN, with
+// FP64 eigenvectors by inverse iteration (k_tridiag_values + k_tridiag_invit) for n <= kInvitMaxN, with
 // the warp QL inside the kernel for pairs it cannot take, and for kSmallMaxN < n <= kInvitBigMaxN,
 // where such pairs are flagged and the rotation-log QL (k_ql_chain + k_ql_apply_rows) redone for
 // them only; the rotation-log QL for every other n and for the mixed form.
@@ -265,11 +265,14 @@ inline bool eig_by_inverse_iteration(int n, bool single) {
 }
 // Kernels one eigensolve stage launches for order n.
 inline int eig_kernel_count(int n, bool single) {
-    if (single) return 5;          // k_ql_values, k_tridiag_invit, Q-apply, refinement, fallback
+    if (single) return 5;          // k_tridiag_values, k_tridiag_invit, Q-apply, refinement, fallback
     if (n <= kInvitMaxN) return 2;
     return n > kSmallMaxN && n <= kInvitBigMaxN ? 4 : 2;
 }
-// Eigenvalues (k_ql_values) and inverse-iteration eigenvectors (k_tridiag_invit) of every pair;
+// Eigenvalues of every pair's tridiagonal (d, e) by bisection (csrc/tridiag.cu), ascending; NaN for
+// pairs with info != 0.  Honours the pair selection.
+cudaError_t launch_tridiag_values(int n, int batch, const Workspace& ws, double* W, int* info, cudaStream_t stream);
+// Eigenvalues (k_tridiag_values) and inverse-iteration eigenvectors (k_tridiag_invit) of every pair;
 // flag_redo: pairs it cannot take get ws.flag = 2 (and no output) instead of the in-kernel QL.
 cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                              int chain_threads, bool flag_redo, cudaStream_t stream);

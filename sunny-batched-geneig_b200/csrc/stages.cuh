@@ -172,13 +172,24 @@ __device__ void hetrd_lower(cplx<R>* A, int lda, int n, R* d, R* e, cplx<R>* tau
 }
 
 // ============================================================================ tridiagonal QL
+// The power of two that scales a T of max-norm anorm to [1/2, 1) (exactly: a diagonal T keeps its
+// entries); 1 for a zero or non-finite norm.  Kept within the normal range, as is its reciprocal.
+template <typename R>
+__device__ __forceinline__ R pow2_norm(R anorm) {
+    if (!(anorm > R(0)) || !isfinite(anorm)) return R(1);
+    int ex;
+    frexp(anorm, &ex);
+    constexpr int kMost = sizeof(R) == 8 ? 1022 : 126;
+    return scalbn(R(1), min(max(ex, -kMost), kMost));
+}
+
 // Eigen-decomposition of the real symmetric tridiagonal (d, e) by implicit QL
 // with Wilkinson-type shifts, accumulating the rotations into Z (row-major,
 // Z[r * ldz + c], initialised to I by the caller).  One warp per problem: every
 // lane runs the same scalar recurrence (so no broadcast is needed) and applies
 // each rotation to the rows it owns (r = lane + 32 q).  The deflation test is
 // LAPACK dsteqr's relative one, |e_m|^2 <= eps^2 |d_m| |d_{m+1}| + safmin, and the
-// matrix is scaled to unit max-norm first (dsteqr scales only at the range
+// matrix is scaled by a power of two to max-norm in [1/2, 1) first (dsteqr scales only at the range
 // limits; scaling always keeps the single-precision variant safe).
 // Eigenvalues come back ascending with Z's columns permuted alike (dsteqr's
 // final selection sort).  Returns the number of off-diagonals that failed to
@@ -190,11 +201,11 @@ __device__ int tridiag_ql(int n, R* d, R* e, R* Z, int ldz) {
     const R eps = sizeof(R) == 8 ? R(1.1102230246251565e-16) : R(5.9604645e-08);
     const R eps2 = eps * eps;
     const R safmin = sizeof(R) == 8 ? R(2.2250738585072014e-308) : R(1.17549435e-38);
-    // scale to unit max-norm
+    // scale to max-norm in [1/2, 1)
     R anorm = R(0);
     for (int i = 0; i < n; ++i) anorm = fmax(anorm, fabs(d[i]));
     for (int i = 0; i + 1 < n; ++i) anorm = fmax(anorm, fabs(e[i]));
-    if (!(anorm > R(0)) || !isfinite(anorm)) anorm = R(1);
+    anorm = pow2_norm(anorm);
     const R sc = R(1) / anorm;
     __syncwarp();
     if (lane == 0) {
@@ -303,7 +314,7 @@ __device__ int ql_chain(int n, R* d, R* e, int stride, cplx<R>* log, int cap, in
     R anorm = R(0);
     for (int i = 0; i < n; ++i) anorm = fmax(anorm, fabs(D(i)));
     for (int i = 0; i + 1 < n; ++i) anorm = fmax(anorm, fabs(E(i)));
-    if (!(anorm > R(0)) || !isfinite(anorm)) anorm = R(1);
+    anorm = pow2_norm(anorm);
     const R sc = R(1) / anorm;
     for (int i = 0; i < n; ++i) D(i) *= sc;
     for (int i = 0; i + 1 < n; ++i) E(i) *= sc;
