@@ -1307,9 +1307,11 @@ cudaError_t launch_reduce_big(const double2* A, const double2* B, int n, int bat
     if (batch <= 0) return cudaSuccess;
     if (!A || !B || !X || !info || !ws.LV || !ws.d || !ws.e || !ws.tau) return cudaErrorInvalidValue;
     if (!big_path(n) || mode < kBigFull || mode > kBigHetrdOnly) return cudaErrorInvalidValue;
-    // the Householder alone: one CTA per pair, one pass over the L2-resident packed triangle per step
-    // (k_hetrd_l2), measured faster than both the shared-memory tile of k_reduce_mid (1.04x at
-    // n = 96, 1.3x at n = 128 and 160, whole reduce stage) and the 8-CTA cluster (4.7x at n = 192)
+    // the Householder alone: up to kHetrdRegMaxN with the matrix on the SM (k_hetrd_reg, 2.4x the
+    // L2-resident walk at n = 96, 2.1x at n = 128), above it one CTA per pair, one pass over the
+    // L2-resident packed triangle per step (k_hetrd_l2), measured faster than both the shared-memory
+    // tile of k_reduce_mid (1.3x at n = 160, whole reduce stage) and the 8-CTA cluster (4.7x at n = 192)
+    if (mode == kBigHetrdOnly && n <= kHetrdRegMaxN) return launch_hetrd_reg(n, batch, X, ws, info, stream);
     if (mode == kBigHetrdOnly) return launch_hetrd_l2(n, batch, X, ws, info, stream);
     if (n <= kMidMaxN) {                     // one CTA per pair: no cluster barriers
         if (n <= 96) run_reduce_mid<12>(A, B, n, batch, ws, X, info, stream, mode);
@@ -1340,7 +1342,7 @@ cudaError_t launch_hetrd_c64_big(int n, int batch, const double2* C, const Works
 cudaError_t launch_hetrd_l2(int n, int batch, const double2* C, const Workspace& ws, int* info,
                            cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
-    if (n <= kSmallMaxN || n > kBigMaxN || !C || !info || !ws.LV || !ws.d || !ws.e || !ws.tau || !ws.log)
+    if (n <= kHetrdRegMaxN || n > kBigMaxN || !C || !info || !ws.LV || !ws.d || !ws.e || !ws.tau || !ws.log)
         return cudaErrorInvalidValue;
     if (static_cast<size_t>(ws.log_stride) < static_cast<size_t>(n) * (n + 1) / 2) return cudaErrorInvalidValue;
     const size_t smem = L2HetrdSmem(n).total;
@@ -1356,7 +1358,7 @@ size_t ql_rows_smem_bytes(int n, bool single) { return single ? ql_rows_bytes<fl
 size_t big_stage_smem_bytes(int n, bool tc, int chain_threads) {
     size_t m = std::max(ql_rows_smem_bytes(n, false), ql_chain_smem_bytes(n, chain_threads, false));
     if (eig_by_inverse_iteration(n, false)) m = std::max(m, invit_smem_bytes(n, false));
-    if (tc) return std::max(m, L2HetrdSmem(n).total);       // k_reduce_tc / k_back_*_tc: static only
+    if (tc) return std::max(m, n <= kHetrdRegMaxN ? hetrd_reg_smem_bytes(n) : L2HetrdSmem(n).total);       // k_reduce_tc / k_back_*_tc: static only
     return std::max(m, std::max(big_reduce_smem_bytes(n), BigBackSmem(n).total));
 }
 

@@ -45,7 +45,7 @@ int supported_max_n(int precision) {
             continue;
         }
         size_t need = std::max(sbg::reduce_smem_bytes(sbg::kReduceFull, n), sbg::back_smem_bytes(n));
-        need = std::max(need, sbg::hetrd_smem_bytes(n, 128));
+        need = std::max(need, sbg::hetrd_reg_smem_bytes(n));
         need = std::max(need, sbg::ql_apply_smem_bytes(n, 1, false));
         need = std::max(need, sbg::ql_chain_smem_bytes(n, 32, false));
         if (big_mixed) {
@@ -403,7 +403,7 @@ void geneig_reduce_eig_n54_launch(const cuDoubleComplex* d_H, const cuDoubleComp
         sbg::Workspace ws = s->workspace(0, 1, stream);
         check_cuda(sbg::launch_reduce(sbg::kReduceFull, c2(d_H), c2(d_S), 54, 1, ws, c2(d_V), d_info,
                                       s->sched.shape(), stream), "reduce kernel");
-        check_cuda(sbg::launch_hetrd(54, 1, c2(d_V), ws, d_info, s->sched.shape(), stream), "hetrd kernel");
+        check_cuda(sbg::launch_hetrd(54, 1, c2(d_V), ws, d_info, stream), "hetrd kernel");
         check_cuda(sbg::launch_ql_logged(54, 1, ws, d_W, c2(d_V), d_info, false, s->sched.chain_threads,
                                          s->sched.ql_warps, stream), "QL kernels");
         check_cuda(sbg::launch_back(sbg::kBackQOnly, 54, 1, ws, c2(d_V), d_info, s->sched.shape(), stream),
@@ -439,7 +439,7 @@ void geneig_finish_n54_launch(const cuDoubleComplex* d_L, const cuDoubleComplex*
             const int cnt = std::min(ws.capacity, batch_size - off);
             check_cuda(sbg::launch_reduce(sbg::kReduceFromLM, nullptr, c2(d_L) + nn * off, 54, cnt, ws,
                                           nullptr, d_info + off, s->sched.shape(), stream), "reduce kernel");
-            check_cuda(sbg::launch_hetrd(54, cnt, c2(d_M) + nn * off, ws, d_info + off, s->sched.shape(), stream),
+            check_cuda(sbg::launch_hetrd(54, cnt, c2(d_M) + nn * off, ws, d_info + off, stream),
                        "hetrd kernel");
             check_cuda(sbg::launch_ql_logged(54, cnt, ws, d_W + 54 * off, c2(d_U) + nn * off, d_info + off, false,
                                              s->sched.chain_threads, s->sched.ql_warps, stream), "QL kernels");

@@ -1,0 +1,367 @@
+// Householder tridiagonalisation with the matrix in REGISTERS and shared memory (k_hetrd_reg), NW
+// warps per pair, for n <= kHetrdRegMaxN.
+//
+// zhetd2's steps (LAPACK's reflectors, p = tau A v, w = p - tau/2 (p^H v) v, A -= v w^H + w v^H) on
+// the full Hermitian matrix: warp w holds the columns j = w (mod NW), lane l of it the rows
+// l, l + RS, .. (RS = ceil(n / R) <= 32).  The warp's last NS columns, which live longest, stay in
+// its registers (R x NS complex entries a thread); the earlier ones are in shared memory, each lane
+// reading and writing its own rows.  Keeping both triangles costs 12 m^2 FMAs a step instead of 8, but every row sum
+// of the matvec is then a sum over a thread's own registers and NW partials: no column walk, no
+// reduction per column, and the only operands read are the vectors' entries v_j, w_j of the warp's
+// column -- one address for the whole warp (a broadcast, half the cost of a 16-byte load with
+// distinct addresses), used for R rows.
+//
+// One pass per step: step k - 1's update is applied to each live column just before the column's
+// part of the matvec with v_k; column k alone is updated ahead, for the reflector formed from it.
+//
+// The kernels it replaces walked the packed triangle in shared memory (a warp per pair, each lane
+// its own row: 47 K shared-memory wavefronts per pair at n = 54, 62 % of the load/store unit's rate),
+// a full tile in shared memory by 256 threads (66 <= n <= 84), or the triangle in L2 (n > 84).
+// Microseconds per 1,000 pairs before -> now: n = 24 48 -> 21, 32 80 -> 34, 47 191 -> 139, 54 284 -> 166,
+// 72 1,197 -> 471, 96 2,013 -> 838, 128 4,600 -> 2,240.  It is bound by the latency of a step's chain
+// (column sum, norm, square root, reflector) at the few pairs an SM holds: FP64 pipe 34 % busy, a
+// third of the stalls LDS and shuffle results, a quarter the wait for the warp that forms the reflector.
+#include "kernels.cuh"
+#include "stages.cuh"
+
+#include <type_traits>
+
+namespace sbg {
+
+namespace {
+
+// Shared memory: v of this step and the next, w per warp, the matvec's partial row sums and v^H A v
+// per warp, (tau, beta) of two steps, and the columns of the first `off` slots.  The vectors have rv + 1 rows:
+// every thread's rows and every slot's column, and one spare row for the lanes that hold no row; a
+// column has rn + 1.
+template <int R, int NW>
+struct RegHetrdSmem {
+    int rs, rn, rv, off;
+    size_t v, w, part, spart, tau, cols, total;
+    __host__ __device__ RegHetrdSmem(int n, int ns) {
+        const int slots = (n + NW - 1) / NW;
+        rs = (n + R - 1) / R;
+        rn = R * rs;
+        off = slots > ns ? slots - ns : 0;
+        rv = NW * (off + ns) > rn ? NW * (off + ns) : rn;
+        const size_t row = 16 * static_cast<size_t>(rv + 1);
+        size_t o = 0;
+        v = o;     o += 2 * row;
+        w = o;     o += NW * row;
+        part = o;  o += NW > 1 ? NW * row : 0;
+        spart = o; o += 8 * ((NW + 1) & ~1);
+        tau = o;   o += 16 * 4;
+        cols = o;  o += 16 * static_cast<size_t>(off) * NW * (rn + 1);
+        total = o;
+    }
+};
+
+constexpr int kBlock = 2;                    // columns between two tests for live ones
+
+template <int NW>
+__device__ __forceinline__ void pair_sync() {
+    if constexpr (NW == 1) __syncwarp(); else __syncthreads();
+}
+
+// The reflector that zeroes column c below row c + 1, formed by the warp that holds the column
+// (x[s]: its entry of row s RS + lane, zero outside the matrix; la: the lane of row c + 1): v into
+// vnext at the thread's rows (at[s]; zero up to row c), tau and beta into stau[0..1], d[c] to dg.
+template <int R>
+__device__ __forceinline__ void form_reflector(int c, int RS, int la, const double2 (&x)[R], const int (&at)[R],
+                                               double2* vnext, double2* stau, double* dg) {
+    const int lane = threadIdx.x & 31;
+    const bool in = lane < RS;
+    double2 alpha = make_double2(0.0, 0.0);
+    double s2 = 0.0;
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+        const int r = s * RS + lane;
+        const double t = fma(x[s].x, x[s].x, x[s].y * x[s].y);
+        s2 += r > c + 1 && in ? t : 0.0;
+        if (r == c + 1) alpha = x[s];                             // (lanes >= RS hold row r + .. of no slot: not read)
+    }
+    alpha = cshfl(alpha, la);
+    s2 = warp_sum(s2);
+    // beta = -sign(Re alpha) ||(alpha, x)||, tau = (beta - alpha) / beta, scale = 1 / (alpha - beta);
+    // H = I for a zero tail and a real alpha.  The norm is n2 rsqrt(n2) after one Newton step.
+    const bool id = s2 == 0.0 && alpha.y == 0.0;
+    const double n2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, s2));
+    const double rn = rsqrt(n2);
+    double nrm = n2 * rn;
+    nrm = fma(fma(-nrm, nrm, n2), 0.5 * rn, nrm);
+    const double beta = alpha.x >= 0.0 ? -nrm : nrm, ib = alpha.x >= 0.0 ? -rn : rn;
+    const double ar = alpha.x - beta, ai = alpha.y;
+    const double rd = recip_nr(fma(ar, ar, ai * ai));
+    const double2 scale = id ? make_double2(0.0, 0.0) : make_double2(ar * rd, -ai * rd);
+    const double2 tk = id ? make_double2(0.0, 0.0) : make_double2((beta - alpha.x) * ib, -alpha.y * ib);
+    double2 v[R];
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+        const int r = s * RS + lane;
+        v[s] = cmul(x[s], scale);
+        if (r <= c + 1 || !in) v[s] = make_double2(r == c + 1 && in ? 1.0 : 0.0, 0.0);
+        vnext[at[s]] = v[s];
+    }
+    if (lane == 0) { stau[0] = tk; stau[1] = make_double2(id ? alpha.x : beta, 0.0); }
+#pragma unroll
+    for (int s = 0; s < R; ++s)
+        if (in && s * RS + lane == c) dg[c] = x[s].x;
+}
+
+// One case per column slot: a sweep over the live slots q0 .. NS - 1 jumps into the sequence once
+// and falls through.  The columns of slot q0 that are dead already meet v = w = 0.
+#define SBG_ASC16(C) C(0) C(1) C(2) C(3) C(4) C(5) C(6) C(7) C(8) C(9) C(10) C(11) C(12) C(13) C(14) C(15)
+#define SBG_ASC32(C) C(0) C(1) C(2) C(3) C(4) C(5) C(6) C(7) C(8) C(9) C(10) C(11) C(12) C(13) C(14) C(15) \
+    C(16) C(17) C(18) C(19) C(20) C(21) C(22) C(23) C(24) C(25) C(26) C(27) C(28) C(29) C(30) C(31)
+
+template <int R, int NW, int NS, int MINB>
+__global__ void __launch_bounds__(32 * NW, MINB) k_hetrd_reg(int n, int batch, const double2* __restrict__ C,
+                                                             Workspace ws, const int* __restrict__ info) {
+    const int b = blockIdx.x;
+    if (b >= batch || !pair_selected(ws, b)) return;
+    if (info[b] != 0) return;                                     // uniform
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const RegHetrdSmem<R, NW> lay(n, NS);
+    const int RS = lay.rs, RV = lay.rv, CR = lay.rn + 1, off = lay.off;
+    double2* vbuf = reinterpret_cast<double2*>(smem + lay.v);
+    double2* wb = reinterpret_cast<double2*>(smem + lay.w) + warp * (RV + 1);
+    double2* part = reinterpret_cast<double2*>(smem + lay.part);
+    double* spart = reinterpret_cast<double*>(smem + lay.spart);
+    double2* stau = reinterpret_cast<double2*>(smem + lay.tau);
+    double2* cols = reinterpret_cast<double2*>(smem + lay.cols) + warp * CR;       // slot q's column: + q NW CR
+    const size_t mat = static_cast<size_t>(n) * n;
+    const double2* Cb = C + mat * b;
+    double* dg = ws.d + static_cast<size_t>(n) * b;
+    double* eg = ws.e + static_cast<size_t>(n) * b;
+    double2* taug = ws.tau + static_cast<size_t>(n) * b;
+    double2* LVg = ws.LV + mat * b;
+    const bool lv_cols = n > kSmallMaxN;
+    const double2 zero = make_double2(0.0, 0.0);
+    const bool in = lane < RS;
+    // where the thread's rows are in the vectors and columns; lanes without a row use the spare row (zero)
+    int at[R], ac[R];
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+        at[s] = in ? s * RS + lane : RV;
+        ac[s] = in ? s * RS + lane : CR - 1;
+    }
+
+    // C's lower triangle, mirrored
+    auto entry = [&](int r, int j) {
+        double2 z = zero;
+        if (r < n && j < n) {
+            z = r >= j ? Cb[r + static_cast<size_t>(j) * n] : Cb[j + static_cast<size_t>(r) * n];
+            if (r < j) z.y = -z.y;
+            if (r == j) z.y = 0.0;
+        }
+        return z;
+    };
+#pragma unroll 4
+    for (int q = 0; q < off; ++q)
+#pragma unroll
+        for (int s = 0; s < R; ++s)
+            cols[q * NW * CR + ac[s]] = entry(in ? s * RS + lane : n, q * NW + warp);
+    double2 a[R][NS];
+#pragma unroll
+    for (int q = 0; q < NS; ++q)
+#pragma unroll
+        for (int s = 0; s < R; ++s) a[s][q] = entry(in ? s * RS + lane : n, (off + q) * NW + warp);
+    for (int i = threadIdx.x; i < 2 * (RV + 1); i += 32 * NW) vbuf[i] = zero;    // rows n .. RV stay zero
+    for (int i = lane; i <= RV; i += 32) wb[i] = zero;
+    pair_sync<NW>();
+    if (warp == 0) {
+        double2 x[R];
+#pragma unroll
+        for (int s = 0; s < R; ++s) x[s] = off > 0 ? cols[ac[s]] : a[s][0];
+        form_reflector<R>(0, RS, RS > 1 ? 1 : 0, x, at, vbuf, stau, dg);
+    }
+    pair_sync<NW>();
+
+    double2 vr[R], wr[R];                                         // v, w of the pending update: the thread's rows
+#pragma unroll
+    for (int s = 0; s < R; ++s) vr[s] = wr[s] = zero;
+    // rows below s0 RS are done from step s0 RS - 1 on: a phase per number of live row slots
+    auto phase = [&](auto first, int k0, int k1) {
+        constexpr int S0 = decltype(first)::value;
+        for (int k = k0; k < k1; ++k) {
+            const double2* v = vbuf + (k & 1) * (RV + 1);
+            const double2* vp = vbuf + ((k + 1) & 1) * (RV + 1);
+            const double2 tk = stau[2 * (k & 1)];
+            const int q0 = (k + 1) / NW, q0r = q0 - off;          // the first live column's slot, register slot
+            // ---- one pass over the live columns: step k - 1's update, then the warp's share of A v
+            double2 acc[R], am[R];                                // the two products of each part apart:
+#pragma unroll
+            for (int s = S0; s < R; ++s) acc[s] = am[s] = zero;   // half as long a dependent chain
+#pragma unroll 2
+            for (int q = q0; q < off; ++q) {
+                const int j = q * NW + warp;
+                const double2 pj = vp[j], wj = wb[j], vj = v[j];
+#pragma unroll
+                for (int s = S0; s < R; ++s) {
+                    double2* c = cols + q * NW * CR + ac[s];
+                    const double2 t = cfmsc(wr[s], pj, cfmsc(vr[s], wj, *c));
+                    *c = t;
+                    acc[s].x = fma(t.x, vj.x, acc[s].x);
+                    acc[s].y = fma(t.x, vj.y, acc[s].y);
+                    am[s].x = fma(t.y, vj.y, am[s].x);
+                    am[s].y = fma(t.y, vj.x, am[s].y);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < NS; q += kBlock) {
+                if (q0r < q + kBlock) {                           // uniform
+                    double2 vj[kBlock], wj[kBlock], pj[kBlock];
+#pragma unroll
+                    for (int u = 0; u < kBlock; ++u)
+                        if (q + u < NS) {
+                            pj[u] = vp[(off + q + u) * NW + warp];
+                            wj[u] = wb[(off + q + u) * NW + warp];
+                            vj[u] = v[(off + q + u) * NW + warp];
+                        }
+#pragma unroll
+                    for (int u = 0; u < kBlock; ++u)
+                        if (q + u < NS) {
+#pragma unroll
+                            for (int s = S0; s < R; ++s) {
+                                const double2 t = cfmsc(wr[s], pj[u], cfmsc(vr[s], wj[u], a[s][q + u]));
+                                a[s][q + u] = t;
+                                acc[s].x = fma(t.x, vj[u].x, acc[s].x);
+                                acc[s].y = fma(t.x, vj[u].y, acc[s].y);
+                                am[s].x = fma(t.y, vj[u].y, am[s].x);
+                                am[s].y = fma(t.y, vj[u].x, am[s].y);
+                            }
+                        }
+                }
+            }
+#pragma unroll
+            for (int s = S0; s < R; ++s) {
+                acc[s].x -= am[s].x;
+                acc[s].y += am[s].y;
+                vr[s] = v[at[s]];
+            }
+            // ---- v^H A v (real) and the row sums over the warps
+            double vav = 0.0;
+#pragma unroll
+            for (int s = S0; s < R; ++s) vav = fma(vr[s].x, acc[s].x, fma(vr[s].y, acc[s].y, vav));
+            if constexpr (NW > 1) {
+#pragma unroll
+                for (int s = S0; s < R; ++s) part[warp * (RV + 1) + at[s]] = acc[s];
+                vav = warp_sum(vav);
+                if (lane == 0) spart[warp] = vav;
+                __syncthreads();
+                double2 pt[R][NW];
+#pragma unroll
+                for (int s = S0; s < R; ++s)
+#pragma unroll
+                    for (int u = 0; u < NW; ++u) pt[s][u] = part[u * (RV + 1) + at[s]];
+                vav = 0.0;
+#pragma unroll
+                for (int u = 0; u < NW; ++u) vav += spart[u];
+#pragma unroll
+                for (int s = S0; s < R; ++s) {
+#pragma unroll
+                    for (int u = 1; u < NW; ++u) pt[s][0] = cadd(pt[s][0], pt[s][u]);
+                    acc[s] = pt[s][0];
+                }
+            } else {
+                vav = warp_sum(vav);
+            }
+            // ---- w = p + a2 v, p = tau A v, a2 = -tau/2 (p^H v) = -|tau|^2 / 2 (v^H A v); every warp all rows
+            const double a2 = -0.5 * cabs2(tk) * vav;
+#pragma unroll
+            for (int s = S0; s < R; ++s) {
+                const double2 p = cmul(tk, acc[s]);
+                const bool live = in && s * RS + lane > k;
+                wr[s] = live ? make_double2(fma(a2, vr[s].x, p.x), fma(a2, vr[s].y, p.y)) : zero;
+                wb[at[s]] = wr[s];
+            }
+            __syncwarp();
+            // ---- column k + 1 (slot q0) takes the update at once and gives the next reflector
+            if (k + 1 - q0 * NW == warp) {
+                double2 x[R];
+#pragma unroll
+                for (int s = 0; s < R; ++s) x[s] = zero;
+#define SBG_S(I) case I: if constexpr ((I) < NS) { _Pragma("unroll") for (int s = S0; s < R; ++s) x[s] = a[s][I]; } break;
+                if (q0r < 0) {
+#pragma unroll
+                    for (int s = S0; s < R; ++s) x[s] = cols[q0 * NW * CR + ac[s]];
+                } else {
+                    switch (q0r) { SBG_ASC32(SBG_S) default: break; }
+                }
+#undef SBG_S
+                const double2 vj = v[k + 1], wj = wb[k + 1];
+#pragma unroll
+                for (int s = S0; s < R; ++s) x[s] = cfmsc(wr[s], vj, cfmsc(vr[s], wj, x[s]));
+                const int la = k + 2 - S0 * RS == RS ? 0 : k + 2 - S0 * RS;       // the lane of row k + 2
+                form_reflector<R>(k + 1, RS, la, x, at, vbuf + ((k + 1) & 1) * (RV + 1), stau + 2 * ((k + 1) & 1), dg);
+            }
+            if (NW == 1 || k + 2 - (k + 2) / NW * NW == warp) {   // meanwhile another warp stores reflector k
+#pragma unroll
+                for (int s = S0; s < R; ++s) {
+                    const int r = s * RS + lane;
+                    if (in && r > k && r < n) {
+                        if (lv_cols) LVg[(r - k - 1) + static_cast<size_t>(n - 1 - k) * n] = vr[s];
+                        else LVg[k + static_cast<size_t>(r) * n] = vr[s];
+                    }
+                }
+                if (lane == 0) { taug[k] = tk; eg[k] = stau[2 * (k & 1) + 1].x; }
+            }
+            pair_sync<NW>();
+        }
+    };
+    auto from = [&](int s) { return s == 0 ? 0 : s == R ? n - 1 : min(n - 1, s * RS - 1); };
+    phase(std::integral_constant<int, 0>{}, from(0), from(1));
+    if constexpr (R > 1) phase(std::integral_constant<int, 1>{}, from(1), from(2));
+    if constexpr (R > 2) phase(std::integral_constant<int, 2>{}, from(2), from(3));
+    if constexpr (R > 3) phase(std::integral_constant<int, 3>{}, from(3), from(4));
+    if constexpr (R > 4) phase(std::integral_constant<int, 4>{}, from(4), from(5));
+    if (threadIdx.x == 0) { eg[n - 1] = 0.0; taug[n - 1] = zero; }
+}
+
+// (rows per lane, warps per pair, column slots in registers, pairs per SM) by n.  Measured over the
+// neighbouring shapes, microseconds per 1,000 pairs: few warps and many pairs per SM win (at n = 54
+// 1 warp 198, 2 warps 166, 3 warps 185, 4 warps 227, 8 warps 327) until a pair's columns no longer fit beside
+// others in shared memory; fewer register slots than these make the shared-memory part the bound.
+#define SBG_HETRD_REG_BY_N(n, F)                                                       \
+    do {                                                                               \
+        if ((n) <= 24) F(1, 1, 8, 24);                                                 \
+        if ((n) <= 32) F(1, 1, 16, 16);                                                \
+        if ((n) <= 40) F(2, 1, 10, 10);                                                \
+        if ((n) <= 56) F(2, 2, 10, 6);                                                 \
+        if ((n) <= 64) F(2, 2, 16, 4);                                                 \
+        if ((n) <= 76) F(3, 4, 7, 3);                                                  \
+        if ((n) <= 96) F(3, 4, 8, 2);                                                  \
+        if ((n) <= 128) F(4, 8, 8, 1);                                                 \
+        F(5, 8, 9, 1);                                                                 \
+    } while (0)
+
+template <int R, int NW, int NS, int MINB>
+cudaError_t run_hetrd_reg(int n, int batch, const double2* C, const Workspace& ws, const int* info,
+                          cudaStream_t stream) {
+    const size_t smem = RegHetrdSmem<R, NW>(n, NS).total;
+    if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
+    static SmemOptIn f;
+    set_smem_limit(reinterpret_cast<const void*>(k_hetrd_reg<R, NW, NS, MINB>), f, static_cast<int>(smem));
+    k_hetrd_reg<R, NW, NS, MINB><<<batch, 32 * NW, smem, stream>>>(n, batch, C, ws, info);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_hetrd_reg(int n, int batch, const double2* C, const Workspace& ws, const int* info,
+                             cudaStream_t stream) {
+    if (batch <= 0) return cudaSuccess;
+    if (n < 1 || n > kHetrdRegMaxN || !C || !info || !ws.LV || !ws.d || !ws.e || !ws.tau) return cudaErrorInvalidValue;
+#define SBG_RUN(R, NW, NS, MINB) return run_hetrd_reg<R, NW, NS, MINB>(n, batch, C, ws, info, stream)
+    SBG_HETRD_REG_BY_N(n, SBG_RUN);
+#undef SBG_RUN
+}
+
+size_t hetrd_reg_smem_bytes(int n) {
+#define SBG_SIZE(R, NW, NS, MINB) return RegHetrdSmem<R, NW>(n, NS).total
+    SBG_HETRD_REG_BY_N(n, SBG_SIZE);
+#undef SBG_SIZE
+}
+
+}  // namespace sbg

@@ -3,9 +3,9 @@
 //
 //   reduce   k_potrf_warp + k_hegst_col (n <= 56) or k_reduce (57..84): B = L L^H and
 //            C = L^{-1} A L^{-H}; L into the workspace, C into the caller's X buffer.
-//   hetrd    k_hetrd_warp (n <= 65) or k_hetrd: Householder tridiagonalisation of C,
-//            reflectors and (d, e, tau) into the workspace; the mixed form (n <= 56) runs it
-//            in complex64 (k_hetrd_warp_c64).
+//   hetrd    k_hetrd_reg (hetrd_reg.cu): Householder tridiagonalisation of C, reflectors and
+//            (d, e, tau) into the workspace; the mixed form (n <= 63) runs it in complex64
+//            (k_hetrd_warp_c64).
 //   eig      FP64, n <= 63 (and 85..128, launched from bigsolve.cu): k_tridiag_values
 //            (tridiag.cu: bisection on Sturm counts, a thread per one or two eigenvalues) and
 //            k_tridiag_invit (eigenvectors by inverse iteration, one warp per pair).
@@ -385,122 +385,11 @@ __global__ void __launch_bounds__(back_col_threads<NMAX, G>(), G == 1 ? 4 : 3) k
     }
 }
 
-// ----------------------------------------------------------------------------- k_hetrd
-// One CTA per pair, one tile: C (lower triangle) staged by TMA bulk copies, reduced
-// to tridiagonal form; the reflectors go to the upper part of the pair's LV tile.
-struct HetrdSmem {
-    size_t As, vw, pbuf, ww, d, e, tau, bar, total;
-    __host__ __device__ HetrdSmem(int n, int threads) {
-        const size_t ld = static_cast<size_t>(tile_ld(n));
-        const size_t nw = static_cast<size_t>(threads / 32);
-        size_t o = 0;
-        As = o;   o += 16 * ld * n;
-        vw = o;   o += 16 * n * nw;
-        pbuf = o; o += 32 * n;
-        ww = o;   o += 16 * n * nw;
-        d = o;    o += align_up(8 * n, 16);
-        e = o;    o += align_up(8 * n, 16);
-        tau = o;  o += 16 * n;
-        bar = o;  o += 16;
-        total = o;
-    }
-};
-template <int T>
-__global__ void __launch_bounds__(T) k_hetrd(int n, int batch, const double2* __restrict__ C, Workspace ws,
-                                             int* __restrict__ info) {
-    const int b = blockIdx.x;
-    if (b >= batch || !pair_selected(ws, b)) return;
-    if (info[b] != 0) return;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const HetrdSmem lay(n, T);
-    const int ld = tile_ld(n);
-    double2* As = reinterpret_cast<double2*>(smem + lay.As);
-    double2* vw = reinterpret_cast<double2*>(smem + lay.vw);
-    double2* pbuf = reinterpret_cast<double2*>(smem + lay.pbuf);
-    double2* ww = reinterpret_cast<double2*>(smem + lay.ww);
-    double* d_s = reinterpret_cast<double*>(smem + lay.d);
-    double* e_s = reinterpret_cast<double*>(smem + lay.e);
-    double2* tau_s = reinterpret_cast<double2*>(smem + lay.tau);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + lay.bar);
-    const int tid = threadIdx.x;
-    const size_t mat = static_cast<size_t>(n) * n;
-    const double2* Cb = C + mat * b;
-    if (tid == 0) { mbar_init(bar, 1); fence_mbar_init(); }
-    __syncthreads();
-    if (tid < 32) {
-        if (tid == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(16 * (static_cast<size_t>(n) * (n + 1) / 2)));
-        __syncwarp();
-        for (int j = tid; j < n; j += 32)
-            bulk_g2s(As + j + static_cast<size_t>(j) * ld, Cb + j + static_cast<size_t>(j) * n, 16u * (n - j), bar);
-    }
-    wait_copies(bar, info + b);
-    hetrd_lower(As, ld, n, d_s, e_s, tau_s, vw, pbuf, ww);
-    // reflector k, component i >= k+2, sits at A(i, k); it goes to LV(k, i)
-    double2* LVg = ws.LV + mat * b;
-    for (size_t idx = tid; idx < mat; idx += T) {
-        const int i = static_cast<int>(idx / n), k = static_cast<int>(idx - static_cast<size_t>(i) * n);
-        if (i >= k + 2) LVg[k + static_cast<size_t>(i) * n] = As[i + k * ld];
-        else if (i == k + 1) LVg[k + static_cast<size_t>(i) * n] = make_double2(1.0, 0.0);
-    }
-    for (int i = tid; i < n; i += T) {
-        ws.d[static_cast<size_t>(n) * b + i] = d_s[i];
-        ws.e[static_cast<size_t>(n) * b + i] = e_s[i];
-        ws.tau[static_cast<size_t>(n) * b + i] = (i + 1 < n) ? tau_s[i] : make_double2(0.0, 0.0);
-    }
-}
-
-// ----------------------------------------------------------------------------- k_hetrd_warp
-// One WARP per pair (n <= 65): C's lower triangle is bulk-copied column by column into
-// a packed lower-triangular tile (n(n+1)/2 complex; 23.8 KB at n = 54, so eight pairs
-// fit an SM) and reduced by hetrd_warp_packed with warp-level synchronisation only.
-__host__ __device__ inline size_t hetrd_warp_bytes(int n) {
-    return align_up(16 * static_cast<size_t>(n) * (n + 1) / 2, 16) + 16 * 4 * n + 16;
-}
-constexpr int kHetrdWarpMaxN = 65;
-
-__global__ void __launch_bounds__(32 * kMaxPairWarps) k_hetrd_warp(int n, int batch, const double2* __restrict__ C,
-                                                                  Workspace ws, int* __restrict__ info) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (b >= batch || !pair_selected(ws, b)) return;
-    if (info[b] != 0) return;
-    extern __shared__ __align__(16) unsigned char smem[];
-    unsigned char* base = smem + hetrd_warp_bytes(n) * warp;
-    double2* P = reinterpret_cast<double2*>(base);
-    double2* vb = reinterpret_cast<double2*>(base + align_up(16 * static_cast<size_t>(n) * (n + 1) / 2, 16));
-    double2* wb = vb + n;
-    double2* vb2 = wb + n;
-    double2* wb2 = vb2 + n;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(wb2 + n);
-    const size_t mat = static_cast<size_t>(n) * n;
-    const double2* Cb = C + mat * b;
-    if (lane == 0) { mbar_init(bar, 1); fence_mbar_init(); }
-    __syncwarp();
-    if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(16 * (static_cast<size_t>(n) * (n + 1) / 2)));
-    __syncwarp();
-    for (int j = lane; j < n; j += 32)
-        bulk_g2s(P + pk(j, n), Cb + j + static_cast<size_t>(j) * n, 16u * (n - j), bar);
-    wait_copies(bar, info + b);
-    // d, e and tau go straight to the workspace (global memory): that keeps the per-pair shared
-    // memory at what eight pairs per SM allow
-    double* dg = ws.d + static_cast<size_t>(n) * b;
-    double* eg = ws.e + static_cast<size_t>(n) * b;
-    double2* taug = ws.tau + static_cast<size_t>(n) * b;
-    hetrd_warp_packed<double>(P, n, dg, eg, taug, vb, wb, vb2, wb2);
-    double2* LVg = ws.LV + mat * b;
-    for (int k = 0; k + 1 < n; ++k) {                    // LV(k, k+1) = v_k(k+1) = 1
-        const double2* col = P + pk(k, n) - k;           // col[i] = A(i, k), i >= k
-        for (int i = k + 1 + lane; i < n; i += 32)
-            LVg[k + static_cast<size_t>(i) * n] = (i == k + 1) ? make_double2(1.0, 0.0) : col[i];
-    }
-    if (lane == 0) taug[n - 1] = make_double2(0.0, 0.0);
-}
-
 // ----------------------------------------------------------------------------- k_hetrd_warp_c64
 // Mixed form, Householder stage in complex64: one WARP per pair (n <= 65).  C's lower triangle
 // (FP64, in the X buffer) is rounded to complex64 into a packed tile (8 B per entry: 11.9 KB at
-// n = 54, half of k_hetrd_warp's, so twice the pairs fit an SM) and tridiagonalised by
-// hetrd_warp_packed<float>.  Outputs go where k_hetrd_warp puts them, promoted to FP64, so the
+// n = 54) and tridiagonalised by hetrd_warp_packed<float>.  Outputs go where the FP64 form's
+// Householder (k_hetrd_reg) puts them, promoted to FP64, so the
 // FP64 eigen- and back-transform kernels run on them unchanged: reflectors in LV's rows above the
 // superdiagonal, (d, e), and tau rescaled in FP64 so that each H = I - tau v v^H is unitary to
 // FP64 rounding for the promoted v (|tau|^2 ||v||^2 = 2 Re tau; the FP32 tau satisfies it only to
@@ -508,7 +397,7 @@ __global__ void __launch_bounds__(32 * kMaxPairWarps) k_hetrd_warp(int n, int ba
 // also written to the pair's stash in the refinement's tile format (refine_stash_entries), since
 // X, where the reduction left it, is overwritten before the refinement runs.
 __host__ __device__ inline size_t hetrd_c64_bytes(int n) {
-    return align_up(8 * static_cast<size_t>(n) * (n + 1) / 2, 16) + 8 * 4 * n + 2 * align_up(4 * n, 16) +
+    return align_up(8 * static_cast<size_t>(n) * (n + 1) / 2, 16) + 8 * 2 * n + 2 * align_up(4 * n, 16) +
            align_up(8 * n, 16) + 16;
 }
 
@@ -528,9 +417,7 @@ __global__ void __launch_bounds__(32 * kMaxPairWarps) k_hetrd_warp_c64(int n, in
     float2* P = reinterpret_cast<float2*>(base);
     float2* vb = reinterpret_cast<float2*>(base + align_up(8 * static_cast<size_t>(n) * (n + 1) / 2, 16));
     float2* wb = vb + n;
-    float2* vb2 = wb + n;
-    float2* wb2 = vb2 + n;
-    float* d_s = reinterpret_cast<float*>(wb2 + n);
+    float* d_s = reinterpret_cast<float*>(wb + n);
     float* e_s = d_s + align_up(4 * n, 16) / 4;
     float2* tau_s = reinterpret_cast<float2*>(e_s + align_up(4 * n, 16) / 4);
     const size_t mat = static_cast<size_t>(n) * n;
@@ -552,7 +439,7 @@ __global__ void __launch_bounds__(32 * kMaxPairWarps) k_hetrd_warp_c64(int n, in
         }
     }
     __syncwarp();
-    hetrd_warp_packed<float, false>(P, n, d_s, e_s, tau_s, vb, wb, vb2, wb2);
+    hetrd_warp_packed<float>(P, n, d_s, e_s, tau_s, vb, wb);
     double2* LVg = ws.LV + mat * b;
     for (int k = 0; k + 1 < n; ++k) {                    // LV(k, k+1) = v_k(k+1) = 1
         const float2* col = P + pk(k, n) - k;            // col[i] = v_k(i), i >= k + 2
@@ -1321,36 +1208,11 @@ cudaError_t launch_reduce(int mode, const double2* A, const double2* B, int n, i
     return cudaGetLastError();
 }
 
-size_t hetrd_smem_bytes(int n, int threads) { return HetrdSmem(n, threads).total; }
-
-cudaError_t launch_hetrd(int n, int batch, const double2* C, const Workspace& ws, int* info, const LaunchShape& shape,
-                         cudaStream_t stream) {
-    const int threads = shape.threads;
+cudaError_t launch_hetrd(int n, int batch, const double2* C, const Workspace& ws, int* info, cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
-    if (!C || !info || !ws.LV || !ws.d || !ws.e || !ws.tau) return cudaErrorInvalidValue;
-    if (n > kSmallMaxN) return big_path(n) ? cudaSuccess : cudaErrorInvalidValue;   // done by the reduce kernel
-    if (n <= kHetrdWarpMaxN) {
-        const int pw = pair_warps_of(shape);
-        const size_t smem = hetrd_warp_bytes(n) * pw;
-        if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
-        static SmemOptIn fw;
-        set_max_smem_once(k_hetrd_warp, fw);
-        k_hetrd_warp<<<(batch + pw - 1) / pw, 32 * pw, smem, stream>>>(n, batch, C, ws, info);
-        return cudaGetLastError();
-    }
-    const size_t smem = hetrd_smem_bytes(n, threads == 128 ? 128 : 256);
-    if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
-    static SmemOptIn f128, f256;
-    if (threads == 128) {
-        set_max_smem_once(k_hetrd<128>, f128);
-        k_hetrd<128><<<batch, 128, smem, stream>>>(n, batch, C, ws, info);
-    } else {
-        set_max_smem_once(k_hetrd<256>, f256);
-        k_hetrd<256><<<batch, 256, smem, stream>>>(n, batch, C, ws, info);
-    }
-    return cudaGetLastError();
+    if (n > kSmallMaxN) return big_path(n) ? cudaSuccess : cudaErrorInvalidValue;   // done by the reduce launch
+    return launch_hetrd_reg(n, batch, C, ws, info, stream);
 }
-
 
 size_t ql_chain_smem_bytes(int n, int threads, bool single) {
     return (single ? 4 : 8) * 2 * static_cast<size_t>(n) * threads;
@@ -1441,7 +1303,7 @@ cudaError_t launch_ql_logged(int n, int batch, const Workspace& ws, double* W, d
 size_t hetrd_c64_smem_bytes(int n) { return hetrd_c64_bytes(n) * kMaxPairWarps; }
 
 size_t pair_kernels_smem_bytes(int n, int pair_warps) {
-    const size_t per = std::max(potrf_warp_bytes(n), std::max(hetrd_warp_bytes(n), hetrd_c64_bytes(n)));
+    const size_t per = std::max(potrf_warp_bytes(n), hetrd_c64_bytes(n));
     return per * static_cast<size_t>(pair_warps);
 }
 

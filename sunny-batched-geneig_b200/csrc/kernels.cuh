@@ -123,20 +123,18 @@ enum BackMode : int {
 };
 
 // Launch shape of the stage kernels, the part of a schedule the autotuner varies:
-//   threads     threads per CTA of k_hetrd (66 <= n <= 84): 128 or 256
-//   pair_warps  pairs (one warp each) per CTA of k_potrf_warp, k_hetrd_warp, k_hetrd_warp_c64
-//               (n <= 65): 1, 2 or 4 -- the reference's "batches per block"
+//   pair_warps  pairs (one warp each) per CTA of k_potrf_warp, k_hetrd_warp_c64 (n <= 65): 1, 2 or
+//               4 -- the reference's "batches per block"
 //   col_exact   k_hegst_col / k_back_col: the exact-n instantiation where one exists (n = 32, 54)
 //               instead of the one for the next larger NMAX
 //   back_lanes  lanes per column of k_back_col (n <= 56): 1 or 2
 //   back_qpass  reflectors per pass of k_back_col's Q application (n <= 56): 1 or 2
 //   reduce_tc   n > 56: the triangular stages on the FP64 tensor cores -- Cholesky and reduction by
 //               the blocked kernel k_reduce_tc (above kSmallMaxN, FP64 form, then the Householder
-//               alone by k_hetrd_l2 instead of k_reduce_mid / k_reduce_big doing all three), and
+//               alone by k_hetrd_reg or k_hetrd_l2 instead of k_reduce_mid / k_reduce_big doing all three), and
 //               X = L^{-H} Y by k_back_tc after the Q-only back-transform, which above kSmallMaxN is
 //               the compact-WY tensor-core kernel k_back_q_tc
 struct LaunchShape {
-    int threads = 256;
     int pair_warps = 2;
     int col_exact = 1;
     int back_lanes = 1;
@@ -149,9 +147,14 @@ cudaError_t launch_reduce(int mode, const double2* A, const double2* B, int n, i
                           const Workspace& ws, double2* out, int* info, const LaunchShape& shape, cudaStream_t stream);
 // Householder tridiagonalisation of C (lower triangle read, column-major, ld = n) ->
 // reflectors into ws.LV (rows above the superdiagonal), tau, d, e.  Pairs with info != 0 skip.
-cudaError_t launch_hetrd(int n, int batch, const double2* C, const Workspace& ws, int* info, const LaunchShape& shape,
-                         cudaStream_t stream);
-size_t hetrd_smem_bytes(int n, int threads);
+cudaError_t launch_hetrd(int n, int batch, const double2* C, const Workspace& ws, int* info, cudaStream_t stream);
+// The same for n <= kHetrdRegMaxN (csrc/hetrd_reg.cu, which launch_hetrd runs); reflectors along LV's
+// rows up to kSmallMaxN, its columns above.  Honours the pair selection.  kHetrdRegMaxN is where a
+// pair's matrix still fits one SM's registers and shared memory together.
+constexpr int kHetrdRegMaxN = 144;
+size_t hetrd_reg_smem_bytes(int n);      // dynamic shared memory of its CTA
+cudaError_t launch_hetrd_reg(int n, int batch, const double2* C, const Workspace& ws, const int* info,
+                             cudaStream_t stream);
 // Two-kernel QL: thread-per-pair scalar chain logging rotations, then a warp-per-pair
 // application of the log to Z (single = FP32 chain and Z, the mixed form's first half).
 cudaError_t launch_ql_logged(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
@@ -171,8 +174,7 @@ cudaError_t launch_refine_mixed(int n, int batch, const Workspace& ws, double* W
 cudaError_t launch_eig_mixed(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                              int refine_steps, int chain_threads, const LaunchShape& shape, cudaStream_t stream);
 size_t hetrd_c64_smem_bytes(int n);
-// Dynamic shared memory of a CTA of the warp-per-pair kernels (k_potrf_warp, k_hetrd_warp,
-// k_hetrd_warp_c64) with pair_warps pairs.
+// Dynamic shared memory of a CTA of the warp-per-pair kernels (k_potrf_warp, k_hetrd_warp_c64) with pair_warps pairs.
 size_t pair_kernels_smem_bytes(int n, int pair_warps);
 size_t refine_c_smem_bytes(int n);
 size_t mixed_fallback_smem_bytes(int n);
@@ -199,7 +201,7 @@ size_t ql_rows_smem_bytes(int n, bool single);
 size_t big_stage_smem_bytes(int n, bool tc, int chain_threads);
 // mode: kBigFull (Cholesky, reduction, Householder: k_reduce_mid / k_reduce_big), kBigHegstOnly (the
 // same kernels, stopping after C = L^{-1} A L^{-H}: C's lower triangle in X, L in LV) or kBigHetrdOnly
-// (the Householder alone by k_hetrd_l2, from C's lower triangle in X with L already in LV, as
+// (the Householder alone by k_hetrd_reg or k_hetrd_l2, from C's lower triangle in X with L already in LV, as
 // k_reduce_tc leaves them; pairs with info != 0 are skipped).
 enum BigReduceMode : int { kBigFull = 0, kBigHegstOnly = 1, kBigHetrdOnly = 2 };
 cudaError_t launch_reduce_big(const double2* A, const double2* B, int n, int batch, const Workspace& ws, double2* X,
@@ -214,7 +216,7 @@ cudaError_t launch_reduce_big(const double2* A, const double2* B, int n, int bat
 //                          cores; ws.rstat gets each pair's outcome.
 cudaError_t launch_hetrd_c64_big(int n, int batch, const double2* C, const Workspace& ws, int* info,
                                  cudaStream_t stream);
-// The FP64 Householder alone for n > kSmallMaxN after launch_reduce_tc (C's lower triangle in X),
+// The FP64 Householder alone for n > kHetrdRegMaxN after launch_reduce_tc (C's lower triangle in X),
 // one CTA per pair with the packed triangle in the pair's rotation-log region (L2-resident global
 // memory): reflectors to LV's columns, d, e, tau; pairs with info != 0 are skipped.
 cudaError_t launch_hetrd_l2(int n, int batch, const double2* C, const Workspace& ws, int* info,

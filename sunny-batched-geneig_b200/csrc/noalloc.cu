@@ -96,7 +96,7 @@ extern "C" int sbg_geneig_full_noalloc_launch(int n, const cuDoubleComplex* d_A,
     const double2* B = reinterpret_cast<const double2*>(d_B);
     double2* X = reinterpret_cast<double2*>(d_X);
     e = sbg::launch_reduce(sbg::kReduceFull, A, B, n, batch, ws, X, d_info, sch.shape(), stream);
-    if (e == cudaSuccess) e = sbg::launch_hetrd(n, batch, X, ws, d_info, sch.shape(), stream);
+    if (e == cudaSuccess) e = sbg::launch_hetrd(n, batch, X, ws, d_info, stream);
     if (e == cudaSuccess)
         e = sbg::launch_ql_logged(n, batch, ws, d_W, X, d_info, false, sch.chain_threads, sch.ql_warps, stream);
     if (e == cudaSuccess) e = sbg::launch_back(sbg::kBackFull, n, batch, ws, X, d_info, sch.shape(), stream);

@@ -244,7 +244,7 @@ struct sbg_solver {
         sel.sel_mask = 1 << sbg::kRefineRedo;                   // the FP64 solve of the pairs left over
         check_cuda(sbg::launch_reduce(sbg::kReduceFull, A, B, n, cnt, sel, X, info, sched.shape(), stream),
                    "reduce kernel (FP64 redo)");
-        check_cuda(sbg::launch_hetrd(n, cnt, X, sel, info, sched.shape(), stream), "hetrd kernel (FP64 redo)");
+        check_cuda(sbg::launch_hetrd(n, cnt, X, sel, info, stream), "hetrd kernel (FP64 redo)");
         check_cuda(sbg::launch_ql_logged(n, cnt, sel, W, X, info, false, sched.chain_threads, sched.ql_warps, stream),
                    "QL kernels (FP64 redo)");
         check_cuda(sbg::launch_back(sbg::kBackFull, n, cnt, sel, X, info, sched.shape(), stream),
@@ -269,7 +269,7 @@ struct sbg_solver {
         if (mixed)
             check_cuda(sbg::launch_hetrd_c64(n, cnt, X, ws, info, sched.shape(), stream), "complex64 hetrd kernel");
         else
-            check_cuda(sbg::launch_hetrd(n, cnt, X, ws, info, sched.shape(), stream), "hetrd kernel");
+            check_cuda(sbg::launch_hetrd(n, cnt, X, ws, info, stream), "hetrd kernel");
         stage_end(stream, ev, 1, n > sbg::kSmallMaxN ? 0 : 1);       // large n: inside the reduce kernel
         stage_begin(stream, &ev);
         if (mixed)             // eigenpairs of the complex64 T, Y = Q Z, FP64 refinement against C

@@ -45,7 +45,7 @@ bool fits(int n, int precision, const Schedule& s) {
         return big_reduce_smem_bytes(n) <= lim && ql_rows_smem_bytes(n, false) <= lim &&
                ql_chain_smem_bytes(n, s.chain_threads, false) <= lim;
     }
-    if (reduce_smem_bytes(kReduceFull, n) > lim || back_smem_bytes(n) > lim || hetrd_smem_bytes(n, s.hetrd_threads) > lim) return false;
+    if (reduce_smem_bytes(kReduceFull, n) > lim || back_smem_bytes(n) > lim) return false;
     if (ql_chain_smem_bytes(n, s.chain_threads, false) > lim) return false;
     if (ql_apply_smem_bytes(n, s.ql_warps, false) > lim) return false;
     if (n <= 65 && pair_kernels_smem_bytes(n, s.pair_warps) > lim) return false;
@@ -224,7 +224,7 @@ struct Bench {
     void reduce(const Schedule& s) { launch_reduce(kReduceFull, a(), b(), n, count, ws, x(), inf(), s.shape(), st); }
     void tridiag(const Schedule& s) {
         if (mixed()) launch_hetrd_c64(n, count, x(), ws, inf(), s.shape(), st);
-        else launch_hetrd(n, count, x(), ws, inf(), s.shape(), st);
+        else launch_hetrd(n, count, x(), ws, inf(), st);
     }
     void eig(const Schedule& s) {
         if (mixed())
@@ -266,15 +266,13 @@ bool sweep(int n, int precision, const TuneRequest& req, Schedule& best, double&
     cudaMemcpy(bench.A.p, hA.data(), 16 * bench.nn * count, cudaMemcpyHostToDevice);
     cudaMemcpy(bench.B.p, hB.data(), 16 * bench.nn * count, cudaMemcpyHostToDevice);
     const Schedule base = default_schedule(n, precision);
-    const bool small = n <= kSmallMaxN;
     // pairs per CTA of the warp-per-pair kernels (the reference's batches per block, its BPB
     // sweep over {16, 8, 4, 2, 1}); here at most 4 warps share a CTA
     const std::vector<int> bpb_opts = req.force_bpb && n <= 65 ? std::vector<int>{req.force_bpb}
                                       : n <= 65 ? std::vector<int>{1, 2, 4} : std::vector<int>{base.pair_warps};
     const std::vector<int> exact_opts = (n == 32 || n == 54) ? std::vector<int>{1, 0} : std::vector<int>{base.col_exact};
     const std::vector<int> thread_opts = req.force_threads ? std::vector<int>{req.force_threads}
-                                         : (small && n > 65) ? std::vector<int>{128, 256}
-                                                             : std::vector<int>{base.hetrd_threads};
+                                                           : std::vector<int>{base.hetrd_threads};
     // pairs per CTA of the rotation apply; the inverse-iteration paths have no such parameter
     const bool invit = eig_by_inverse_iteration(n, false);
     const std::vector<int> warp_opts = req.force_bpb && n > 65 ? std::vector<int>{req.force_bpb}

@@ -21,8 +21,9 @@
 namespace sbg {
 
 struct Schedule {
-    int hetrd_threads = 256;    // threads per CTA of k_hetrd (66 <= n <= 84)
-    int pair_warps = 2;         // pairs (warps) per CTA of k_potrf_warp / k_hetrd_warp / k_hetrd_warp_c64
+    int hetrd_threads = 256;    // what block_dim_x reports and force_block_dim_x sets (128 or 256); no kernel's
+                                // CTA size depends on it
+    int pair_warps = 2;         // pairs (warps) per CTA of k_potrf_warp / k_hetrd_warp_c64
                                 // (n <= 65): the reference's batches per block
     int col_exact = 1;          // exact-n column kernels (k_hegst_col, k_back_col) where they exist
     int back_lanes = 1;         // lanes per column of k_back_col (n <= 56)
@@ -32,7 +33,6 @@ struct Schedule {
     int chain_threads = 128;    // pairs (threads) per CTA of the QL scalar-chain kernels
     LaunchShape shape() const {
         LaunchShape l;
-        l.threads = hetrd_threads;
         l.pair_warps = pair_warps;
         l.col_exact = col_exact;
         l.back_lanes = back_lanes;
