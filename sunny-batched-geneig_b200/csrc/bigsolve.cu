@@ -1023,41 +1023,39 @@ __global__ void __launch_bounds__(kMidThreads, 3) k_hetrd_l2(int n, int batch, c
 }
 
 // ----------------------------------------------------------------------------- k_ql_apply_rows
-template <typename R>
 __host__ __device__ inline size_t ql_rows_bytes(int n) {
-    return big_align(sizeof(R) * 32 * static_cast<size_t>(tile_ld(n)), 16) + 64 * sizeof(cplx<R>) +
-           big_align(sizeof(R) * 2 * static_cast<size_t>(n), 16);
+    return big_align(8 * 32 * static_cast<size_t>(tile_ld(n)), 16) + 64 * 16 +
+           big_align(8 * 2 * static_cast<size_t>(n), 16);
 }
 
-// redo: only the pairs flagged by k_tridiag_invit (ws.flag 2, or 3 after a log overflow).
-template <typename R>
+// The rotation-log QL's second half, for the pairs flagged kFlagRedo (or 3 after a log overflow): the
+// log applied to one 32-row block of Z per CTA.
 __global__ void __launch_bounds__(32) k_ql_apply_rows(int n, int batch, Workspace ws, double* __restrict__ W,
-                                                      double2* __restrict__ X, int* __restrict__ info, int redo) {
-    using C = cplx<R>;
+                                                      double2* __restrict__ X, int* __restrict__ info) {
     const int nrb = (n + 31) / 32;                     // row blocks per pair
     const int b = blockIdx.x / nrb, rb = blockIdx.x - b * nrb, lane = threadIdx.x;
     if (b >= batch || !pair_selected(ws, b)) return;
-    if (redo && ws.flag[b] < 2) return;
+    if (ws.flag[b] != kFlagRedo && ws.flag[b] != 3) return;
     if (info[b] > n || info[b] < 0) return;            // B not positive definite: the back stage writes NaN
     extern __shared__ __align__(16) unsigned char smem[];
     const int ldz = tile_ld(n);
-    R* Z = reinterpret_cast<R*>(smem);
-    C* stage = reinterpret_cast<C*>(smem + big_align(sizeof(R) * 32 * static_cast<size_t>(ldz), 16));
-    R* dd = reinterpret_cast<R*>(reinterpret_cast<unsigned char*>(stage) + 64 * sizeof(C));
-    R* ee = dd + n;
+    double* Z = reinterpret_cast<double*>(smem);
+    double2* stage = reinterpret_cast<double2*>(smem + big_align(8 * 32 * static_cast<size_t>(ldz), 16));
+    double* dd = reinterpret_cast<double*>(stage + 64);
+    double* ee = dd + n;
     const size_t mat = static_cast<size_t>(n) * n;
-    R* Zg = reinterpret_cast<R*>(X + mat * b);
-    if (ws.flag[b] != 0 && ws.flag[b] != 2) {          // log overflow: warp QL on block 0
+    double* Zg = reinterpret_cast<double*>(X + mat * b);
+    if (ws.flag[b] == 3) {                             // log overflow: warp QL on block 0
         if (rb != 0) return;
-        R* Zs = reinterpret_cast<R*>(reinterpret_cast<unsigned char*>(X + mat * b) + 8 * mat);   // row-major, ld n
-        for (size_t idx = lane; idx < mat; idx += 32) Zs[idx] = (idx / n == idx % n) ? R(1) : R(0);
+        double* Zs = Zg + mat;                         // the second half of the X slot, row-major, ld n
+        for (size_t idx = lane; idx < mat; idx += 32) Zs[idx] = (idx / n == idx % n) ? 1.0 : 0.0;
         for (int i = lane; i < n; i += 32) {
-            dd[i] = static_cast<R>(ws.d[static_cast<size_t>(n) * b + i]);
-            ee[i] = static_cast<R>(ws.e[static_cast<size_t>(n) * b + i]);
+            dd[i] = ws.d[static_cast<size_t>(n) * b + i];
+            ee[i] = ws.e[static_cast<size_t>(n) * b + i];
         }
         __syncwarp();
-        const int unconv = tridiag_ql<R>(n, dd, ee, Zs, n);
-        for (int i = lane; i < n; i += 32) W[static_cast<size_t>(n) * b + i] = static_cast<double>(dd[i]);
+        const int unconv = tridiag_ql<double>(n, dd, ee, Zs, n);
+        for (int i = lane; i < n; i += 32) W[static_cast<size_t>(n) * b + i] = dd[i];
         if (lane == 0 && unconv) info[b] = unconv;
         __syncwarp();
         for (int row = lane; row < n; row += 32)
@@ -1066,12 +1064,12 @@ __global__ void __launch_bounds__(32) k_ql_apply_rows(int n, int batch, Workspac
     }
     const int row = rb * 32 + lane;
     const bool own = row < n;
-    R* zrow = Z + lane * ldz;
+    double* zrow = Z + lane * ldz;
     if (own)
-        for (int c = 0; c < n; ++c) zrow[c] = (row == c) ? R(1) : R(0);
+        for (int c = 0; c < n; ++c) zrow[c] = (row == c) ? 1.0 : 0.0;
     __syncwarp();
-    ql_log_apply_row<R>(reinterpret_cast<const C*>(ws.log) + static_cast<size_t>(ws.log_cap) * b, ws.log_cap, stage,
-                        zrow, own);
+    ql_log_apply_row<double>(reinterpret_cast<const double2*>(ws.log) + static_cast<size_t>(ws.log_cap) * b, ws.log_cap,
+                             stage, zrow, own);
     if (own) {
         const int* perm = ws.perm + static_cast<size_t>(n) * b;
         for (int k = 0; k < n; ++k) Zg[row + static_cast<size_t>(k) * n] = zrow[perm[k]];
@@ -1353,41 +1351,30 @@ cudaError_t launch_hetrd_l2(int n, int batch, const double2* C, const Workspace&
     return cudaGetLastError();
 }
 
-size_t ql_rows_smem_bytes(int n, bool single) { return single ? ql_rows_bytes<float>(n) : ql_rows_bytes<double>(n); }
+size_t ql_rows_smem_bytes(int n) { return ql_rows_bytes(n); }
 
 size_t big_stage_smem_bytes(int n, bool tc, int chain_threads) {
-    size_t m = std::max(ql_rows_smem_bytes(n, false), ql_chain_smem_bytes(n, chain_threads, false));
-    if (eig_by_inverse_iteration(n, false)) m = std::max(m, invit_smem_bytes(n, false));
-    if (tc) return std::max(m, n <= kHetrdRegMaxN ? hetrd_reg_smem_bytes(n) : L2HetrdSmem(n).total);       // k_reduce_tc / k_back_*_tc: static only
+    size_t m = std::max(ql_rows_smem_bytes(n), ql_chain_smem_bytes(n, chain_threads));
+    m = std::max(m, std::max(invit_smem_bytes(n, false), tridiag_ortho_smem_bytes(n, false)));
+    if (tc) return std::max(m, n <= kHetrdRegMaxN ? hetrd_reg_smem_bytes(n) : L2HetrdSmem(n).total);
+    // k_reduce_tc / k_back_*_tc: static only
     return std::max(m, std::max(big_reduce_smem_bytes(n), BigBackSmem(n).total));
 }
 
-cudaError_t launch_ql_rows(int n, int batch, const Workspace& ws, double* W, double2* X, int* info, bool single,
+cudaError_t launch_ql_rows(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                            int chain_threads, cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (!W || !X || !info || !ws.d || !ws.e || !ws.log || !ws.perm || !ws.flag) return cudaErrorInvalidValue;
-    const size_t cs = ql_chain_smem_bytes(n, chain_threads, single);
-    const size_t as = ql_rows_smem_bytes(n, single);
+    const size_t cs = ql_chain_smem_bytes(n, chain_threads), as = ql_rows_smem_bytes(n);
     if (cs > static_cast<size_t>(max_smem_optin()) || as > static_cast<size_t>(max_smem_optin()))
         return cudaErrorInvalidValue;
-    // FP64 up to kInvitBigMaxN: inverse iteration for every pair it can take, then the rotation-log
-    // QL below for the pairs it flagged only
-    const bool redo = eig_by_inverse_iteration(n, single);
-    if (redo) {
-        cudaError_t err = launch_eig_invit(n, batch, ws, W, X, info, chain_threads, true, stream);
-        if (err != cudaSuccess) return err;
-    }
-    cudaError_t err = launch_ql_chain(n, batch, ws, W, info, single, chain_threads, stream, redo);
+    // inverse iteration for every pair it can take, then the rotation-log QL for the pairs it flagged
+    cudaError_t err = launch_eig_invit(n, batch, ws, W, X, info, true, stream);
+    if (err == cudaSuccess) err = launch_ql_chain(n, batch, ws, W, info, chain_threads, stream);
     if (err != cudaSuccess) return err;
-    const int grid = ((n + 31) / 32) * batch;
-    static SmemOptIn fd, ff;
-    if (single) {
-        set_big_smem_once(k_ql_apply_rows<float>, ff, static_cast<size_t>(max_smem_optin()));
-        k_ql_apply_rows<float><<<grid, 32, as, stream>>>(n, batch, ws, W, X, info, 0);
-    } else {
-        set_big_smem_once(k_ql_apply_rows<double>, fd, static_cast<size_t>(max_smem_optin()));
-        k_ql_apply_rows<double><<<grid, 32, as, stream>>>(n, batch, ws, W, X, info, redo ? 1 : 0);
-    }
+    static SmemOptIn fd;
+    set_big_smem_once(k_ql_apply_rows, fd, static_cast<size_t>(max_smem_optin()));
+    k_ql_apply_rows<<<((n + 31) / 32) * batch, 32, as, stream>>>(n, batch, ws, W, X, info);
     return cudaGetLastError();
 }
 

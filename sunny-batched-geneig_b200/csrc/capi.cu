@@ -38,16 +38,16 @@ int supported_max_n(int precision) {
         if (single && n > sbg::kMixedBigMaxN) break;
         const bool big_mixed = single && n > sbg::kMixedMaxN;
         if (n > sbg::kSmallMaxN) {          // cluster kernels
-            size_t need = std::max(sbg::big_reduce_smem_bytes(n), sbg::ql_rows_smem_bytes(n, false));
-            need = std::max(need, sbg::ql_chain_smem_bytes(n, 32, false));
+            size_t need = std::max(sbg::big_reduce_smem_bytes(n), sbg::ql_rows_smem_bytes(n));
+            need = std::max(need, sbg::ql_chain_smem_bytes(n, 32));
             if (big_mixed) need = std::max(need, sbg::hetrd_c64_big_smem_bytes(n));
             if (sbg::big_path(n) && need <= lim) best = n;
             continue;
         }
         size_t need = std::max(sbg::reduce_smem_bytes(sbg::kReduceFull, n), sbg::back_smem_bytes(n));
         need = std::max(need, sbg::hetrd_reg_smem_bytes(n));
-        need = std::max(need, sbg::ql_apply_smem_bytes(n, 1, false));
-        need = std::max(need, sbg::ql_chain_smem_bytes(n, 32, false));
+        need = std::max(need, sbg::ql_apply_smem_bytes(n, 1));
+        need = std::max(need, sbg::ql_chain_smem_bytes(n, 32));
         if (big_mixed) {
             need = std::max(need, sbg::hetrd_c64_big_smem_bytes(n));
         } else if (single) {                // complex64 Householder + FP64 tensor-core refinement
@@ -404,8 +404,7 @@ void geneig_reduce_eig_n54_launch(const cuDoubleComplex* d_H, const cuDoubleComp
         check_cuda(sbg::launch_reduce(sbg::kReduceFull, c2(d_H), c2(d_S), 54, 1, ws, c2(d_V), d_info,
                                       s->sched.shape(), stream), "reduce kernel");
         check_cuda(sbg::launch_hetrd(54, 1, c2(d_V), ws, d_info, stream), "hetrd kernel");
-        check_cuda(sbg::launch_ql_logged(54, 1, ws, d_W, c2(d_V), d_info, false, s->sched.chain_threads,
-                                         s->sched.ql_warps, stream), "QL kernels");
+        check_cuda(sbg::launch_eig(54, 1, ws, d_W, c2(d_V), d_info, s->sched.chain_threads, stream), "eigensolve kernels");
         check_cuda(sbg::launch_back(sbg::kBackQOnly, 54, 1, ws, c2(d_V), d_info, s->sched.shape(), stream),
                    "back kernel");
     }));
@@ -414,7 +413,7 @@ unsigned int geneig_reduce_eig_n54_block_dim_x(void) { return sbg::default_sched
 unsigned int geneig_reduce_eig_n54_shared_mem_bytes(void) { return geneig_full_n54_batched_shared_mem_bytes(); }
 unsigned int geneig_reduce_eig_n54_chol_smem_bytes(void) { return static_cast<unsigned>(sbg::reduce_smem_bytes(sbg::kReduceFull, 54)); }
 unsigned int geneig_reduce_eig_n54_heev_smem_bytes(void) {
-    return static_cast<unsigned>(sbg::ql_apply_smem_bytes(54, sbg::default_schedule(54, SBG_PRECISION_FP64).ql_warps, false));
+    return static_cast<unsigned>(sbg::ql_apply_smem_bytes(54, sbg::default_schedule(54, SBG_PRECISION_FP64).ql_warps));
 }
 unsigned int geneig_reduce_eig_n54_heev_workspace(void) {
     return static_cast<unsigned>(sbg::workspace_bytes_per_pair(54) / 16);
@@ -441,8 +440,8 @@ void geneig_finish_n54_launch(const cuDoubleComplex* d_L, const cuDoubleComplex*
                                           nullptr, d_info + off, s->sched.shape(), stream), "reduce kernel");
             check_cuda(sbg::launch_hetrd(54, cnt, c2(d_M) + nn * off, ws, d_info + off, stream),
                        "hetrd kernel");
-            check_cuda(sbg::launch_ql_logged(54, cnt, ws, d_W + 54 * off, c2(d_U) + nn * off, d_info + off, false,
-                                             s->sched.chain_threads, s->sched.ql_warps, stream), "QL kernels");
+            check_cuda(sbg::launch_eig(54, cnt, ws, d_W + 54 * off, c2(d_U) + nn * off, d_info + off,
+                                       s->sched.chain_threads, stream), "eigensolve kernels");
             check_cuda(sbg::launch_back(sbg::kBackFull, 54, cnt, ws, c2(d_U) + nn * off, d_info + off,
                                         s->sched.shape(), stream), "back kernel");
         }

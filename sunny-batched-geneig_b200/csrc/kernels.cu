@@ -6,11 +6,10 @@
 //   hetrd    k_hetrd_reg (hetrd_reg.cu): Householder tridiagonalisation of C, reflectors and
 //            (d, e, tau) into the workspace; the mixed form (n <= 63) runs it in complex64
 //            (k_hetrd_warp_c64).
-//   eig      FP64, n <= 63 (and 85..128, launched from bigsolve.cu): k_tridiag_values
-//            (tridiag.cu: bisection on Sturm counts, a thread per one or two eigenvalues) and
-//            k_tridiag_invit (eigenvectors by inverse iteration, one warp per pair).
-//            Otherwise k_ql_chain logs the recurrence's rotations and k_ql_apply /
-//            k_ql_apply_reg replay the log onto Z (W ascending).  The mixed form refines
+//   eig      k_tridiag_values (tridiag.cu: bisection on Sturm counts), k_tridiag_invit
+//            (eigenvectors by inverse iteration, one warp per pair) and k_tridiag_ortho
+//            (tridiag.cu: pairs with large clusters); k_ql_chain + k_ql_apply_rows (n > 63) or a
+//            warp QL inside those kernels for the pairs they cannot take.  The mixed form refines
 //            Y = Q Z against C afterwards (refine.cu).
 //   back     k_back_col (n <= 56) or k_back: X = L^{-H} Q Z, written over Z (the mixed
 //            form: Y = Q Z, then X = L^{-H} Y after the refinement).
@@ -465,211 +464,32 @@ __global__ void __launch_bounds__(32 * kMaxPairWarps) k_hetrd_warp_c64(int n, in
 }
 
 // ----------------------------------------------------------------------------- k_ql_chain
-// One THREAD per pair: the scalar QL recurrence with (d, e) in shared memory
-// interleaved over the CTA, rotations appended to the pair's log.  All 32 lanes of
-// a warp do useful work, so the FP64 pipe runs the chains of 32 pairs at once.
-// redo: only the pairs k_tridiag_invit flagged (ws.flag == 2); they keep 2, or 3 on a log overflow.
-template <typename R>
-__global__ void k_ql_chain(int n, int batch, Workspace ws, double* __restrict__ W, int* __restrict__ info,
-                           int redo) {
+// The rotation-log QL's first half, for the pairs flagged kFlagRedo only (they keep the flag, or get 3
+// on a log overflow): one THREAD per pair, the scalar QL recurrence with (d, e) in shared memory
+// interleaved over the CTA, rotations appended to the pair's log.
+__global__ void k_ql_chain(int n, int batch, Workspace ws, double* __restrict__ W, int* __restrict__ info) {
     const int tid = threadIdx.x, T = blockDim.x;
     const int b = blockIdx.x * T + tid;
     extern __shared__ __align__(16) unsigned char smem[];
-    R* d = reinterpret_cast<R*>(smem) + tid;
-    R* e = reinterpret_cast<R*>(smem) + static_cast<size_t>(n) * T + tid;
+    double* d = reinterpret_cast<double*>(smem) + tid;
+    double* e = reinterpret_cast<double*>(smem) + static_cast<size_t>(n) * T + tid;
     if (b >= batch || !pair_selected(ws, b)) return;
-    if (redo) {
-        if (ws.flag[b] != 2) return;
-        if (info[b] > 0 && info[b] <= n) info[b] = 0;          // QL non-convergence: run it again here
-    }
+    if (ws.flag[b] != kFlagRedo) return;
+    if (info[b] > 0 && info[b] <= n) info[b] = 0;              // QL non-convergence: run it again here
     double* Wb = W + static_cast<size_t>(n) * b;
-    cplx<R>* log = reinterpret_cast<cplx<R>*>(ws.log) + static_cast<size_t>(ws.log_cap) * b;
-    if (!redo) ws.flag[b] = 0;
+    double2* log = reinterpret_cast<double2*>(ws.log) + static_cast<size_t>(ws.log_cap) * b;
     if (info[b] != 0) {
         for (int i = 0; i < n; ++i) Wb[i] = __longlong_as_double(0x7ff8000000000000ll);
-        log[0] = mk<R>(R(-1), R(0));
+        log[0] = make_double2(-1.0, 0.0);
         return;
     }
     for (int i = 0; i < n; ++i) {
-        d[i * T] = static_cast<R>(ws.d[static_cast<size_t>(n) * b + i]);
-        e[i * T] = static_cast<R>(ws.e[static_cast<size_t>(n) * b + i]);
+        d[i * T] = ws.d[static_cast<size_t>(n) * b + i];
+        e[i * T] = ws.e[static_cast<size_t>(n) * b + i];
     }
-    const int r = ql_chain<R>(n, d, e, T, log, ws.log_cap, ws.perm + static_cast<size_t>(n) * b, Wb);
-    if (r < 0) ws.flag[b] = redo ? 3 : 1;
+    const int r = ql_chain<double>(n, d, e, T, log, ws.log_cap, ws.perm + static_cast<size_t>(n) * b, Wb);
+    if (r < 0) ws.flag[b] = 3;
     else if (r > 0) info[b] = r;
-}
-
-// ----------------------------------------------------------------------------- k_ql_apply
-// Applies each pair's rotation log to Z = I.  Rows of Z are independent, so a pair
-// gets ceil(n / 32) warps and every lane owns ONE row (Z row-major in shared memory,
-// odd leading dimension); the warps of a pair stream the log independently and never
-// synchronise with each other.  The log is read 32 entries at a time (one coalesced
-// load, staged in a per-warp shared buffer, read back by broadcast); within a sweep
-// the rotation at column i loads z_i and carries z_{i+1} in a register.  Columns are
-// written out in the sorted order of the eigenvalues.  A pair whose log overflowed is
-// solved by the warp-per-pair QL on warp 0 of that pair instead.
-template <typename R>
-__host__ __device__ inline size_t ql_apply_pair_bytes(int n) {
-    const int wpp = (n + 31) / 32;
-    return align_up(sizeof(R) * static_cast<size_t>(n) * tile_ld(n), 16) +
-           static_cast<size_t>(wpp) * 2 * 32 * sizeof(cplx<R>) + align_up(sizeof(R) * 2 * n, 16);
-}
-
-template <typename R>
-__global__ void k_ql_apply(int n, int batch, Workspace ws, double* __restrict__ W, double2* __restrict__ X,
-                           int* __restrict__ info) {
-    using C = cplx<R>;
-    const int wpp = (n + 31) / 32;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pair_in_cta = warp / wpp, wip = warp - pair_in_cta * wpp;
-    const int pairs_per_cta = (blockDim.x >> 5) / wpp;
-    const int b = blockIdx.x * pairs_per_cta + pair_in_cta;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int ldz = tile_ld(n);
-    unsigned char* base = smem + ql_apply_pair_bytes<R>(n) * pair_in_cta;
-    R* Z = reinterpret_cast<R*>(base);
-    C* stage = reinterpret_cast<C*>(base + align_up(sizeof(R) * static_cast<size_t>(n) * ldz, 16)) + wip * 64;
-    R* dd = reinterpret_cast<R*>(base + align_up(sizeof(R) * static_cast<size_t>(n) * ldz, 16) +
-                                 static_cast<size_t>(wpp) * 2 * 32 * sizeof(C));
-    R* ee = dd + n;
-    const bool live = b < batch && pair_selected(ws, b) && !(info[b] > n || info[b] < 0);
-    const int row = wip * 32 + lane;
-    const bool own = live && row < n;
-    R* zrow = Z + row * ldz;
-    if (own)
-        for (int c = 0; c < n; ++c) zrow[c] = (row == c) ? R(1) : R(0);
-    __syncthreads();      // every row is initialised before a fallback warp rotates all of them
-    const bool fallback = live && ws.flag[b] != 0;
-    if (live && !fallback)
-        ql_log_apply_row<R>(reinterpret_cast<const C*>(ws.log) + static_cast<size_t>(ws.log_cap) * b, ws.log_cap,
-                            stage, zrow, own);
-    if (fallback && wip == 0) {
-        for (int i = lane; i < n; i += 32) {
-            dd[i] = static_cast<R>(ws.d[static_cast<size_t>(n) * b + i]);
-            ee[i] = static_cast<R>(ws.e[static_cast<size_t>(n) * b + i]);
-        }
-        __syncwarp();
-        const int unconv = tridiag_ql<R>(n, dd, ee, Z, ldz);
-        for (int i = lane; i < n; i += 32) W[static_cast<size_t>(n) * b + i] = static_cast<double>(dd[i]);
-        if (lane == 0 && unconv) info[b] = unconv;
-    }
-    __syncthreads();      // the fallback's warp wrote every row; all rows are final
-    if (own) {
-        const size_t mat = static_cast<size_t>(n) * n;
-        R* Zg = reinterpret_cast<R*>(X + mat * b);
-        const int* perm = ws.perm + static_cast<size_t>(n) * b;
-        for (int k = 0; k < n; ++k) Zg[row + static_cast<size_t>(k) * n] = zrow[fallback ? k : perm[k]];
-    }
-}
-
-// ----------------------------------------------------------------------------- k_ql_apply_reg
-// The rotation log applied with each lane's row of Z in REGISTERS (n <= NMAX = 32): a sweep
-// of rotations at columns col, col-1, ... enters an unrolled descending chain at case col
-// (every register index static) and updates (z_i, z_{i+1}) in place; the stage buffer
-// streaming is ql_log_apply_row's.  The columns are stored through the inverse sort
-// permutation (z[c] -> column pinv[c]), so no register is ever indexed at run time.  A pair
-// whose log overflowed is solved by the warp QL on its first warp with Z in the second half
-// of the pair's X slice (no shared-memory Z tile is kept for it).
-template <typename R>
-__host__ __device__ inline size_t ql_apply_reg_pair_bytes(int n) {
-    const int wpp = (n + 31) / 32;
-    return static_cast<size_t>(wpp) * 2 * 32 * sizeof(cplx<R>) + align_up(4 * static_cast<size_t>(n), 16) +
-           align_up(sizeof(R) * 2 * static_cast<size_t>(n), 16);
-}
-
-template <int NMAX, typename R>
-__global__ void k_ql_apply_reg(int n, int batch, Workspace ws, double* __restrict__ W, double2* __restrict__ X,
-                               int* __restrict__ info) {
-    using C = cplx<R>;
-    const int wpp = (n + 31) / 32;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pair_in_cta = warp / wpp, wip = warp - pair_in_cta * wpp;
-    const int pairs_per_cta = (blockDim.x >> 5) / wpp;
-    const int b = blockIdx.x * pairs_per_cta + pair_in_cta;
-    extern __shared__ __align__(16) unsigned char smem[];
-    unsigned char* base = smem + ql_apply_reg_pair_bytes<R>(n) * pair_in_cta;
-    C* stage = reinterpret_cast<C*>(base) + wip * 64;
-    int* pinv = reinterpret_cast<int*>(base + static_cast<size_t>(wpp) * 2 * 32 * sizeof(C));
-    R* dd = reinterpret_cast<R*>(base + static_cast<size_t>(wpp) * 2 * 32 * sizeof(C) + align_up(4 * static_cast<size_t>(n), 16));
-    R* ee = dd + n;
-    const bool live = b < batch && !(info[min(b, batch - 1)] > n || info[min(b, batch - 1)] < 0);
-    const bool fallback = live && ws.flag[b] != 0;
-    const int row = wip * 32 + lane;
-    const bool own = live && row < n;
-    R z[NMAX];
-#pragma unroll
-    for (int c = 0; c < NMAX; ++c) z[c] = (row == c) ? R(1) : R(0);
-    if (live && !fallback) {
-        const C* log = reinterpret_cast<const C*>(ws.log) + static_cast<size_t>(ws.log_cap) * b;
-        const int cap = ws.log_cap;
-        int loaded = 0, buf = 0, remaining = 0, col = 0;
-        C pre = log[lane];
-        bool done = false;
-        while (!done) {
-            stage[buf * 32 + lane] = pre;
-            __syncwarp();
-            loaded += 32;
-            if (loaded < cap) pre = log[min(loaded + lane, cap - 1)];
-            const C* st = stage + buf * 32;
-            int k = 0;
-            while (k < 32) {
-                if (remaining == 0) {
-                    const C h = st[k++];
-                    const int top = static_cast<int>(h.x);
-                    if (top < 0) { done = true; break; }
-                    remaining = static_cast<int>(h.y);
-                    col = top;
-                    continue;
-                }
-                const int take = min(remaining, 32 - k);
-                const C* e = st + k;
-                int rem = take;
-                // rotation at column I: (z_I, z_{I+1}) <- (c z_I - s z_{I+1}, s z_I + c z_{I+1})
-#define SBG_ROT(I) case I: if constexpr ((I) + 1 < NMAX) { if (rem == 0) break; const C cs = *e++; \
-                const R zi = z[I], zj = z[(I) + 1]; z[(I) + 1] = fma(cs.y, zi, cs.x * zj); \
-                z[I] = fma(cs.x, zi, -cs.y * zj); --rem; }
-                switch (col) { SBG_DESC64(SBG_ROT) default: break; }
-#undef SBG_ROT
-                k += take;
-                col -= take;
-                remaining -= take;
-            }
-            __syncwarp();
-            buf ^= 1;
-            if (!done && loaded >= cap) done = true;      // malformed log guard (never reached)
-        }
-    }
-    // inverse sort permutation, by the pair's threads
-    if (live && !fallback) {
-        const int* perm = ws.perm + static_cast<size_t>(n) * b;
-        for (int i = wip * 32 + lane; i < n; i += wpp * 32) pinv[perm[i]] = i;
-    }
-    __syncthreads();
-    const size_t mat = static_cast<size_t>(n) * n;
-    if (fallback) {
-        if (wip != 0) return;
-        R* Zs = reinterpret_cast<R*>(reinterpret_cast<unsigned char*>(X + mat * b) + 8 * mat);   // row-major, ld n
-        for (size_t idx = lane; idx < mat; idx += 32) Zs[idx] = (idx / n == idx % n) ? R(1) : R(0);
-        for (int i = lane; i < n; i += 32) {
-            dd[i] = static_cast<R>(ws.d[static_cast<size_t>(n) * b + i]);
-            ee[i] = static_cast<R>(ws.e[static_cast<size_t>(n) * b + i]);
-        }
-        __syncwarp();
-        const int unconv = tridiag_ql<R>(n, dd, ee, Zs, n);
-        for (int i = lane; i < n; i += 32) W[static_cast<size_t>(n) * b + i] = static_cast<double>(dd[i]);
-        if (lane == 0 && unconv) info[b] = unconv;
-        __syncwarp();
-        R* Zg = reinterpret_cast<R*>(X + mat * b);
-        for (int r = lane; r < n; r += 32)
-            for (int k = 0; k < n; ++k) Zg[r + static_cast<size_t>(k) * n] = Zs[static_cast<size_t>(r) * n + k];
-        return;
-    }
-    if (own) {
-        R* Zg = reinterpret_cast<R*>(X + mat * b);
-#pragma unroll
-        for (int c = 0; c < NMAX; ++c)
-            if (c < n) Zg[row + static_cast<size_t>(pinv[c]) * n] = z[c];
-    }
 }
 
 // ----------------------------------------------------------------------------- k_tridiag_invit
@@ -680,10 +500,11 @@ __global__ void k_ql_apply_reg(int n, int batch, Workspace ws, double* __restric
 // per vector against the O(n^2) of applying every QL rotation to it.  The vectors of
 // eigenvalues closer than kInvitOrtol ||T|| (a cluster) are computed in order, one lane per
 // cluster, with three solves each orthogonalised against the cluster's earlier vectors
-// (modified Gram-Schmidt); the other vectors' orthogonality is ~eps ||T|| / gap.  Every
-// vector must pass ||T z - lambda z|| <= kInvitTol ||T||; a pair with a failed vector, a
-// cluster of more than kInvitMaxCluster eigenvalues (a spectrum dominated by one huge
-// eigenvalue), or a T that is not finite is recomputed by the warp QL instead.
+// (modified Gram-Schmidt); the other vectors' orthogonality is ~eps ||T|| / gap.  A pair with a
+// cluster of more than kInvitMaxCluster eigenvalues (a spectrum dominated by one huge eigenvalue) or
+// more than 32 cluster members gets every vector as if it stood alone, and k_tridiag_ortho
+// orthonormalises them.  Every vector must pass ||T z - lambda z|| <= kInvitTol ||T||; a pair with a
+// failed vector or a T that is not finite is recomputed by the QL instead.
 // Per-lane scratch (1/u and the vector) is interleaved [i * 33 + lane]: lane-parallel
 // recurrences read consecutive words, and the warp's column-by-column copy to the caller's X
 // buffer (Z, column k = vector k) reads it across lanes without bank conflicts.
@@ -797,7 +618,7 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
                                                       int flag_redo) {
     const int b = blockIdx.x, lane = threadIdx.x & 31;
     if (b >= batch || !pair_selected(ws, b)) return;
-    if (flag_redo && lane == 0) ws.flag[b] = 0;
+    if (lane == 0) ws.flag[b] = kFlagDone;
     const int inf = info[b];
     if (inf > n || inf < 0) return;                   // an earlier stage failed: W and X are NaN
     extern __shared__ __align__(16) unsigned char smem[];
@@ -841,7 +662,8 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
     }
     __syncwarp();
     const int cnt = sflag[1];
-    bool fallback = inf != 0 || sflag[0] > kInvitMaxCluster || cnt > 32;
+    bool fallback = inf != 0;
+    const bool together = sflag[0] > kInvitMaxCluster || cnt > 32;    // all vectors here, then k_tridiag_ortho
     if (!fallback) {
         bool ok = true;
         double* invu = scr;
@@ -850,7 +672,7 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
         // pseudo-random start, residual test; 32 at a time, then copied out column by column
         for (int base = 0; base < n; base += 32) {
             const int j = base + lane;
-            if (j < n && cls[j] == j) {
+            if (j < n && (together || cls[j] == j)) {
                 invit_factor(n, lam[j], dd, ee, tiny, invu);
                 double s2 = invit_solve<true>(n, ee, invu, zs, 1.0, j);
                 const bool f1 = s2 > 0.0 && isfinite(s2);
@@ -863,7 +685,7 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
             const int top = min(32, n - base);
             for (int L = 0; L < top; ++L) {
                 const int jj = base + L;
-                if (cls[jj] != jj) continue;          // uniform
+                if (!together && cls[jj] != jj) continue;     // uniform
                 double* zc = Zg + static_cast<size_t>(jj) * n;
                 for (int i = lane; i < n; i += 32) zc[i] = zs[i * kInvitLd + L];
             }
@@ -873,7 +695,7 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
         // (2) the other cluster members, one lane each, all at once: three rounds of a solve
         // (every lane its own member) and modified Gram-Schmidt in index order (the whole warp,
         // lanes over rows) against the cluster's first vector and its earlier members
-        if (ok && cnt > 0) {
+        if (ok && cnt > 0 && !together) {
             const int jm = lane < cnt ? members[lane] : -1;
             if (jm >= 0) {
                 invit_factor(n, lam[jm], dd, ee, tiny, invu);
@@ -916,8 +738,9 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
         }
         fallback = !__all_sync(0xffffffffu, ok);
     }
+    if (!fallback && together && lane == 0) ws.flag[b] = kFlagOrtho;
     if (fallback && flag_redo) {
-        if (lane == 0) ws.flag[b] = 2;
+        if (lane == 0) ws.flag[b] = kFlagRedo;
         return;
     }
     if (fallback) {                                   // the warp QL, Z tile over the lane scratch
@@ -1214,34 +1037,27 @@ cudaError_t launch_hetrd(int n, int batch, const double2* C, const Workspace& ws
     return launch_hetrd_reg(n, batch, C, ws, info, stream);
 }
 
-size_t ql_chain_smem_bytes(int n, int threads, bool single) {
-    return (single ? 4 : 8) * 2 * static_cast<size_t>(n) * threads;
-}
-// pairs_per_cta pairs of ceil(n / 32) warps each share a CTA.
-size_t ql_apply_smem_bytes(int n, int pairs_per_cta, bool single) {
-    return (single ? ql_apply_pair_bytes<float>(n) : ql_apply_pair_bytes<double>(n)) * pairs_per_cta;
+size_t ql_chain_smem_bytes(int n, int threads) { return 8 * 2 * static_cast<size_t>(n) * threads; }
+size_t ql_apply_smem_bytes(int n, int pairs_per_cta) {
+    const size_t rows = (static_cast<size_t>(n) + 31) / 32;
+    return (align_up(8 * static_cast<size_t>(n) * tile_ld(n), 16) + rows * 2 * 32 * 16 + align_up(16 * static_cast<size_t>(n), 16)) *
+           pairs_per_cta;
 }
 
-cudaError_t launch_ql_chain(int n, int batch, const Workspace& ws, double* W, int* info, bool single,
-                            int chain_threads, cudaStream_t stream, bool redo) {
+cudaError_t launch_ql_chain(int n, int batch, const Workspace& ws, double* W, int* info, int chain_threads,
+                            cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (!W || !info || !ws.d || !ws.e || !ws.log || !ws.perm || !ws.flag) return cudaErrorInvalidValue;
-    const size_t cs = ql_chain_smem_bytes(n, chain_threads, single);
+    const size_t cs = ql_chain_smem_bytes(n, chain_threads);
     if (cs > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
-    const int cgrid = (batch + chain_threads - 1) / chain_threads;
-    static SmemOptIn fcd, fcf;
-    if (single) {
-        set_max_smem_once(k_ql_chain<float>, fcf);
-        k_ql_chain<float><<<cgrid, chain_threads, cs, stream>>>(n, batch, ws, W, info, redo ? 1 : 0);
-    } else {
-        set_max_smem_once(k_ql_chain<double>, fcd);
-        k_ql_chain<double><<<cgrid, chain_threads, cs, stream>>>(n, batch, ws, W, info, redo ? 1 : 0);
-    }
+    static SmemOptIn f;
+    set_max_smem_once(k_ql_chain, f);
+    k_ql_chain<<<(batch + chain_threads - 1) / chain_threads, chain_threads, cs, stream>>>(n, batch, ws, W, info);
     return cudaGetLastError();
 }
 
 cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
-                             int chain_threads, bool flag_redo, cudaStream_t stream) {
+                             bool flag_redo, cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (!W || !X || !info || !ws.d || !ws.e || !ws.flag) return cudaErrorInvalidValue;
     const size_t is = InvitSmem(n, !flag_redo).per_warp;
@@ -1251,53 +1067,14 @@ cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, d
     const cudaError_t err = launch_tridiag_values(n, batch, ws, W, info, stream);
     if (err != cudaSuccess) return err;
     k_tridiag_invit<<<batch, 32, is, stream>>>(n, batch, ws, W, X, info, flag_redo ? 1 : 0);
-    return cudaGetLastError();
+    return launch_tridiag_ortho(n, batch, ws, W, X, info, !flag_redo, stream);
 }
 
-cudaError_t launch_ql_logged(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
-                             bool single, int chain_threads, int apply_warps, cudaStream_t stream) {
+cudaError_t launch_eig(int n, int batch, const Workspace& ws, double* W, double2* X, int* info, int chain_threads,
+                       cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
-    if (!W || !X || !info || !ws.d || !ws.e || !ws.log || !ws.perm || !ws.flag) return cudaErrorInvalidValue;
-    if (n > kSmallMaxN) return launch_ql_rows(n, batch, ws, W, X, info, single, chain_threads, stream);
-    if (eig_by_inverse_iteration(n, single))                        // eigenvalues by QL, vectors by inverse iteration
-        return launch_eig_invit(n, batch, ws, W, X, info, chain_threads, false, stream);
-    const size_t cs = ql_chain_smem_bytes(n, chain_threads, single);
-    const size_t as = ql_apply_smem_bytes(n, apply_warps, single);
-    if (cs > static_cast<size_t>(max_smem_optin()) || as > static_cast<size_t>(max_smem_optin()))
-        return cudaErrorInvalidValue;
-    const int cgrid = (batch + chain_threads - 1) / chain_threads;
-    const int agrid = (batch + apply_warps - 1) / apply_warps;     // apply_warps = pairs per CTA
-    const int athreads = 32 * ((n + 31) / 32) * apply_warps;
-    if (n <= 32) {                                                  // Z rows in registers
-        // (measured: at n = 32 this beats the shared-memory Z tile by ~4 %; at n = 54 it is 30 %
-        // slower: 148 registers a lane and the per-chunk jump into the rotation chain cost more)
-        cudaError_t err = launch_ql_chain(n, batch, ws, W, info, single, chain_threads, stream);
-        if (err != cudaSuccess) return err;
-        // one pair per CTA: ~150 registers a lane, so small CTAs pack the SM best
-        const size_t rs = single ? ql_apply_reg_pair_bytes<float>(n) : ql_apply_reg_pair_bytes<double>(n);
-        const int rgrid = batch, rthreads = 32 * ((n + 31) / 32);
-        static SmemOptIn r32d, r32f;
-#define SBG_RUN_REG(NM, R, FLAG)                                                                 \
-        { set_max_smem_once(k_ql_apply_reg<NM, R>, FLAG);                                          \
-          k_ql_apply_reg<NM, R><<<rgrid, rthreads, rs, stream>>>(n, batch, ws, W, X, info); }
-        if (single) SBG_RUN_REG(32, float, r32f)
-        else SBG_RUN_REG(32, double, r32d)
-#undef SBG_RUN_REG
-        return cudaGetLastError();
-    }
-    static SmemOptIn fcd, fcf, fad, faf;
-    if (single) {
-        set_max_smem_once(k_ql_chain<float>, fcf);
-        set_max_smem_once(k_ql_apply<float>, faf);
-        k_ql_chain<float><<<cgrid, chain_threads, cs, stream>>>(n, batch, ws, W, info, 0);
-        k_ql_apply<float><<<agrid, athreads, as, stream>>>(n, batch, ws, W, X, info);
-    } else {
-        set_max_smem_once(k_ql_chain<double>, fcd);
-        set_max_smem_once(k_ql_apply<double>, fad);
-        k_ql_chain<double><<<cgrid, chain_threads, cs, stream>>>(n, batch, ws, W, info, 0);
-        k_ql_apply<double><<<agrid, athreads, as, stream>>>(n, batch, ws, W, X, info);
-    }
-    return cudaGetLastError();
+    if (n > kInvitQlMaxN) return launch_ql_rows(n, batch, ws, W, X, info, chain_threads, stream);
+    return launch_eig_invit(n, batch, ws, W, X, info, false, stream);
 }
 
 size_t hetrd_c64_smem_bytes(int n) { return hetrd_c64_bytes(n) * kMaxPairWarps; }

@@ -155,14 +155,13 @@ constexpr int kHetrdRegMaxN = 144;
 size_t hetrd_reg_smem_bytes(int n);      // dynamic shared memory of its CTA
 cudaError_t launch_hetrd_reg(int n, int batch, const double2* C, const Workspace& ws, const int* info,
                              cudaStream_t stream);
-// Two-kernel QL: thread-per-pair scalar chain logging rotations, then a warp-per-pair
-// application of the log to Z (single = FP32 chain and Z, the mixed form's first half).
-cudaError_t launch_ql_logged(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
-                             bool single, int chain_threads, int apply_warps, cudaStream_t stream);
+// Eigenvalues W and eigenvectors Z (real, in X) of every pair's tridiagonal (see the eigensolve below).
+cudaError_t launch_eig(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
+                       int chain_threads, cudaStream_t stream);
 // Mixed form (n <= kMixedMaxN), after the FP64 reduction left C in X:
 //   launch_hetrd_c64     complex64 Householder (warp per pair); FP64-promoted reflectors, tau (made
 //                        unitary in FP64) and T into the workspace, C into the pair's stash;
-//   launch_eig_mixed     eigenpairs of that T (launch_eig_invit, FP64), Y = Q Z
+//   launch_eig_mixed     eigenpairs of that T (launch_eig_invit), Y = Q Z
 //                        (launch_back(kBackQOnly)), then launch_refine_mixed: FP64 Ogita-Aishima
 //                        refinement of (W, Y) against the stashed C on the FP64 tensor cores, and
 //                        the FP64 fallback for pairs it cannot take;
@@ -172,7 +171,7 @@ cudaError_t launch_hetrd_c64(int n, int batch, const double2* C, const Workspace
 cudaError_t launch_refine_mixed(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                                 int refine_steps, cudaStream_t stream);
 cudaError_t launch_eig_mixed(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
-                             int refine_steps, int chain_threads, const LaunchShape& shape, cudaStream_t stream);
+                             int refine_steps, const LaunchShape& shape, cudaStream_t stream);
 size_t hetrd_c64_smem_bytes(int n);
 // Dynamic shared memory of a CTA of the warp-per-pair kernels (k_potrf_warp, k_hetrd_warp_c64) with pair_warps pairs.
 size_t pair_kernels_smem_bytes(int n, int pair_warps);
@@ -195,7 +194,7 @@ constexpr int kSmallMaxN = 84;
 constexpr int kBigMaxN = 256;
 bool big_path(int n);
 size_t big_reduce_smem_bytes(int n);
-size_t ql_rows_smem_bytes(int n, bool single);
+size_t ql_rows_smem_bytes(int n);
 // Largest dynamic shared memory per CTA among the FP64 kernels a solve of order n > kSmallMaxN
 // launches: tc = the schedule's reduce_tc, chain_threads its QL chain width.
 size_t big_stage_smem_bytes(int n, bool tc, int chain_threads);
@@ -241,47 +240,50 @@ cudaError_t launch_refine_big(int n, int batch, const Workspace& ws, double* W, 
                               int refine_steps, cudaStream_t stream);
 size_t hetrd_c64_big_smem_bytes(int n);
 size_t refine_big_smem_bytes();
-cudaError_t launch_ql_rows(int n, int batch, const Workspace& ws, double* W, double2* X, int* info, bool single,
+cudaError_t launch_ql_rows(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                            int chain_threads, cudaStream_t stream);
 cudaError_t launch_back_big(int mode, int n, int batch, const Workspace& ws, double2* X, const int* info,
                             cudaStream_t stream);
-// The QL scalar chain alone (thread per pair): W, the rotation log, perm, flag.
-// redo: only pairs with ws.flag == 2 (flagged by launch_eig_invit); they keep 2, or get 3 on a
-// log overflow.
-cudaError_t launch_ql_chain(int n, int batch, const Workspace& ws, double* W, int* info, bool single,
-                            int chain_threads, cudaStream_t stream, bool redo = false);
+// The QL scalar chain (thread per pair) of the pairs with ws.flag == kFlagRedo: W, the rotation log, perm;
+// the flag stays, or becomes 3 on a log overflow.
+cudaError_t launch_ql_chain(int n, int batch, const Workspace& ws, double* W, int* info, int chain_threads,
+                            cudaStream_t stream);
 
 // Kernels one full reduce launch (kReduceFull) issues for order n: the warp Cholesky and the
 // column hegst kernel for n <= 56; above kSmallMaxN with the tensor-core reduction (tc), k_reduce_tc
 // and the Householder kernel; one kernel otherwise.
 inline int reduce_kernel_count(int n, bool tc = false) { return n <= 56 || (n > kSmallMaxN && tc) ? 2 : 1; }
 // (57 <= n <= 84 with tc: k_reduce_tc alone, the Householder being its own stage there.)
-// FP64 eigenvectors by inverse iteration (k_tridiag_values + k_tridiag_invit) for n <= kInvitMaxN, with
-// the warp QL inside the kernel for pairs it cannot take, and for kSmallMaxN < n <= kInvitBigMaxN,
-// where such pairs are flagged and the rotation-log QL (k_ql_chain + k_ql_apply_rows) redone for
-// them only; the rotation-log QL for every other n and for the mixed form.
-constexpr int kInvitMaxN = 63;
-constexpr int kInvitBigMaxN = 128;
-inline bool eig_by_inverse_iteration(int n, bool single) {
-    return !single && (n <= kInvitMaxN || (n > kSmallMaxN && n <= kInvitBigMaxN));
-}
+// ---- Eigensolve of the tridiagonals, FP64: eigenvalues by bisection (k_tridiag_values), eigenvectors by
+// inverse iteration (k_tridiag_invit), orthonormalised together where many eigenvalues are close
+// (k_tridiag_ortho).  A pair these cannot take (vectors of one eigenspace, a T that is not finite) goes
+// through the QL: in those kernels, one warp, for n <= kInvitQlMaxN; above it by the rotation-log QL
+// (k_ql_chain + k_ql_apply_rows), which runs for the flagged pairs alone.
+constexpr int kInvitQlMaxN = 63;
+// Workspace::flag of a pair after k_tridiag_invit (1 and 3 are the rotation log's overflow marks).
+constexpr int kFlagDone = 0, kFlagRedo = 2, kFlagOrtho = 4;
 // Kernels one eigensolve stage launches for order n.
 inline int eig_kernel_count(int n, bool single) {
-    if (single) return 5;          // k_tridiag_values, k_tridiag_invit, Q-apply, refinement, fallback
-    if (n <= kInvitMaxN) return 2;
-    return n > kSmallMaxN && n <= kInvitBigMaxN ? 4 : 2;
+    if (single) return 6;          // k_tridiag_values, _invit, _ortho, Q-apply, refinement, fallback
+    return n <= kInvitQlMaxN ? 3 : 5;
 }
 // Eigenvalues of every pair's tridiagonal (d, e) by bisection (csrc/tridiag.cu), ascending; NaN for
 // pairs with info != 0.  Honours the pair selection.
 cudaError_t launch_tridiag_values(int n, int batch, const Workspace& ws, double* W, int* info, cudaStream_t stream);
-// Eigenvalues (k_tridiag_values) and inverse-iteration eigenvectors (k_tridiag_invit) of every pair;
-// flag_redo: pairs it cannot take get ws.flag = 2 (and no output) instead of the in-kernel QL.
+// Orthonormalises Z of the pairs with ws.flag == kFlagOrtho (csrc/tridiag.cu); with_ql: the warp QL for those
+// it cannot, otherwise they get kFlagRedo.  Honours the pair selection.
+cudaError_t launch_tridiag_ortho(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
+                                 bool with_ql, cudaStream_t stream);
+size_t tridiag_ortho_smem_bytes(int n, bool with_ql);
+// The three kernels above for every pair; flag_redo: pairs they cannot take get ws.flag = kFlagRedo
+// (and no vectors) instead of the in-kernel QL.
 cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
-                             int chain_threads, bool flag_redo, cudaStream_t stream);
+                             bool flag_redo, cudaStream_t stream);
 
 size_t reduce_smem_bytes(int mode, int n);
-size_t ql_chain_smem_bytes(int n, int threads, bool single);
-size_t ql_apply_smem_bytes(int n, int warps_per_cta, bool single);
+size_t ql_chain_smem_bytes(int n, int threads);
+// The bound on ql_warps (pairs per CTA): each pair's Z tile, log stage and T in shared memory.
+size_t ql_apply_smem_bytes(int n, int pairs_per_cta);
 size_t back_smem_bytes(int n);
 size_t invit_smem_bytes(int n, bool with_tile);
 // r[i] = recip_nr(u[i]) for i < count (device self-test of the inverse iteration's reciprocal).

@@ -230,8 +230,8 @@ struct sbg_solver {
         check_cuda(sbg::launch_hetrd_c64_big(n, cnt, X, ws, info, stream), "complex64 hetrd kernel");
         stage_end(stream, ev, 1, 1);
         stage_begin(stream, &ev);
-        check_cuda(sbg::launch_ql_logged(n, cnt, ws, W, X, info, false, sched.chain_threads, sched.ql_warps, stream),
-                   "QL kernels");
+        check_cuda(sbg::launch_eig(n, cnt, ws, W, X, info, sched.chain_threads, stream),
+                   "eigensolve kernels");
         check_cuda(sbg::launch_back(sbg::kBackQOnly, n, cnt, ws, X, info, sched.shape(), stream), "Q-apply kernel");
         check_cuda(sbg::launch_refine_big(n, cnt, ws, W, X, info, refine_steps, stream), "refinement kernel");
         stage_end(stream, ev, 2, sbg::eig_kernel_count(n, false) + 2);
@@ -245,8 +245,8 @@ struct sbg_solver {
         check_cuda(sbg::launch_reduce(sbg::kReduceFull, A, B, n, cnt, sel, X, info, sched.shape(), stream),
                    "reduce kernel (FP64 redo)");
         check_cuda(sbg::launch_hetrd(n, cnt, X, sel, info, stream), "hetrd kernel (FP64 redo)");
-        check_cuda(sbg::launch_ql_logged(n, cnt, sel, W, X, info, false, sched.chain_threads, sched.ql_warps, stream),
-                   "QL kernels (FP64 redo)");
+        check_cuda(sbg::launch_eig(n, cnt, sel, W, X, info, sched.chain_threads, stream),
+                   "eigensolve kernels (FP64 redo)");
         check_cuda(sbg::launch_back(sbg::kBackFull, n, cnt, sel, X, info, sched.shape(), stream),
                    "back-transform kernel (FP64 redo)");
         stage_end(stream, ev, 3, 1 + 1 + (n > sbg::kSmallMaxN ? 0 : 1) + sbg::eig_kernel_count(n, false) + 1);
@@ -273,12 +273,11 @@ struct sbg_solver {
         stage_end(stream, ev, 1, n > sbg::kSmallMaxN ? 0 : 1);       // large n: inside the reduce kernel
         stage_begin(stream, &ev);
         if (mixed)             // eigenpairs of the complex64 T, Y = Q Z, FP64 refinement against C
-            check_cuda(sbg::launch_eig_mixed(n, cnt, ws, W, X, info, refine_steps, sched.chain_threads, sched.shape(),
+            check_cuda(sbg::launch_eig_mixed(n, cnt, ws, W, X, info, refine_steps, sched.shape(),
                                              stream),
                        "mixed eigensolve kernels");
         else
-            check_cuda(sbg::launch_ql_logged(n, cnt, ws, W, X, info, false, sched.chain_threads, sched.ql_warps,
-                                             stream), "QL kernels");
+            check_cuda(sbg::launch_eig(n, cnt, ws, W, X, info, sched.chain_threads, stream), "eigensolve kernels");
         stage_end(stream, ev, 2, sbg::eig_kernel_count(n, mixed));
         stage_begin(stream, &ev);
         check_cuda(sbg::launch_back(mixed ? sbg::kBackLOnly : sbg::kBackFull, n, cnt, ws, X, info, sched.shape(),

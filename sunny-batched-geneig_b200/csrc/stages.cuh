@@ -192,8 +192,8 @@ __device__ __forceinline__ R pow2_norm(R anorm) {
 // matrix is scaled by a power of two to max-norm in [1/2, 1) first (dsteqr scales only at the range
 // limits; scaling always keeps the single-precision variant safe).
 // Eigenvalues come back ascending with Z's columns permuted alike (dsteqr's
-// final selection sort).  Returns the number of off-diagonals that failed to
-// converge within 30 iterations per eigenvalue (0 on success).
+// final selection sort).  Returns the number of off-diagonals that had not
+// converged after 30 n iterations (0 on success).
 // d, e live in shared memory private to the warp; only lane 0 writes them.
 template <typename R>
 __device__ int tridiag_ql(int n, R* d, R* e, R* Z, int ldz) {
@@ -214,10 +214,9 @@ __device__ int tridiag_ql(int n, R* d, R* e, R* Z, int ldz) {
         e[n - 1] = R(0);
     }
     __syncwarp();
-    int unconverged = 0;
-    const int maxit = 30;
-    for (int l = 0; l < n; ++l) {
-        int iter = 0;
+    int unconverged = 0, iter = 0;
+    const int maxit = 30 * n;                                // in all, as dsteqr
+    for (int l = 0; l < n && unconverged == 0; ++l) {
         for (;;) {
             int m = l;
             for (; m < n - 1; ++m) {
@@ -225,7 +224,10 @@ __device__ int tridiag_ql(int n, R* d, R* e, R* Z, int ldz) {
                 if (em * em <= (eps2 * fabs(d[m])) * fabs(d[m + 1]) + safmin) break;
             }
             if (m == l) break;
-            if (iter == maxit) { ++unconverged; break; }
+            if (iter == maxit) {
+                for (int i = l; i + 1 < n; ++i) unconverged += e[i] != R(0) ? 1 : 0;
+                break;
+            }
             ++iter;
             const R el = e[l], dl = d[l];
             R g = (d[l + 1] - dl) / (R(2) * el);
@@ -319,10 +321,9 @@ __device__ int ql_chain(int n, R* d, R* e, int stride, cplx<R>* log, int cap, in
     for (int i = 0; i < n; ++i) D(i) *= sc;
     for (int i = 0; i + 1 < n; ++i) E(i) *= sc;
     E(n - 1) = R(0);
-    int pos = 0, unconverged = 0;
-    const int maxit = 30;
-    for (int l = 0; l < n; ++l) {
-        int iter = 0;
+    int pos = 0, unconverged = 0, iter = 0;
+    const int maxit = 30 * n;                                // in all, as dsteqr
+    for (int l = 0; l < n && unconverged == 0; ++l) {
         for (;;) {
             int m = l;
             for (; m < n - 1; ++m) {
@@ -330,7 +331,10 @@ __device__ int ql_chain(int n, R* d, R* e, int stride, cplx<R>* log, int cap, in
                 if (em * em <= (eps2 * fabs(D(m))) * fabs(D(m + 1)) + safmin) break;
             }
             if (m == l) break;
-            if (iter == maxit) { ++unconverged; break; }
+            if (iter == maxit) {
+                for (int i = l; i + 1 < n; ++i) unconverged += E(i) != R(0) ? 1 : 0;
+                break;
+            }
             ++iter;
             int hdr = 0;
             if constexpr (LOG) {

@@ -42,12 +42,12 @@ bool fits(int n, int precision, const Schedule& s) {
     }
     if (n > kSmallMaxN) {                 // cluster kernels (FP64 only)
         if (precision == SBG_PRECISION_MIXED || !big_path(n)) return false;
-        return big_reduce_smem_bytes(n) <= lim && ql_rows_smem_bytes(n, false) <= lim &&
-               ql_chain_smem_bytes(n, s.chain_threads, false) <= lim;
+        return big_reduce_smem_bytes(n) <= lim && ql_rows_smem_bytes(n) <= lim &&
+               ql_chain_smem_bytes(n, s.chain_threads) <= lim;
     }
     if (reduce_smem_bytes(kReduceFull, n) > lim || back_smem_bytes(n) > lim) return false;
-    if (ql_chain_smem_bytes(n, s.chain_threads, false) > lim) return false;
-    if (ql_apply_smem_bytes(n, s.ql_warps, false) > lim) return false;
+    if (ql_chain_smem_bytes(n, s.chain_threads) > lim) return false;
+    if (ql_apply_smem_bytes(n, s.ql_warps) > lim) return false;
     if (n <= 65 && pair_kernels_smem_bytes(n, s.pair_warps) > lim) return false;
     if (precision == SBG_PRECISION_MIXED &&
         (n > kMixedMaxN || refine_c_smem_bytes(n) > lim || mixed_fallback_smem_bytes(n) > lim ||
@@ -228,9 +228,9 @@ struct Bench {
     }
     void eig(const Schedule& s) {
         if (mixed())
-            launch_eig_mixed(n, count, ws, w(), x(), inf(), 5, s.chain_threads, s.shape(), st);
+            launch_eig_mixed(n, count, ws, w(), x(), inf(), 5, s.shape(), st);
         else
-            launch_ql_logged(n, count, ws, w(), x(), inf(), false, s.chain_threads, s.ql_warps, st);
+            launch_eig(n, count, ws, w(), x(), inf(), s.chain_threads, st);
     }
     void back(const Schedule& s) {
         launch_back(mixed() ? kBackLOnly : kBackFull, n, count, ws, x(), inf(), s.shape(), st);
@@ -273,10 +273,9 @@ bool sweep(int n, int precision, const TuneRequest& req, Schedule& best, double&
     const std::vector<int> exact_opts = (n == 32 || n == 54) ? std::vector<int>{1, 0} : std::vector<int>{base.col_exact};
     const std::vector<int> thread_opts = req.force_threads ? std::vector<int>{req.force_threads}
                                                            : std::vector<int>{base.hetrd_threads};
-    // pairs per CTA of the rotation apply; the inverse-iteration paths have no such parameter
-    const bool invit = eig_by_inverse_iteration(n, false);
+    // ql_warps shapes no kernel (the eigenvectors come from inverse iteration): kept as asked or built in
     const std::vector<int> warp_opts = req.force_bpb && n > 65 ? std::vector<int>{req.force_bpb}
-                                       : invit ? std::vector<int>{base.ql_warps} : std::vector<int>{1, 2, 4, 8};
+                                                               : std::vector<int>{base.ql_warps};
     Schedule win = base;
     double t_total = 0.0;
     // reduction + tridiagonalisation together (pair_warps is shared by their warp-per-pair kernels)
@@ -427,7 +426,7 @@ TuneResult select_schedule(const TuneRequest& req) {
             if (req.force_bpb != 1 && req.force_bpb != 2 && req.force_bpb != 4)
                 throw std::runtime_error("batches_per_block must be 1, 2 or 4 for n <= 65");
             r.sched.pair_warps = req.force_bpb;
-        } else {                      // pairs per CTA of the QL rotation apply
+        } else {                      // ql_warps
             if (req.force_bpb < 1 || req.force_bpb > 16) throw std::runtime_error("batches_per_block must be 1..16");
             r.sched.ql_warps = req.force_bpb;
         }

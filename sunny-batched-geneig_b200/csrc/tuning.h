@@ -29,8 +29,9 @@ struct Schedule {
     int back_lanes = 1;         // lanes per column of k_back_col (n <= 56)
     int back_qpass = 1;         // reflectors per pass of k_back_col's Q application (n <= 56): 1 or 2
     int reduce_tc = 0;          // n > 84: the triangular stages on the tensor cores (k_reduce_tc, k_back_tc)
-    int ql_warps = 4;           // pairs (warps) per CTA of the QL rotation-application kernel
-    int chain_threads = 128;    // pairs (threads) per CTA of the QL scalar-chain kernels
+    int ql_warps = 4;           // batches_per_block above n = 65, bounded by shared memory; no kernel's shape
+                                // depends on it
+    int chain_threads = 128;    // pairs (threads) per CTA of the QL scalar-chain kernel (n > 63, flagged pairs)
     LaunchShape shape() const {
         LaunchShape l;
         l.pair_warps = pair_warps;
