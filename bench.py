@@ -57,7 +57,7 @@ STAGE_BYTES = {"reduce": 32 * N * N, "tridiag": 0, "eig": 16 * N, "back": 16 * N
 # DRAM bytes (read + write) per pair of each FP64 stage at n = 54: ncu's dram__bytes_read.sum +
 # dram__bytes_write.sum of each stage kernel, one capture of a 16,384-pair solve of this workload
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum --clock-control none \
-#       -k regex:"k_potrf_warp|k_hegst_col|k_hetrd_warp|k_tridiag_values|k_tridiag_invit|k_back_col" -s 6 -c 6 \
+#       -k regex:"k_potrf_warp|k_hegst_col|k_hetrd_reg|k_tridiag_values|k_tridiag_invit|k_back_dmma" -s 6 -c 6 \
 #       python bench.py --pairs 16384 --steps 1 --warmup 1 --no-e2e --no-cpu --forms fp64 --sample 64
 # divided by the pairs.  Traffic grows in proportion to the pairs a launch processes, so traffic per
 # launch = this x pairs per launch.

@@ -1,0 +1,257 @@
+// Back-transform X = L^{-H} Q Z on the FP64 tensor cores with the columns in REGISTERS (k_back_dmma),
+// one CTA per pair, one warp per eight columns, n <= kBackDmmaMaxN.
+//
+// A warp holds its columns transposed, Y^T (8 columns x n rows), as accumulators of
+// mma.sync.m8n8k4.f64: lane (g, t) = (lane / 4, lane % 4) has column g, rows 8 I + 2t and 8 I + 2t + 1
+// of every 8-row tile I.  The same registers are the A operand of the next product if its
+// contraction runs over the rows in the order 0 2 4 6, 1 3 5 7 -- a sum in another order -- so no
+// element of Y ever moves: only V and L, shared by all warps, are read from shared memory.  There
+// row k of the LV tile (LV(k, i) = v_k(i), i > k; L below and on the diagonal) has an odd leading
+// dimension, which keeps the 16-byte fragment loads free of bank conflicts in both orders.
+//
+//   Q    blocks of 8 reflectors in compact WY form (zlarft's T), last to first:
+//        W^T = Y^T conj(V), W^T <- W^T T^T, Y^T -= W^T V^T
+//   L    X_I^T = (Y_I^T - sum_{J > I} X_J^T conj(L_JI)) conj(L_II^{-1}), tile by tile from the last
+//
+// Bound by the tensor pipe and its latency: the products alone take 20.4 K cycles per pair and SM at
+// n = 54 (NT = 7), the kernel 33 K.  It replaced a thread per column (n <= 56: one 16-byte broadcast per
+// complex FMA, FP64 pipe 29 % busy), 4 or 8 lanes per column (57 .. 84) and, for 85 .. 96, tile products
+// through L2.  Microseconds per 1,000 pairs before -> now: n = 24 22 -> 14, 32 29 -> 24, 47 178 -> 71, 54
+// 174 -> 113, 64 472 -> 143, 72 1,286 -> 257, 96 1,441 -> 517; 8 pairs of n = 54: 87 -> 30 us.
+#include "kernels.cuh"
+#include "stages.cuh"
+#include "tiles.cuh"
+
+namespace sbg {
+
+namespace {
+
+constexpr int kBlkLd = 9;                   // an 8 x 8 block (T, L_II^{-1}) in shared memory: (i, j) at i + 9 j
+constexpr int kBlk = 8 * kBlkLd;
+
+template <int NT>
+struct BackDmmaSmem {
+    static constexpr int kLd = 8 * NT + 1;
+    static constexpr size_t lv = 0;
+    static constexpr size_t t = lv + 16 * static_cast<size_t>(kLd) * 8 * NT;
+    static constexpr size_t linv = t + 16 * static_cast<size_t>(kBlk) * NT;
+    static constexpr size_t tau = linv + 16 * static_cast<size_t>(kBlk) * NT;
+    static constexpr size_t total = tau + 16 * 8 * NT;
+};
+
+// (dr, di) += (ar + i ai)(br + i bi): four real products; nai = -ai.
+__device__ __forceinline__ void cmma(double (&dr)[2], double (&di)[2], double ar, double ai, double nai, double2 b) {
+    dmma(dr[0], dr[1], ar, b.x);
+    dmma(di[0], di[1], ai, b.x);
+    dmma(dr[0], dr[1], nai, b.y);
+    dmma(di[0], di[1], ar, b.y);
+}
+
+template <int NT, int MINB>
+__global__ void __launch_bounds__(32 * NT, MINB) k_back_dmma(int mode, int n, int batch, Workspace ws,
+                                                             double2* __restrict__ X, const int* __restrict__ info) {
+    using Sm = BackDmmaSmem<NT>;
+    constexpr int kLd = Sm::kLd, kThreads = 32 * NT;
+    const int b = blockIdx.x;
+    if (b >= batch || !pair_selected(ws, b)) return;
+    const size_t mat = static_cast<size_t>(n) * n;
+    double2* Xb = X + mat * b;
+    const int tid = threadIdx.x;
+    if (info[b] > n || info[b] < 0) {                             // uniform: B was not positive definite
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        for (size_t idx = tid; idx < mat; idx += kThreads) Xb[idx] = make_double2(nan, nan);
+        return;
+    }
+    extern __shared__ __align__(16) unsigned char smem[];
+    double2* LV = reinterpret_cast<double2*>(smem + Sm::lv);
+    double2* Tm = reinterpret_cast<double2*>(smem + Sm::t);
+    double2* Li = reinterpret_cast<double2*>(smem + Sm::linv);
+    double2* tau = reinterpret_cast<double2*>(smem + Sm::tau);
+    const int lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+    const double2 zero = make_double2(0.0, 0.0);
+    // ---- LV into shared memory, padded with the identity
+    {
+        const double2* LVg = ws.LV + mat * b;
+        const bool cols = n > kSmallMaxN;                         // reflectors along LV's columns
+        for (int j = w; j < 8 * NT; j += NT)
+            for (int i = lane; i < 8 * NT; i += 32) {
+                double2 v = make_double2(i == j ? 1.0 : 0.0, 0.0);
+                if (i < n && j < n) {
+                    if (i >= j || !cols) v = LVg[i + static_cast<size_t>(j) * n];
+                    else v = LVg[(j - i - 1) + static_cast<size_t>(n - 1 - i) * n];      // v_i(j)
+                }
+                LV[i + j * kLd] = v;
+            }
+        for (int i = tid; i < 8 * NT; i += kThreads) tau[i] = i < n ? ws.tau[static_cast<size_t>(n) * b + i] : zero;
+    }
+    // ---- the warp's columns
+    double yr[NT][2], yi[NT][2];
+    const int col = 8 * w + g;
+    const double* Zg = reinterpret_cast<const double*>(Xb);
+#pragma unroll
+    for (int I = 0; I < NT; ++I)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int r = 8 * I + 2 * t + q;
+            double2 v = zero;
+            if (r < n && col < n) {
+                if (mode == kBackLOnly) v = Xb[r + static_cast<size_t>(col) * n];
+                else v.x = Zg[r + static_cast<size_t>(col) * n];
+            }
+            yr[I][q] = v.x;
+            yi[I][q] = v.y;
+        }
+    __syncthreads();                                              // every Z is read before any X is stored
+    // V(8 I + i, 8 B + k): zero on and above the diagonal of the tile I == B
+    auto vat = [&](int I, int B, int i, int k) {
+        double2 v = LV[(8 * B + k) + (8 * I + i) * kLd];
+        if (I == B && i <= k) v = zero;
+        return v;
+    };
+    // ---- warp w: T of block w of reflectors, the inverse of diagonal block w of L
+    if (mode != kBackLOnly) {
+        double gr[2] = {0.0, 0.0}, gi[2] = {0.0, 0.0};            // G(g, 2t + q) = v_g^H v_{2t+q}
+        for (int I = w; I < NT; ++I)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const double2 v = vat(I, w, 2 * t + q, g);
+                cmma(gr, gi, v.x, -v.y, v.y, v);
+            }
+        double2* T = Tm + w * kBlk;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) T[g + kBlkLd * (2 * t + q)] = make_double2(gr[q], gi[q]);
+        __syncwarp();
+        if (lane < 8) {                                           // lane i: row i of T
+            double2 row[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                double2 s = zero;
+#pragma unroll
+                for (int l = 0; l < j; ++l) s = cfma(row[l], T[l + kBlkLd * j], s);
+                const double2 tj = tau[8 * w + j];
+                row[j] = j == lane ? tj : j > lane ? cmul(s, make_double2(-tj.x, -tj.y)) : zero;
+            }
+            __syncwarp(0xffu);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) T[lane + kBlkLd * j] = row[j];
+        }
+    }
+    if (mode != kBackQOnly && lane < 8) {                         // lane j: column j of L_ww^{-1}
+        const double2* D = LV + 8 * w + 8 * w * kLd;
+        double2 x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            double2 s = make_double2(i == lane ? 1.0 : 0.0, 0.0);
+#pragma unroll
+            for (int l = 0; l < i; ++l) s = cfms(D[i + l * kLd], x[l], s);
+            x[i] = cscale(s, 1.0 / D[i + i * kLd].x);
+            Li[w * kBlk + i + kBlkLd * lane] = x[i];
+        }
+    }
+    __syncthreads();
+    // ---- Y <- Q Y
+    if (mode != kBackLOnly) {
+        for (int B = NT - 1; B >= 0; --B) {
+            if (8 * B + 1 >= n) continue;                         // no reflector in the block
+            double wr[2] = {0.0, 0.0}, wi[2] = {0.0, 0.0};
+#pragma unroll
+            for (int I = 0; I < NT; ++I) {
+                if (I < B) continue;                              // uniform
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    double2 v = vat(I, B, 2 * t + q, g);
+                    v.y = -v.y;
+                    cmma(wr, wi, yr[I][q], yi[I][q], -yi[I][q], v);
+                }
+            }
+            double ur[2] = {0.0, 0.0}, ui[2] = {0.0, 0.0};
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                cmma(ur, ui, wr[q], wi[q], -wi[q], Tm[B * kBlk + g + kBlkLd * (2 * t + q)]);
+#pragma unroll
+            for (int I = 0; I < NT; ++I) {
+                if (I < B) continue;
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    cmma(yr[I], yi[I], -ur[q], -ui[q], ui[q], vat(I, B, g, 2 * t + q));
+            }
+        }
+    }
+    // ---- Y <- L^{-H} Y
+    if (mode != kBackQOnly) {
+#pragma unroll
+        for (int I = NT - 1; I >= 0; --I) {
+#pragma unroll
+            for (int J = NT - 1; J > I; --J)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    double2 l = LV[(8 * J + 2 * t + q) + (8 * I + g) * kLd];
+                    l.y = -l.y;
+                    cmma(yr[I], yi[I], -yr[J][q], -yi[J][q], yi[J][q], l);
+                }
+            double xr[2] = {0.0, 0.0}, xi[2] = {0.0, 0.0};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                double2 l = Li[I * kBlk + (2 * t + q) + kBlkLd * g];
+                l.y = -l.y;
+                cmma(xr, xi, yr[I][q], yi[I][q], -yi[I][q], l);
+            }
+            yr[I][0] = xr[0]; yr[I][1] = xr[1];
+            yi[I][0] = xi[0]; yi[I][1] = xi[1];
+        }
+    }
+    if (col < n) {
+#pragma unroll
+        for (int I = 0; I < NT; ++I)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int r = 8 * I + 2 * t + q;
+                if (r < n) Xb[r + static_cast<size_t>(col) * n] = make_double2(yr[I][q], yi[I][q]);
+            }
+    }
+}
+
+template <int NT, int MINB>
+cudaError_t run_back_dmma(int mode, int n, int batch, const Workspace& ws, double2* X, const int* info,
+                          cudaStream_t stream) {
+    const size_t smem = BackDmmaSmem<NT>::total;
+    if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
+    static SmemOptIn f;
+    set_smem_limit(reinterpret_cast<const void*>(k_back_dmma<NT, MINB>), f, static_cast<int>(smem));
+    k_back_dmma<NT, MINB><<<batch, 32 * NT, smem, stream>>>(mode, n, batch, ws, X, info);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_back_dmma(int mode, int n, int batch, const Workspace& ws, double2* X, const int* info,
+                             cudaStream_t stream) {
+    if (batch <= 0) return cudaSuccess;
+    if (n < 1 || n > kBackDmmaMaxN || !X || !info || !ws.LV || !ws.tau) return cudaErrorInvalidValue;
+#define SBG_CASE(NT, MINB) case NT: return run_back_dmma<NT, MINB>(mode, n, batch, ws, X, info, stream)
+    // (column tiles = warps, CTAs per SM): as many CTAs as the columns' registers allow without spills that
+    // cost more (n = 72: 338 us per 1,000 pairs with one CTA, 257 with two and 176 bytes spilled)
+    switch ((n + 7) / 8) {
+        SBG_CASE(1, 16);
+        SBG_CASE(2, 16);
+        SBG_CASE(3, 8);
+        SBG_CASE(4, 6);
+        SBG_CASE(5, 4);
+        SBG_CASE(6, 3);
+        SBG_CASE(7, 2);
+        SBG_CASE(8, 2);
+        SBG_CASE(9, 2);
+        SBG_CASE(10, 1);
+        SBG_CASE(11, 1);
+        SBG_CASE(12, 1);
+        default: return cudaErrorInvalidValue;
+    }
+#undef SBG_CASE
+}
+
+size_t back_dmma_smem_bytes(int n) {
+    const size_t nt = static_cast<size_t>((n + 7) / 8);
+    return 16 * (8 * nt * (8 * nt + 1) + 2 * kBlk * nt + 8 * nt);
+}
+
+}  // namespace sbg

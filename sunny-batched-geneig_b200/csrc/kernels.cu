@@ -11,8 +11,8 @@
 //            (tridiag.cu: pairs with large clusters); k_ql_chain + k_ql_apply_rows (n > 63) or a
 //            warp QL inside those kernels for the pairs they cannot take.  The mixed form refines
 //            Y = Q Z against C afterwards (refine.cu).
-//   back     k_back_col (n <= 56) or k_back: X = L^{-H} Q Z, written over Z (the mixed
-//            form: Y = Q Z, then X = L^{-H} Y after the refinement).
+//   back     k_back_dmma (back_dmma.cu): X = L^{-H} Q Z, written over Z (the mixed form:
+//            Y = Q Z, then X = L^{-H} Y after the refinement).
 //
 // The split follows where the work is latency bound: the QL recurrence is a
 // dependent scalar chain per pair, so it runs with many pairs per SM, while the
@@ -179,20 +179,6 @@ __global__ void __launch_bounds__(T, RM <= 8 ? 2 : 1) k_reduce(int mode, const d
     if (tid == 0) info[b] = copy_status;
 }
 
-struct BackSmem {
-    size_t LVs, invd, tau, cpair, bar, total;
-    __host__ __device__ BackSmem(int n, int tile_ld_override = 0) {
-        const size_t ld = static_cast<size_t>(tile_ld_override > 0 ? tile_ld_override : tile_ld(n));
-        size_t o = 0;
-        LVs = o;  o += 16 * ld * n;
-        invd = o; o += align_up(8 * n, 16);
-        tau = o;  o += 16 * n;
-        cpair = o; o += 16 * n;
-        bar = o;  o += 16;
-        total = o;
-    }
-};
-
 // ----------------------------------------------------------------------------- k_potrf_warp
 // One WARP per pair (n <= 64): B's lower triangle bulk-copied into a packed tile,
 // Cholesky by potrf_warp_packed; L goes to `out` (strict upper zeroed, the staged
@@ -299,88 +285,6 @@ __global__ void __launch_bounds__(NMAX, 4) k_hegst_col(int mode, const double2* 
         });
         if (mode == kReduceHegst)
             for (int k = i + 1; k < n; ++k) Ob[i + static_cast<size_t>(k) * n] = make_double2(0.0, 0.0);
-    }
-}
-
-// ----------------------------------------------------------------------------- k_back_col
-// One CTA per pair (n <= NMAX): the G adjacent lanes of group j hold column j of Z in
-// registers (rows G r + g), apply Q and L^{-H}, and store X(:, j) (kBackQOnly: Q Z).  The
-// CTA is rounded up to whole warps; lanes of columns j >= n run the sweeps on zeros (the
-// group shuffles need the full warp) and store nothing.
-template <int NMAX, int G>
-__host__ __device__ constexpr int back_col_threads() { return (NMAX * G + 31) / 32 * 32; }
-
-template <int NMAX, int G, bool EXACT, int QP>
-__global__ void __launch_bounds__(back_col_threads<NMAX, G>(), G == 1 ? 4 : 3) k_back_col(int mode, int n_arg, int batch,
-                                                                            Workspace ws, double2* __restrict__ X,
-                                                                            int* __restrict__ info) {
-    const int n = EXACT ? NMAX : n_arg;              // EXACT: n is a compile-time constant
-    constexpr int T = back_col_threads<NMAX, G>();
-    constexpr int RM = (NMAX + G - 1) / G;
-    // tile_ld(NMAX) as a compile-time stride: every row slot's offset is an immediate
-    constexpr int LDC = (((NMAX | 1) & 7) == 7) ? (NMAX | 1) + 2 : (NMAX | 1);
-    const int b = blockIdx.x;
-    if (b >= batch) return;
-    const size_t mat = static_cast<size_t>(n) * n;
-    double2* Xb = X + mat * b;
-    const int tid = threadIdx.x;
-    if (info[b] > n || info[b] < 0) {
-        const double nan = __longlong_as_double(0x7ff8000000000000ll);
-        for (size_t idx = tid; idx < mat; idx += T) Xb[idx] = make_double2(nan, nan);
-        return;
-    }
-    extern __shared__ __align__(16) unsigned char smem[];
-    const BackSmem lay(n, LDC);
-    constexpr int ld = LDC;
-    double2* LVs = reinterpret_cast<double2*>(smem + lay.LVs);
-    double* invd = reinterpret_cast<double*>(smem + lay.invd);
-    double2* tau_s = reinterpret_cast<double2*>(smem + lay.tau);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + lay.bar);
-    const double2* LVg = ws.LV + mat * b;
-    if (tid == 0) { mbar_init(bar, 1); fence_mbar_init(); }
-    __syncthreads();
-    if (tid < 32) {
-        if (tid == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(16 * mat));
-        __syncwarp();
-        for (int j = tid; j < n; j += 32)
-            bulk_g2s(LVs + static_cast<size_t>(j) * ld, LVg + static_cast<size_t>(j) * n, 16u * n, bar);
-    }
-    const int col = tid / G, g = tid - col * G;
-    const bool own = col < n;
-    const double* Zg = reinterpret_cast<const double*>(Xb);
-    double2 y[RM];
-    if (mode == kBackLOnly) {                        // complex Y in the X buffer
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-            const int i = G * r + g;
-            y[r] = (own && i < n) ? Xb[i + static_cast<size_t>(col) * n] : make_double2(0.0, 0.0);
-        }
-    } else {                                         // real Z in the X buffer
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-            const int i = G * r + g;
-            y[r] = make_double2((own && i < n) ? Zg[i + static_cast<size_t>(col) * n] : 0.0, 0.0);
-        }
-    }
-    for (int i = tid; i < n; i += T) tau_s[i] = ws.tau[static_cast<size_t>(n) * b + i];
-    wait_copies(bar, info + b);
-    for (int i = tid; i < n; i += T) invd[i] = 1.0 / LVs[i + i * ld].x;
-    double2* cpair = reinterpret_cast<double2*>(smem + lay.cpair);
-    if (QP == 2 && mode != kBackLOnly) reflector_couplings<double>(LVs, ld, n, cpair, T);
-    __syncthreads();               // all of Z is in registers before any X is stored over it
-    if (mode != kBackLOnly) {
-        if constexpr (QP == 2) grp_apply_q2<G, RM, double>(LVs, ld, tau_s, cpair, y, n, g);
-        else grp_apply_q<G, RM, double>(LVs, ld, tau_s, y, n, g);
-    }
-    double2* xcol = Xb + static_cast<size_t>(col) * n;
-    if (mode == kBackFull || mode == kBackLOnly) {
-        grp_trsm_lowerH2<G, RM>(LVs, ld, invd, y, n, g, [&](int k, double2 x) { if (own) xcol[k] = x; });
-    } else if (own) {
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-            const int i = G * r + g;
-            if (i < n) xcol[i] = y[r];
-        }
     }
 }
 
@@ -762,69 +666,6 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
     }
 }
 
-// ----------------------------------------------------------------------------- k_back
-// One CTA per pair: X = L^{-H} Q Z.  Column j of Z is held in registers by a group
-// of G lanes (lane g owns rows g + G r), read straight from the X buffer; only the
-// LV tile (L below, reflectors above the superdiagonal) is staged in shared memory
-// by TMA bulk copies.  The result is written over Z.
-
-template <int T, int G, int RM>
-__global__ void __launch_bounds__(T, RM <= 8 ? 2 : 1) k_back(int mode, int n, int batch, Workspace ws,
-                                            double2* __restrict__ X, int* __restrict__ info) {
-    const int b = blockIdx.x;
-    if (b >= batch || !pair_selected(ws, b)) return;
-    const size_t mat = static_cast<size_t>(n) * n;
-    double2* Xb = X + mat * b;
-    const int tid = threadIdx.x;
-    if (info[b] > n || info[b] < 0) {     // B not positive definite: nothing to transform
-        const double nan = __longlong_as_double(0x7ff8000000000000ll);
-        for (size_t idx = tid; idx < mat; idx += T) Xb[idx] = make_double2(nan, nan);
-        return;
-    }
-    extern __shared__ __align__(16) unsigned char smem[];
-    const BackSmem lay(n);
-    const int ld = tile_ld(n);
-    double2* LVs = reinterpret_cast<double2*>(smem + lay.LVs);
-    double* invd = reinterpret_cast<double*>(smem + lay.invd);
-    double2* tau_s = reinterpret_cast<double2*>(smem + lay.tau);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + lay.bar);
-
-    const double2* LVg = ws.LV + mat * b;
-    if (tid == 0) { mbar_init(bar, 1); fence_mbar_init(); }
-    __syncthreads();
-    if (tid < 32) {
-        if (tid == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(16 * mat));
-        __syncwarp();
-        for (int j = tid; j < n; j += 32)
-            bulk_g2s(LVs + static_cast<size_t>(j) * ld, LVg + static_cast<size_t>(j) * n, 16u * n, bar);
-    }
-    const int g = tid % G, j = tid / G;
-    const bool valid = j < n;
-    const double* Zg = reinterpret_cast<const double*>(Xb);
-    double2 y[RM];
-#pragma unroll
-    for (int r = 0; r < RM; ++r) {
-        const int i = g + G * r;
-        if (mode == kBackLOnly)            // complex Y in the X buffer
-            y[r] = (valid && i < n) ? Xb[i + static_cast<size_t>(j) * n] : make_double2(0.0, 0.0);
-        else                               // real Z in the X buffer
-            y[r] = make_double2((valid && i < n) ? Zg[i + static_cast<size_t>(j) * n] : 0.0, 0.0);
-    }
-    for (int i = tid; i < n; i += T) tau_s[i] = ws.tau[static_cast<size_t>(n) * b + i];
-    wait_copies(bar, info + b);
-    for (int i = tid; i < n; i += T) invd[i] = 1.0 / LVs[i + i * ld].x;
-    __syncthreads();              // also: every thread has read its Z before any X is written
-    if (mode != kBackLOnly) seg_apply_q<G, RM>(LVs, ld, tau_s, y, n, g);
-    if (mode == kBackFull || mode == kBackLOnly) seg_trsm_lowerH<G, RM>(LVs, ld, invd, y, n, g);
-    if (valid) {
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-            const int i = g + G * r;
-            if (i < n) Xb[i + static_cast<size_t>(j) * n] = y[r];
-        }
-    }
-}
-
 // Pairs (warps) per CTA of the warp-per-pair kernels: 1, 2 or 4 (anything else: the default 2).
 inline int pair_warps_of(const LaunchShape& s) {
     return (s.pair_warps == 1 || s.pair_warps == 2 || s.pair_warps == 4) ? s.pair_warps : 2;
@@ -950,7 +791,6 @@ void set_smem_limit(const void* kernel, SmemOptIn& rec, int bytes) {
 }
 
 size_t reduce_smem_bytes(int, int n) { return ReduceSmem(n).total; }
-size_t back_smem_bytes(int n) { return BackSmem(n).total; }
 size_t invit_smem_bytes(int n, bool with_tile) { return InvitSmem(n, with_tile).per_warp; }
 
 // The register-segment kernels: (threads T, lanes per column G, rows per lane RM) by
@@ -968,14 +808,6 @@ void run_reduce(int mode, const double2* A, const double2* B, int n, int batch, 
     static SmemOptIn f;
     set_max_smem_once(k_reduce<T, G, RM>, f);
     k_reduce<T, G, RM><<<batch, T, smem, stream>>>(mode, A, B, n, batch, ws, out, info);
-}
-
-template <int T, int G, int RM>
-void run_back(int mode, int n, int batch, const Workspace& ws, double2* X, int* info, size_t smem,
-              cudaStream_t stream) {
-    static SmemOptIn f;
-    set_max_smem_once(k_back<T, G, RM>, f);
-    k_back<T, G, RM><<<batch, T, smem, stream>>>(mode, n, batch, ws, X, info);
 }
 
 template <int NMAX, bool EXACT = false>
@@ -1098,22 +930,6 @@ cudaError_t launch_hetrd_c64(int n, int batch, const double2* C, const Workspace
     return cudaGetLastError();
 }
 
-template <int NMAX, int G, bool EXACT = false>
-void run_back_col_g(int mode, int n, int batch, const Workspace& ws, double2* X, int* info, size_t smem,
-                    cudaStream_t stream, int qpass) {
-    smem = BackSmem(n, (((NMAX | 1) & 7) == 7) ? (NMAX | 1) + 2 : (NMAX | 1)).total;
-    if (qpass == 2) {
-        static SmemOptIn f2;
-        set_max_smem_once(k_back_col<NMAX, G, EXACT, 2>, f2);
-        k_back_col<NMAX, G, EXACT, 2><<<batch, back_col_threads<NMAX, G>(), smem, stream>>>(mode, n, batch, ws, X, info);
-    } else {
-        static SmemOptIn f1;
-        set_max_smem_once(k_back_col<NMAX, G, EXACT, 1>, f1);
-        k_back_col<NMAX, G, EXACT, 1><<<batch, back_col_threads<NMAX, G>(), smem, stream>>>(mode, n, batch, ws, X, info);
-    }
-}
-
-
 // ----------------------------------------------------------------------------- k_pull_pairs
 // Pairs are walked grid-stride, each by the whole CTA; every thread keeps 4 independent 16-byte
 // loads in flight (their latency is the host link's, about a microsecond), then stores them.
@@ -1157,49 +973,14 @@ cudaError_t launch_back(int mode, int n, int batch, const Workspace& ws, double2
                         const LaunchShape& shape, cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (!X || !info || !ws.LV || !ws.tau) return cudaErrorInvalidValue;
-    if (n > kSmallMaxN) {
-        if (shape.reduce_tc) {                          // Q Z and L^{-H} on the tensor cores
-            if (mode != kBackLOnly) {
-                const cudaError_t err = launch_back_q_tc(n, batch, ws, X, info, stream);
-                if (err != cudaSuccess || mode == kBackQOnly) return err;
-            }
-            return launch_back_tc(n, batch, ws, X, info, stream);
-        }
-        return launch_back_big(mode, n, batch, ws, X, info, stream);
+    if (n <= kSmallMaxN || (n <= kBackDmmaMaxN && shape.reduce_tc))
+        return launch_back_dmma(mode, n, batch, ws, X, info, stream);
+    if (!shape.reduce_tc) return launch_back_big(mode, n, batch, ws, X, info, stream);
+    if (mode != kBackLOnly) {                           // Q Z and L^{-H} as products through L2
+        const cudaError_t err = launch_back_q_tc(n, batch, ws, X, info, stream);
+        if (err != cudaSuccess || mode == kBackQOnly) return err;
     }
-    const size_t smem = back_smem_bytes(n);
-    if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
-    if (n <= kColMaxN) {
-        const bool two = shape.back_lanes == 2;
-        const int qp = shape.back_qpass == 2 ? 2 : 1;
-        if (n == 32 && shape.col_exact) {
-            if (two) run_back_col_g<32, 2, true>(mode, n, batch, ws, X, info, smem, stream, qp);
-            else run_back_col_g<32, 1, true>(mode, n, batch, ws, X, info, smem, stream, qp);
-        } else if (n == 54 && shape.col_exact) {
-            if (two) run_back_col_g<54, 2, true>(mode, n, batch, ws, X, info, smem, stream, qp);
-            else run_back_col_g<54, 1, true>(mode, n, batch, ws, X, info, smem, stream, qp);
-        } else if (n <= 32) {
-            if (two) run_back_col_g<32, 2>(mode, n, batch, ws, X, info, smem, stream, qp);
-            else run_back_col_g<32, 1>(mode, n, batch, ws, X, info, smem, stream, qp);
-        } else if (n <= 48) {
-            if (two) run_back_col_g<48, 2>(mode, n, batch, ws, X, info, smem, stream, qp);
-            else run_back_col_g<48, 1>(mode, n, batch, ws, X, info, smem, stream, qp);
-        } else {
-            if (two) run_back_col_g<56, 2>(mode, n, batch, ws, X, info, smem, stream, qp);
-            else run_back_col_g<56, 1>(mode, n, batch, ws, X, info, smem, stream, qp);
-        }
-        return cudaGetLastError();
-    }
-    if (shape.reduce_tc && mode != kBackQOnly) {        // Q Z by the CTA kernel, L^{-H} on the tensor cores
-        if (mode == kBackFull) {
-            SBG_DISPATCH_BY_N(n, run_back, kBackQOnly, n, batch, ws, X, info, smem, stream);
-            const cudaError_t err = cudaGetLastError();
-            if (err != cudaSuccess) return err;
-        }
-        return launch_back_tc(n, batch, ws, X, info, stream);
-    }
-    SBG_DISPATCH_BY_N(n, run_back, mode, n, batch, ws, X, info, smem, stream);
-    return cudaGetLastError();
+    return launch_back_tc(n, batch, ws, X, info, stream);
 }
 
 // Device self-test of recip_nr (the inverse iteration's reciprocal): r[i] = recip_nr(u[i]).

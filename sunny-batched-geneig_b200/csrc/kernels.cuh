@@ -125,20 +125,16 @@ enum BackMode : int {
 // Launch shape of the stage kernels, the part of a schedule the autotuner varies:
 //   pair_warps  pairs (one warp each) per CTA of k_potrf_warp, k_hetrd_warp_c64 (n <= 65): 1, 2 or
 //               4 -- the reference's "batches per block"
-//   col_exact   k_hegst_col / k_back_col: the exact-n instantiation where one exists (n = 32, 54)
-//               instead of the one for the next larger NMAX
-//   back_lanes  lanes per column of k_back_col (n <= 56): 1 or 2
-//   back_qpass  reflectors per pass of k_back_col's Q application (n <= 56): 1 or 2
+//   col_exact   k_hegst_col: the exact-n instantiation where one exists (n = 32, 54) instead of the one
+//               for the next larger NMAX
 //   reduce_tc   n > 56: the triangular stages on the FP64 tensor cores -- Cholesky and reduction by
 //               the blocked kernel k_reduce_tc (above kSmallMaxN, FP64 form, then the Householder
 //               alone by k_hetrd_reg or k_hetrd_l2 instead of k_reduce_mid / k_reduce_big doing all three), and
-//               X = L^{-H} Y by k_back_tc after the Q-only back-transform, which above kSmallMaxN is
-//               the compact-WY tensor-core kernel k_back_q_tc
+//               above kSmallMaxN the back-transform by k_back_dmma or k_back_q_tc + k_back_tc instead of
+//               k_back_big
 struct LaunchShape {
     int pair_warps = 2;
     int col_exact = 1;
-    int back_lanes = 1;
-    int back_qpass = 1;
     int reduce_tc = 0;
 };
 
@@ -184,6 +180,12 @@ size_t mixed_fallback_smem_bytes(int n);
 cudaError_t launch_pull_pairs(const double2* src, double2* dst, int count, int n, bool lower, cudaStream_t stream);
 cudaError_t launch_back(int mode, int n, int batch, const Workspace& ws, double2* X, int* info,
                         const LaunchShape& shape, cudaStream_t stream);
+
+// The back-transform of n <= kBackDmmaMaxN on the FP64 tensor cores (csrc/back_dmma.cu), every mode;
+// reflectors along LV's rows up to kSmallMaxN, its columns above.  Honours the pair selection.
+constexpr int kBackDmmaMaxN = 96;
+cudaError_t launch_back_dmma(int mode, int n, int batch, const Workspace& ws, double2* X, const int* info,
+                             cudaStream_t stream);
 
 // Pairs with n <= kSmallMaxN are solved by CTA-per-pair (or warp-per-pair) stage kernels;
 // kSmallMaxN < n <= kBigMaxN by the cluster kernels of bigsolve.cu.  For those the reduce
@@ -284,7 +286,7 @@ size_t reduce_smem_bytes(int mode, int n);
 size_t ql_chain_smem_bytes(int n, int threads);
 // The bound on ql_warps (pairs per CTA): each pair's Z tile, log stage and T in shared memory.
 size_t ql_apply_smem_bytes(int n, int pairs_per_cta);
-size_t back_smem_bytes(int n);
+size_t back_dmma_smem_bytes(int n);
 size_t invit_smem_bytes(int n, bool with_tile);
 // r[i] = recip_nr(u[i]) for i < count (device self-test of the inverse iteration's reciprocal).
 cudaError_t launch_selftest_recip(const double* u, double* r, int count, cudaStream_t stream);

@@ -450,59 +450,6 @@ __device__ __forceinline__ void seg_trsm_right_lowerH(const C* L, int ldl, const
     }
 }
 
-// y <- Q y, Q = H_0 ... H_{n-2}, with the reflectors along the rows of LV: component i >= k+2
-// of v_k sits at LV(k, i) (above the superdiagonal); v_k(k+1) = 1 is implicit.
-template <int G, int RM, typename C>
-__device__ __forceinline__ void seg_apply_q(const C* LV, int ld, const C* tau, C (&y)[RM], int n, int g) {
-    using R = decltype(C().x);
-    for (int k = n - 2; k >= 0; --k) {
-        const C tk = tau[k];
-        if (tk.x == R(0) && tk.y == R(0)) continue;
-        const C* vrow = LV + k;                    // v_k(i) = LV(k, i) = vrow[i * ld], i >= k + 2
-        C s = mk<R>(R(0), R(0));
-#pragma unroll
-        for (int r = RM - 1; r >= 0; --r) {          // active rows i > k form a suffix of r
-            const int i = g + G * r;
-            if (i <= k) break;
-            if (i < n) {
-                const C vi = (i == k + 1) ? mk<R>(R(1), R(0)) : vrow[i * ld];
-                s = cfmac(vi, y[r], s);
-            }
-        }
-        s.x = group_sum(s.x, G);
-        s.y = group_sum(s.y, G);
-        s = cmul(tk, s);
-#pragma unroll
-        for (int r = RM - 1; r >= 0; --r) {
-            const int i = g + G * r;
-            if (i <= k) break;
-            if (i < n) {
-                const C vi = (i == k + 1) ? mk<R>(R(1), R(0)) : vrow[i * ld];
-                y[r] = cfms(vi, s, y[r]);
-            }
-        }
-    }
-}
-
-// y <- L^{-H} y (backward substitution) on the column segment.
-template <int G, int RM, typename C, typename R>
-__device__ __forceinline__ void seg_trsm_lowerH(const C* L, int ldl, const R* invd, C (&y)[RM], int n, int g) {
-    for (int k = n - 1; k >= 0; --k) {
-        const int owner = k % G, rk = k / G;
-        C xk = seg_get(y, rk);
-        xk = cscale(xk, invd[k]);
-        if (g == owner) seg_set(y, rk, xk);
-        xk = cshfl(xk, owner, G);
-        const C* lrow = L + k;                     // L(k, i) = lrow[i * ldl], i < k
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {               // active rows i < k form a prefix of r
-            const int i = g + G * r;
-            if (i >= k) break;
-            y[r] = cfms(cconj(lrow[i * ldl]), xk, y[r]);
-        }
-    }
-}
-
 // ============================================================================ QL log application
 // Applies one pair's rotation log (ql_chain's format: a header (top, count), then count
 // rotations (c, s) for columns top, top-1, ...; a header with top < 0 ends the log) to

@@ -45,7 +45,7 @@ bool fits(int n, int precision, const Schedule& s) {
         return big_reduce_smem_bytes(n) <= lim && ql_rows_smem_bytes(n) <= lim &&
                ql_chain_smem_bytes(n, s.chain_threads) <= lim;
     }
-    if (reduce_smem_bytes(kReduceFull, n) > lim || back_smem_bytes(n) > lim) return false;
+    if (reduce_smem_bytes(kReduceFull, n) > lim || back_dmma_smem_bytes(n) > lim) return false;
     if (ql_chain_smem_bytes(n, s.chain_threads) > lim) return false;
     if (ql_apply_smem_bytes(n, s.ql_warps) > lim) return false;
     if (n <= 65 && pair_kernels_smem_bytes(n, s.pair_warps) > lim) return false;
@@ -311,25 +311,14 @@ bool sweep(int n, int precision, const TuneRequest& req, Schedule& best, double&
             }
         t_total += bt;
     }
-    // back-transform (restores its input before every run: the kernel overwrites it with X)
+    // back-transform (no choice left to make; restores its input before every run: the kernel overwrites it)
     {
         bench.eig(win);
         cudaMemcpyAsync(bench.Z.p, bench.X.p, 16 * bench.nn * count, cudaMemcpyDeviceToDevice, bench.st);
-        double bt = 1e30;
-        const std::vector<int> lane_opts = n <= 56 ? std::vector<int>{1, 2} : std::vector<int>{base.back_lanes};
-        const std::vector<int> qpass_opts = n <= 56 ? std::vector<int>{2, 1} : std::vector<int>{base.back_qpass};
-        for (int gl : lane_opts)
-            for (int qp : qpass_opts) {
-                Schedule s = win;
-                s.back_lanes = gl;
-                s.back_qpass = qp;
-                const double ms = median_ms([&] {
-                    cudaMemcpyAsync(bench.X.p, bench.Z.p, 16 * bench.nn * count, cudaMemcpyDeviceToDevice, bench.st);
-                    bench.back(s);
-                }, 3, bench.st);
-                if (ms < bt) { bt = ms; win.back_lanes = gl; win.back_qpass = qp; }
-            }
-        t_total += bt;
+        t_total += median_ms([&] {
+            cudaMemcpyAsync(bench.X.p, bench.Z.p, 16 * bench.nn * count, cudaMemcpyDeviceToDevice, bench.st);
+            bench.back(win);
+        }, 3, bench.st);
     }
     // validate the winner against the built-in schedule and against the residual
     const int spot = std::min(count, 8);
@@ -380,8 +369,6 @@ Schedule default_schedule(int n, int precision) {
     s.pair_warps = 2;
     s.col_exact = 1;
     s.back_lanes = 1;
-    // two reflectors per pass measured 7.8 % faster at n = 54 (13.79 -> 12.72 ms per 65,536 pairs)
-    // and 10 % slower at n = 32 (2.01 -> 2.21 ms), where it lifts the kernel from 162 to 254 registers
     s.back_qpass = n > 32 ? 2 : 1;
     s.ql_warps = n <= 32 ? 8 : (n <= 64 ? 4 : 2);
     s.chain_threads = 128;

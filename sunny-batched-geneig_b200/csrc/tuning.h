@@ -25,9 +25,9 @@ struct Schedule {
                                 // CTA size depends on it
     int pair_warps = 2;         // pairs (warps) per CTA of k_potrf_warp / k_hetrd_warp_c64
                                 // (n <= 65): the reference's batches per block
-    int col_exact = 1;          // exact-n column kernels (k_hegst_col, k_back_col) where they exist
-    int back_lanes = 1;         // lanes per column of k_back_col (n <= 56)
-    int back_qpass = 1;         // reflectors per pass of k_back_col's Q application (n <= 56): 1 or 2
+    int col_exact = 1;          // the exact-n k_hegst_col where it exists
+    int back_lanes = 1;         // 1 or 2, kept from earlier tables: no kernel depends on it
+    int back_qpass = 1;         // 1 or 2, likewise
     int reduce_tc = 0;          // n > 84: the triangular stages on the tensor cores (k_reduce_tc, k_back_tc)
     int ql_warps = 4;           // batches_per_block above n = 65, bounded by shared memory; no kernel's shape
                                 // depends on it
@@ -36,8 +36,6 @@ struct Schedule {
         LaunchShape l;
         l.pair_warps = pair_warps;
         l.col_exact = col_exact;
-        l.back_lanes = back_lanes;
-        l.back_qpass = back_qpass;
         l.reduce_tc = reduce_tc;
         return l;
     }
