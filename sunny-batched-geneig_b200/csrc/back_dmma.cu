@@ -75,12 +75,14 @@ __global__ void __launch_bounds__(32 * NT, MINB) k_back_dmma(int mode, int n, in
         const bool cols = n > kSmallMaxN;                         // reflectors along LV's columns
         for (int j = w; j < 8 * NT; j += NT)
             for (int i = lane; i < 8 * NT; i += 32) {
-                double2 v = make_double2(i == j ? 1.0 : 0.0, 0.0);
+                double2* e = LV + i + j * kLd;
                 if (i < n && j < n) {
-                    if (i >= j || !cols) v = LVg[i + static_cast<size_t>(j) * n];
-                    else v = LVg[(j - i - 1) + static_cast<size_t>(n - 1 - i) * n];      // v_i(j)
+                    // (v_i(j) above the diagonal)
+                    cp_async16(e, i >= j || !cols ? LVg + i + static_cast<size_t>(j) * n
+                                                  : LVg + (j - i - 1) + static_cast<size_t>(n - 1 - i) * n);
+                } else {
+                    *e = make_double2(i == j ? 1.0 : 0.0, 0.0);
                 }
-                LV[i + j * kLd] = v;
             }
         for (int i = tid; i < 8 * NT; i += kThreads) tau[i] = i < n ? ws.tau[static_cast<size_t>(n) * b + i] : zero;
     }
@@ -101,6 +103,7 @@ __global__ void __launch_bounds__(32 * NT, MINB) k_back_dmma(int mode, int n, in
             yr[I][q] = v.x;
             yi[I][q] = v.y;
         }
+    cp_async_wait();
     __syncthreads();                                              // every Z is read before any X is stored
     // V(8 I + i, 8 B + k): zero on and above the diagonal of the tile I == B
     auto vat = [&](int I, int B, int i, int k) {

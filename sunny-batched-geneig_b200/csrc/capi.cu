@@ -44,7 +44,7 @@ int supported_max_n(int precision) {
             if (sbg::big_path(n) && need <= lim) best = n;
             continue;
         }
-        size_t need = std::max(sbg::reduce_smem_bytes(sbg::kReduceFull, n), sbg::back_dmma_smem_bytes(n));
+        size_t need = std::max(sbg::reduce_dmma_smem_bytes(n), sbg::back_dmma_smem_bytes(n));
         need = std::max(need, sbg::hetrd_reg_smem_bytes(n));
         need = std::max(need, sbg::ql_apply_smem_bytes(n, 1));
         need = std::max(need, sbg::ql_chain_smem_bytes(n, 32));
@@ -330,7 +330,7 @@ unsigned int sbg_solver_shared_mem_bytes(const sbg_solver* s) {
     if (!s) return 0;
     size_t m = s->n > sbg::kSmallMaxN
                    ? sbg::big_stage_smem_bytes(s->n, s->sched.reduce_tc != 0, s->sched.chain_threads)
-                   : std::max(sbg::reduce_smem_bytes(sbg::kReduceFull, s->n), sbg::back_dmma_smem_bytes(s->n));
+                   : std::max(sbg::reduce_dmma_smem_bytes(s->n), sbg::back_dmma_smem_bytes(s->n));
     if (sbg::mixed_big(s->n, s->precision == SBG_PRECISION_MIXED))
         m = std::max(m, std::max(sbg::hetrd_c64_big_smem_bytes(s->n), sbg::refine_big_smem_bytes()));
     return static_cast<unsigned>(m);
@@ -370,7 +370,7 @@ void geneig_full_n54_batched_launch(const cuDoubleComplex* d_H, const cuDoubleCo
 }
 unsigned int geneig_full_n54_batched_block_dim_x(void) { return sbg::default_schedule(54, SBG_PRECISION_FP64).hetrd_threads; }
 unsigned int geneig_full_n54_batched_shared_mem_bytes(void) {
-    return static_cast<unsigned>(std::max(sbg::reduce_smem_bytes(sbg::kReduceFull, 54), sbg::back_dmma_smem_bytes(54)));
+    return static_cast<unsigned>(std::max(sbg::reduce_dmma_smem_bytes(54), sbg::back_dmma_smem_bytes(54)));
 }
 
 void chol_n54_launch(const cuDoubleComplex* d_S, cuDoubleComplex* d_L, int* d_info, cudaStream_t stream) {
@@ -382,7 +382,7 @@ void chol_n54_launch(const cuDoubleComplex* d_S, cuDoubleComplex* d_L, int* d_in
     }));
 }
 unsigned int chol_n54_block_dim_x(void) { return sbg::default_schedule(54, SBG_PRECISION_FP64).hetrd_threads; }
-unsigned int chol_n54_shared_mem_bytes(void) { return static_cast<unsigned>(sbg::reduce_smem_bytes(sbg::kReduceChol, 54)); }
+unsigned int chol_n54_shared_mem_bytes(void) { return static_cast<unsigned>(sbg::reduce_dmma_smem_bytes(54)); }
 
 void geneig_reduce_n54_launch(const cuDoubleComplex* d_H, const cuDoubleComplex* d_S, cuDoubleComplex* d_M,
                               int* d_info, cudaStream_t stream) {
@@ -394,7 +394,7 @@ void geneig_reduce_n54_launch(const cuDoubleComplex* d_H, const cuDoubleComplex*
     }));
 }
 unsigned int geneig_reduce_n54_block_dim_x(void) { return sbg::default_schedule(54, SBG_PRECISION_FP64).hetrd_threads; }
-unsigned int geneig_reduce_n54_shared_mem_bytes(void) { return static_cast<unsigned>(sbg::reduce_smem_bytes(sbg::kReduceHegst, 54)); }
+unsigned int geneig_reduce_n54_shared_mem_bytes(void) { return static_cast<unsigned>(sbg::reduce_dmma_smem_bytes(54)); }
 
 void geneig_reduce_eig_n54_launch(const cuDoubleComplex* d_H, const cuDoubleComplex* d_S, double* d_W,
                                   cuDoubleComplex* d_V, int* d_info, cudaStream_t stream) {
@@ -411,7 +411,7 @@ void geneig_reduce_eig_n54_launch(const cuDoubleComplex* d_H, const cuDoubleComp
 }
 unsigned int geneig_reduce_eig_n54_block_dim_x(void) { return sbg::default_schedule(54, SBG_PRECISION_FP64).hetrd_threads; }
 unsigned int geneig_reduce_eig_n54_shared_mem_bytes(void) { return geneig_full_n54_batched_shared_mem_bytes(); }
-unsigned int geneig_reduce_eig_n54_chol_smem_bytes(void) { return static_cast<unsigned>(sbg::reduce_smem_bytes(sbg::kReduceFull, 54)); }
+unsigned int geneig_reduce_eig_n54_chol_smem_bytes(void) { return static_cast<unsigned>(sbg::reduce_dmma_smem_bytes(54)); }
 unsigned int geneig_reduce_eig_n54_heev_smem_bytes(void) {
     return static_cast<unsigned>(sbg::ql_apply_smem_bytes(54, sbg::default_schedule(54, SBG_PRECISION_FP64).ql_warps));
 }

@@ -121,6 +121,13 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                  :: "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
 }
 
+// Global -> shared copy of one 16-byte element (cp.async), for layouts a bulk copy cannot write; both
+// addresses 16-byte aligned.  cp_async_wait: every copy this thread issued has landed.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 constexpr uint32_t kMaxPolls = 1u << 24;   // far beyond any real copy; a timeout is reported, not hung on
 
 // Status bits written to the per-pair info word when something other than the

@@ -1,8 +1,8 @@
 // Stage kernels of the batched generalized eigensolve for n <= 84, and the launchers
 // that route larger n to the cluster kernels of bigsolve.cu.
 //
-//   reduce   k_potrf_warp + k_hegst_col (n <= 56) or k_reduce (57..84): B = L L^H and
-//            C = L^{-1} A L^{-H}; L into the workspace, C into the caller's X buffer.
+//   reduce   k_reduce_dmma (reduce_dmma.cu): B = L L^H and C = L^{-1} A L^{-H}; L into the
+//            workspace, C into the caller's X buffer.
 //   hetrd    k_hetrd_reg (hetrd_reg.cu): Householder tridiagonalisation of C, reflectors and
 //            (d, e, tau) into the workspace; the mixed form (n <= 63) runs it in complex64
 //            (k_hetrd_warp_c64).
@@ -19,7 +19,6 @@
 // BLAS2-shaped stages run a warp or a CTA per pair.
 #include "kernels.cuh"
 #include "stages.cuh"
-#include "colsolve.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -32,261 +31,7 @@ namespace {
 
 __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// Shared-memory carve-up of k_reduce.
-struct ReduceSmem {
-    size_t Ls, As, invd, bar, total;
-    __host__ __device__ ReduceSmem(int n) {
-        const size_t ld = static_cast<size_t>(tile_ld(n));
-        size_t o = 0;
-        Ls = o;   o += 16 * ld * n;
-        As = o;   o += 16 * ld * n;
-        invd = o; o += align_up(8 * n, 16);
-        bar = o;  o += 16;
-        total = o;
-    }
-};
-
-
-// Waits for the bulk copies of this CTA; on the (never expected) timeout it flags
-// the pair (every thread that timed out ORs the bit into the pair's info word, when one is
-// given) and waits once more, bounded, so no copy lands after the CTA exits.  The stage then
-// runs on whatever landed; the flag (info > n) makes the back-transform write NaN for the pair
-// and every later stage skip it.
-__device__ inline bool wait_copies(uint64_t* bar, int* info_word) {
-    if (mbar_wait_bounded(bar, 0, kMaxPolls)) return true;
-    if (info_word) atomicOr(info_word, kInfoCopyTimeout);
-    mbar_wait_bounded(bar, 0, kMaxPolls);
-    return false;
-}
-
-// ----------------------------------------------------------------------------- k_reduce
-template <int T, int G, int RM>
-__global__ void __launch_bounds__(T, RM <= 8 ? 2 : 1) k_reduce(int mode, const double2* __restrict__ A,
-                                              const double2* __restrict__ B, int n, int batch,
-                                              Workspace ws, double2* __restrict__ out,
-                                              int* __restrict__ info) {
-    const int b = blockIdx.x;
-    if (b >= batch || !pair_selected(ws, b)) return;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const ReduceSmem lay(n);
-    const int ld = tile_ld(n);
-    double2* Ls = reinterpret_cast<double2*>(smem + lay.Ls);
-    double2* As = reinterpret_cast<double2*>(smem + lay.As);
-    double* invd = reinterpret_cast<double*>(smem + lay.invd);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + lay.bar);
-
-    const int tid = threadIdx.x;
-    const size_t mat = static_cast<size_t>(n) * n;
-    const double2* Ab = A + mat * b;     // A (unused in kReduceChol / kReduceFromLM)
-    const double2* Bb = B + mat * b;     // B, or L in kReduceFromLM
-    const bool need_a = mode != kReduceChol && mode != kReduceFromLM;
-
-    // ---- stage the pair into shared memory: B (lower part of each column) and A
-    if (tid == 0) { mbar_init(bar, 1); fence_mbar_init(); }
-    __syncthreads();
-    if (tid < 32) {
-        if (tid == 0) {
-            uint32_t bytes = static_cast<uint32_t>(16 * (static_cast<size_t>(n) * (n + 1) / 2));
-            if (need_a) bytes += static_cast<uint32_t>(16 * mat);
-            mbar_arrive_expect_tx(bar, bytes);
-        }
-        __syncwarp();
-        for (int j = tid; j < n; j += 32) {
-            bulk_g2s(Ls + j + static_cast<size_t>(j) * ld, Bb + j + static_cast<size_t>(j) * n, 16u * (n - j), bar);
-            if (need_a) bulk_g2s(As + static_cast<size_t>(j) * ld, Ab + static_cast<size_t>(j) * n, 16u * n, bar);
-        }
-    }
-    // the first stage: info[b] is written only at the end (with the timeout bit of thread 0's wait)
-    const int copy_status = wait_copies(bar, nullptr) ? 0 : kInfoCopyTimeout;
-
-    int st = 0;
-    if (mode == kReduceFromLM) {
-        for (int i = tid; i < n; i += T) invd[i] = 1.0 / Ls[i + i * ld].x;
-        __syncthreads();
-    } else {
-        st = potrf_lower(Ls, ld, n, invd);
-    }
-    if (st != 0) {
-        if (tid == 0) info[b] = ((mode == kReduceFull) ? n + st : st) | copy_status;
-        return;
-    }
-    if (mode == kReduceChol) {
-        for (size_t idx = tid; idx < mat; idx += T) {
-            const int j = static_cast<int>(idx / n), i = static_cast<int>(idx - static_cast<size_t>(j) * n);
-            out[mat * b + idx] = (i >= j) ? Ls[i + j * ld] : make_double2(0.0, 0.0);
-        }
-        if (tid == 0) info[b] = copy_status;
-        return;
-    }
-    if (mode != kReduceFromLM) {
-        const int g = tid % G;
-        double2 y[RM];
-        {   // W = L^{-1} A: column j = tid / G, rows g + G r in registers
-            const int j = tid / G;
-            const bool valid = j < n;
-#pragma unroll
-            for (int r = 0; r < RM; ++r) {
-                const int i = g + G * r;
-                y[r] = (valid && i < n) ? As[i + j * ld] : make_double2(0.0, 0.0);
-            }
-            seg_trsm_lower<G, RM>(Ls, ld, invd, y, n, g);
-            if (valid) {
-#pragma unroll
-                for (int r = 0; r < RM; ++r) {
-                    const int i = g + G * r;
-                    if (i < n) As[i + j * ld] = y[r];
-                }
-            }
-        }
-        __syncthreads();
-        {   // C = W L^{-H} (lower part): row i = tid / G, columns g + G r in registers
-            const int i = tid / G;
-            const bool valid = i < n;
-            const int kmax = min(n - 1, (tid | 31) / G);
-#pragma unroll
-            for (int r = 0; r < RM; ++r) {
-                const int kk = g + G * r;
-                y[r] = (valid && kk < n) ? As[i + kk * ld] : make_double2(0.0, 0.0);
-            }
-            seg_trsm_right_lowerH<G, RM>(Ls, ld, invd, y, kmax, valid ? i : -1, g);
-            if (valid) {
-#pragma unroll
-                for (int r = 0; r < RM; ++r) {
-                    const int kk = g + G * r;
-                    if (kk <= i) As[i + kk * ld] = y[r];
-                }
-            }
-        }
-        __syncthreads();
-    }
-    if (mode == kReduceHegst || mode == kReduceFull) {
-        double2* Mg = out + mat * b;
-        for (size_t idx = tid; idx < mat; idx += T) {
-            const int j = static_cast<int>(idx / n), i = static_cast<int>(idx - static_cast<size_t>(j) * n);
-            double2 v = make_double2(0.0, 0.0);
-            if (i >= j) { v = As[i + j * ld]; if (i == j) v.y = 0.0; }
-            if (i >= j || mode == kReduceHegst) Mg[idx] = v;
-        }
-    }
-    if (mode == kReduceFull || mode == kReduceFromLM) {
-        // L into the lower triangle of the pair's LV tile (the reflectors fill the upper part later)
-        double2* LVg = ws.LV + mat * b;
-        for (size_t idx = tid; idx < mat; idx += T) {
-            const int j = static_cast<int>(idx / n), i = static_cast<int>(idx - static_cast<size_t>(j) * n);
-            if (i >= j) LVg[idx] = Ls[i + j * ld];
-        }
-    }
-    if (tid == 0) info[b] = copy_status;
-}
-
-// ----------------------------------------------------------------------------- k_potrf_warp
-// One WARP per pair (n <= 64): B's lower triangle bulk-copied into a packed tile,
-// Cholesky by potrf_warp_packed; L goes to `out` (strict upper zeroed, the staged
-// Cholesky) or to the lower triangle of the pair's LV tile (the full solve).
-__host__ __device__ inline size_t potrf_warp_bytes(int n) {
-    return align_up(16 * static_cast<size_t>(n) * (n + 1) / 2, 16) + align_up(8 * n, 16) + 16;
-}
-constexpr int kMaxPairWarps = 4;      // warp-per-pair kernels: 1, 2 or 4 pairs (warps) per CTA
-constexpr int kColMaxN = 56;      // column-per-thread kernels: y[NMAX] in registers, NMAX in {32, 48, 56}
-
-__global__ void __launch_bounds__(32 * kMaxPairWarps) k_potrf_warp(int mode, const double2* __restrict__ B, int n,
-                                                                      int batch, Workspace ws, double2* __restrict__ out,
-                                                                      int* __restrict__ info) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (b >= batch) return;
-    extern __shared__ __align__(16) unsigned char smem[];
-    unsigned char* base = smem + potrf_warp_bytes(n) * warp;
-    double2* P = reinterpret_cast<double2*>(base);
-    double* invd = reinterpret_cast<double*>(base + align_up(16 * static_cast<size_t>(n) * (n + 1) / 2, 16));
-    uint64_t* bar = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(invd) + align_up(8 * n, 16));
-    const size_t mat = static_cast<size_t>(n) * n;
-    const double2* Bb = B + mat * b;
-    if (lane == 0) { mbar_init(bar, 1); fence_mbar_init(); }
-    __syncwarp();
-    if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(16 * (static_cast<size_t>(n) * (n + 1) / 2)));
-    __syncwarp();
-    for (int j = lane; j < n; j += 32)
-        bulk_g2s(P + pk(j, n), Bb + j + static_cast<size_t>(j) * n, 16u * (n - j), bar);
-    // the first stage: info[b] is written only at the end, with the timeout bit of lane 0's wait
-    const int copy_status = wait_copies(bar, nullptr) ? 0 : kInfoCopyTimeout;
-    const int st = potrf_warp_packed<double>(P, n, invd);
-    if (st != 0) {
-        if (lane == 0) info[b] = ((mode == kReduceFull) ? n + st : st) | copy_status;
-        return;
-    }
-    __syncwarp();
-    double2* dst = (mode == kReduceChol) ? out + mat * b : ws.LV + mat * b;
-    for (int j = 0; j < n; ++j) {
-        const double2* col = P + pk(j, n) - j;     // col[i] = L(i, j), i >= j
-        for (int i = lane; i < n; i += 32) {
-            if (i >= j) dst[i + static_cast<size_t>(j) * n] = col[i];
-            else if (mode == kReduceChol) dst[i + static_cast<size_t>(j) * n] = make_double2(0.0, 0.0);
-        }
-    }
-    if (lane == 0) info[b] = copy_status;
-}
-
-// ----------------------------------------------------------------------------- k_hegst_col
-// One CTA of NMAX threads per pair (n <= NMAX): C = L^{-1} A L^{-H}.  Thread j solves
-// column j of W = L^{-1} A in registers and stores it to the pair's X slice (in L2);
-// after the barrier thread i reads row i of W back and solves row i of C = W L^{-H},
-// columns k <= i, writing C's lower triangle over its own row.  Only the packed L
-// lives in shared memory.  kReduceHegst also zeroes the strict upper triangle.
-__host__ __device__ inline size_t hegst_col_bytes(int n) {
-    return align_up(16 * static_cast<size_t>(n) * (n + 1) / 2, 16) + align_up(8 * n, 16) + 16;
-}
-
-// EXACT: n == NMAX is a compile-time constant (the common sizes get their own
-// instantiation, so every row-bound test folds away).
-template <int NMAX, bool EXACT>
-__global__ void __launch_bounds__(NMAX, 4) k_hegst_col(int mode, const double2* __restrict__ A, const Workspace ws,
-                                                    double2* __restrict__ out, int n_arg, int batch,
-                                                    int* __restrict__ info) {
-    const int n = EXACT ? NMAX : n_arg;
-    const int b = blockIdx.x;
-    if (b >= batch) return;
-    if (info[b] != 0) return;
-    extern __shared__ __align__(16) unsigned char smem[];
-    double2* Lp = reinterpret_cast<double2*>(smem);
-    double* invd = reinterpret_cast<double*>(smem + align_up(16 * static_cast<size_t>(n) * (n + 1) / 2, 16));
-    uint64_t* bar = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(invd) + align_up(8 * n, 16));
-    const int tid = threadIdx.x;
-    const size_t mat = static_cast<size_t>(n) * n;
-    const double2* Lg = ws.LV + mat * b;
-    const double2* Ab = A + mat * b;
-    double2* Ob = out + mat * b;
-    if (tid == 0) { mbar_init(bar, 1); fence_mbar_init(); }
-    __syncthreads();
-    if (tid < 32) {
-        if (tid == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(16 * (static_cast<size_t>(n) * (n + 1) / 2)));
-        __syncwarp();
-        for (int j = tid; j < n; j += 32)
-            bulk_g2s(Lp + pk(j, n), Lg + j + static_cast<size_t>(j) * n, 16u * (n - j), bar);
-    }
-    const bool own = tid < n;
-    double2 y[NMAX];
-#pragma unroll
-    for (int i = 0; i < NMAX; ++i)
-        y[i] = (own && i < n) ? Ab[i + static_cast<size_t>(tid) * n] : make_double2(0.0, 0.0);
-    wait_copies(bar, info + b);
-    for (int i = tid; i < n; i += NMAX) invd[i] = 1.0 / Lp[pk(i, n)].x;
-    __syncthreads();
-    if (own) col_trsm_lower2<NMAX>(Lp, invd, y, n, [&](int k, double2 w) { Ob[k + static_cast<size_t>(tid) * n] = w; });
-    __syncthreads();
-    if (own) {
-        const int i = tid;
-#pragma unroll
-        for (int kk = 0; kk < NMAX; ++kk) y[kk] = (kk <= i) ? Ob[i + static_cast<size_t>(kk) * n] : make_double2(0.0, 0.0);
-        const int kmax = min(n - 1, (tid | 31));            // the warp's largest row: uniform loop bound
-        row_trsm_right_lowerH2<NMAX>(Lp, invd, y, n, i, kmax, [&](int k, double2 c) {
-            if (k == i) c.y = 0.0;
-            Ob[i + static_cast<size_t>(k) * n] = c;
-        });
-        if (mode == kReduceHegst)
-            for (int k = i + 1; k < n; ++k) Ob[i + static_cast<size_t>(k) * n] = make_double2(0.0, 0.0);
-    }
-}
+constexpr int kMaxPairWarps = 4;      // k_hetrd_warp_c64: 1, 2 or 4 pairs (warps) per CTA
 
 // ----------------------------------------------------------------------------- k_hetrd_warp_c64
 // Mixed form, Householder stage in complex64: one WARP per pair (n <= 65).  C's lower triangle
@@ -790,33 +535,7 @@ void set_smem_limit(const void* kernel, SmemOptIn& rec, int bytes) {
     }
 }
 
-size_t reduce_smem_bytes(int, int n) { return ReduceSmem(n).total; }
 size_t invit_smem_bytes(int n, bool with_tile) { return InvitSmem(n, with_tile).per_warp; }
-
-// The register-segment kernels: (threads T, lanes per column G, rows per lane RM) by
-// size: n <= 32 -> (256, 8, 4), n <= 64 -> (512, 8, 8), else (512, 4, 22) (n <= 88).
-#define SBG_DISPATCH_BY_N(n, KERNEL, ...)                                              \
-    do {                                                                               \
-        if ((n) <= 32) { KERNEL<256, 8, 4>(__VA_ARGS__); }                             \
-        else if ((n) <= 64) { KERNEL<512, 8, 8>(__VA_ARGS__); }                        \
-        else { KERNEL<512, 4, 22>(__VA_ARGS__); }                                      \
-    } while (0)
-
-template <int T, int G, int RM>
-void run_reduce(int mode, const double2* A, const double2* B, int n, int batch, const Workspace& ws, double2* out,
-                int* info, size_t smem, cudaStream_t stream) {
-    static SmemOptIn f;
-    set_max_smem_once(k_reduce<T, G, RM>, f);
-    k_reduce<T, G, RM><<<batch, T, smem, stream>>>(mode, A, B, n, batch, ws, out, info);
-}
-
-template <int NMAX, bool EXACT = false>
-void run_hegst_col(int mode, const double2* A, const Workspace& ws, double2* out, int n, int batch, int* info,
-                   cudaStream_t stream) {
-    static SmemOptIn f;
-    set_max_smem_once(k_hegst_col<NMAX, EXACT>, f);
-    k_hegst_col<NMAX, EXACT><<<batch, NMAX, hegst_col_bytes(n), stream>>>(mode, A, ws, out, n, batch, info);
-}
 
 cudaError_t launch_reduce(int mode, const double2* A, const double2* B, int n, int batch,
                           const Workspace& ws, double2* out, int* info, const LaunchShape& shape, cudaStream_t stream) {
@@ -825,42 +544,15 @@ cudaError_t launch_reduce(int mode, const double2* A, const double2* B, int n, i
     // (below it the reduction never tridiagonalises)
     const bool hegst_only = mode == kReduceMixed;
     if (hegst_only) mode = kReduceFull;
-    if (!B || !info) return cudaErrorInvalidValue;
-    if ((mode == kReduceChol || mode == kReduceHegst || mode == kReduceFull) && !out) return cudaErrorInvalidValue;
-    if ((mode == kReduceHegst || mode == kReduceFull) && !A) return cudaErrorInvalidValue;
-    if ((mode == kReduceFull || mode == kReduceFromLM) && !ws.LV) return cudaErrorInvalidValue;
-    if (n > kSmallMaxN) {
-        if (mode != kReduceFull) return cudaErrorInvalidValue;
-        if (shape.reduce_tc) {                       // tensor-core Cholesky + reduction, then the Householder
-            cudaError_t err = launch_reduce_tc(A, B, n, batch, ws, out, info, stream);
-            if (err != cudaSuccess || hegst_only) return err;
-            return launch_reduce_big(A, B, n, batch, ws, out, info, stream, kBigHetrdOnly);
-        }
+    if (n <= kSmallMaxN) return launch_reduce_dmma(mode, A, B, n, batch, ws, out, info, stream);
+    if (mode != kReduceFull) return cudaErrorInvalidValue;
+    if (!shape.reduce_tc)
         return launch_reduce_big(A, B, n, batch, ws, out, info, stream, hegst_only ? kBigHegstOnly : kBigFull);
-    }
-    // The two-kernel path hands L from k_potrf_warp to k_hegst_col through ws.LV, so it
-    // needs a workspace (the staged Cholesky alone does not).
-    if (n <= kColMaxN && mode != kReduceFromLM && (mode == kReduceChol || ws.LV != nullptr)) {
-        const int pw = pair_warps_of(shape);
-        static SmemOptIn fp;
-        set_max_smem_once(k_potrf_warp, fp);
-        const int grid = (batch + pw - 1) / pw;
-        k_potrf_warp<<<grid, 32 * pw, potrf_warp_bytes(n) * pw, stream>>>(mode, B, n, batch, ws, out, info);
-        if (mode == kReduceChol) return cudaGetLastError();
-        if (n == 32 && shape.col_exact) run_hegst_col<32, true>(mode, A, ws, out, n, batch, info, stream);
-        else if (n == 54 && shape.col_exact) run_hegst_col<54, true>(mode, A, ws, out, n, batch, info, stream);
-        else if (n <= 32) run_hegst_col<32>(mode, A, ws, out, n, batch, info, stream);
-        else if (n <= 48) run_hegst_col<48>(mode, A, ws, out, n, batch, info, stream);
-        else run_hegst_col<56>(mode, A, ws, out, n, batch, info, stream);
-        return cudaGetLastError();
-    }
-    // 57 <= n <= 84 with the tensor-core triangular stages: the blocked Cholesky and reduction
-    // (the Householder is a separate kernel here anyway)
-    if (shape.reduce_tc && mode == kReduceFull) return launch_reduce_tc(A, B, n, batch, ws, out, info, stream);
-    const size_t smem = reduce_smem_bytes(mode, n);
-    if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
-    SBG_DISPATCH_BY_N(n, run_reduce, mode, A, B, n, batch, ws, out, info, smem, stream);
-    return cudaGetLastError();
+    // tensor-core Cholesky + reduction, then the Householder
+    const cudaError_t err = n <= kReduceDmmaMaxN ? launch_reduce_dmma(mode, A, B, n, batch, ws, out, info, stream)
+                                                 : launch_reduce_tc(A, B, n, batch, ws, out, info, stream);
+    if (err != cudaSuccess || hegst_only) return err;
+    return launch_reduce_big(A, B, n, batch, ws, out, info, stream, kBigHetrdOnly);
 }
 
 cudaError_t launch_hetrd(int n, int batch, const double2* C, const Workspace& ws, int* info, cudaStream_t stream) {
@@ -912,8 +604,7 @@ cudaError_t launch_eig(int n, int batch, const Workspace& ws, double* W, double2
 size_t hetrd_c64_smem_bytes(int n) { return hetrd_c64_bytes(n) * kMaxPairWarps; }
 
 size_t pair_kernels_smem_bytes(int n, int pair_warps) {
-    const size_t per = std::max(potrf_warp_bytes(n), hetrd_c64_bytes(n));
-    return per * static_cast<size_t>(pair_warps);
+    return hetrd_c64_bytes(n) * static_cast<size_t>(pair_warps);
 }
 
 cudaError_t launch_hetrd_c64(int n, int batch, const double2* C, const Workspace& ws, int* info,

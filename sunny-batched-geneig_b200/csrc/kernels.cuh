@@ -123,18 +123,14 @@ enum BackMode : int {
 };
 
 // Launch shape of the stage kernels, the part of a schedule the autotuner varies:
-//   pair_warps  pairs (one warp each) per CTA of k_potrf_warp, k_hetrd_warp_c64 (n <= 65): 1, 2 or
-//               4 -- the reference's "batches per block"
-//   col_exact   k_hegst_col: the exact-n instantiation where one exists (n = 32, 54) instead of the one
-//               for the next larger NMAX
-//   reduce_tc   n > 56: the triangular stages on the FP64 tensor cores -- Cholesky and reduction by
-//               the blocked kernel k_reduce_tc (above kSmallMaxN, FP64 form, then the Householder
-//               alone by k_hetrd_reg or k_hetrd_l2 instead of k_reduce_mid / k_reduce_big doing all three), and
-//               above kSmallMaxN the back-transform by k_back_dmma or k_back_q_tc + k_back_tc instead of
-//               k_back_big
+//   pair_warps  pairs (one warp each) per CTA of k_hetrd_warp_c64 (the mixed form, n <= 63): 1, 2 or 4
+//               -- the reference's "batches per block"
+//   reduce_tc   n > 84: the triangular stages on the FP64 tensor cores (k_reduce_dmma or k_reduce_tc,
+//               then the Householder alone by k_hetrd_reg or k_hetrd_l2; the back-transform by
+//               k_back_dmma or k_back_q_tc + k_back_tc) instead of k_reduce_mid / k_reduce_big doing all
+//               three and k_back_big.  Up to n = 84 there is no other.
 struct LaunchShape {
     int pair_warps = 2;
-    int col_exact = 1;
     int reduce_tc = 0;
 };
 
@@ -169,7 +165,7 @@ cudaError_t launch_refine_mixed(int n, int batch, const Workspace& ws, double* W
 cudaError_t launch_eig_mixed(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                              int refine_steps, const LaunchShape& shape, cudaStream_t stream);
 size_t hetrd_c64_smem_bytes(int n);
-// Dynamic shared memory of a CTA of the warp-per-pair kernels (k_potrf_warp, k_hetrd_warp_c64) with pair_warps pairs.
+// Dynamic shared memory of a CTA of k_hetrd_warp_c64 with pair_warps pairs.
 size_t pair_kernels_smem_bytes(int n, int pair_warps);
 size_t refine_c_smem_bytes(int n);
 size_t mixed_fallback_smem_bytes(int n);
@@ -181,6 +177,12 @@ cudaError_t launch_pull_pairs(const double2* src, double2* dst, int count, int n
 cudaError_t launch_back(int mode, int n, int batch, const Workspace& ws, double2* X, int* info,
                         const LaunchShape& shape, cudaStream_t stream);
 
+// Cholesky and reduction of n <= kReduceDmmaMaxN on the FP64 tensor cores (csrc/reduce_dmma.cu), every
+// mode (kReduceMixed as kReduceFull).  Uses the pair's rotation-log region as scratch.  Honours the pair
+// selection.
+constexpr int kReduceDmmaMaxN = 144;
+cudaError_t launch_reduce_dmma(int mode, const double2* A, const double2* B, int n, int batch, const Workspace& ws,
+                               double2* out, int* info, cudaStream_t stream);
 // The back-transform of n <= kBackDmmaMaxN on the FP64 tensor cores (csrc/back_dmma.cu), every mode;
 // reflectors along LV's rows up to kSmallMaxN, its columns above.  Honours the pair selection.
 constexpr int kBackDmmaMaxN = 96;
@@ -251,11 +253,10 @@ cudaError_t launch_back_big(int mode, int n, int batch, const Workspace& ws, dou
 cudaError_t launch_ql_chain(int n, int batch, const Workspace& ws, double* W, int* info, int chain_threads,
                             cudaStream_t stream);
 
-// Kernels one full reduce launch (kReduceFull) issues for order n: the warp Cholesky and the
-// column hegst kernel for n <= 56; above kSmallMaxN with the tensor-core reduction (tc), k_reduce_tc
-// and the Householder kernel; one kernel otherwise.
-inline int reduce_kernel_count(int n, bool tc = false) { return n <= 56 || (n > kSmallMaxN && tc) ? 2 : 1; }
-// (57 <= n <= 84 with tc: k_reduce_tc alone, the Householder being its own stage there.)
+// Kernels one full reduce launch (kReduceFull) issues for order n: the reduction and, above kSmallMaxN
+// with the tensor-core reduction (tc), the Householder kernel.
+inline int reduce_kernel_count(int n, bool tc = false) { return n > kSmallMaxN && tc ? 2 : 1; }
+
 // ---- Eigensolve of the tridiagonals, FP64: eigenvalues by bisection (k_tridiag_values), eigenvectors by
 // inverse iteration (k_tridiag_invit), orthonormalised together where many eigenvalues are close
 // (k_tridiag_ortho).  A pair these cannot take (vectors of one eigenspace, a T that is not finite) goes
@@ -282,7 +283,7 @@ size_t tridiag_ortho_smem_bytes(int n, bool with_ql);
 cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                              bool flag_redo, cudaStream_t stream);
 
-size_t reduce_smem_bytes(int mode, int n);
+size_t reduce_dmma_smem_bytes(int n);
 size_t ql_chain_smem_bytes(int n, int threads);
 // The bound on ql_warps (pairs per CTA): each pair's Z tile, log stage and T in shared memory.
 size_t ql_apply_smem_bytes(int n, int pairs_per_cta);

@@ -15,52 +15,6 @@
 
 namespace sbg {
 
-// ============================================================================ potrf
-// In-place lower Cholesky of the tile L (only the lower triangle is read, as
-// zpotrf 'L'). Right-looking, one CTA barrier per column: in phase k every
-// thread updates the trailing lower triangle with the unscaled column k divided
-// by L_kk, and the scaling of column k itself is deferred to phase k+1, when no
-// thread reads it any more.  invd[k] receives 1 / L_kk.
-// Returns 0, or k+1 for the first leading minor that is not positive definite
-// (also for NaN), the zpotrf convention.  Reference: Cholesky54, geneig_fixed.cu:17-26.
-template <typename R>
-__device__ int potrf_lower(cplx<R>* L, int ld, int n, R* invd) {
-    using C = cplx<R>;
-    const int tid = threadIdx.x, T = blockDim.x;
-    R pd = R(0), pinv = R(0);
-    for (int k = 0; k < n; ++k) {
-        const R dkk = L[k + k * ld].x;
-        if (!(dkk > R(0))) return k + 1;           // uniform: every thread reads the same word
-        const R d = sqrt(dkk);
-        const R inv = R(1) / d;
-        const R invdd = inv * inv;
-        if (k > 0) {                                // deferred scaling of column k-1
-            for (int i = k + tid; i < n; i += T) L[i + (k - 1) * ld] = cscale(L[i + (k - 1) * ld], pinv);
-            if (tid == 0) L[(k - 1) + (k - 1) * ld] = mk<R>(pd, R(0));
-        }
-        if (tid == 0) invd[k] = inv;
-        const int m = n - k - 1;
-        const C* colk = L + k * ld;
-        // thread (row r, column chunk c) updates L(k+1+r, k+1+j) for j in its chunk, j <= r
-        const int chunks = max(1, T / max(m, 1));
-        const int cw = (m + chunks - 1) / chunks;
-        for (int t = tid; t < m * chunks; t += T) {
-            const int r = t % m, c = t / m;
-            const int i = k + 1 + r;
-            const C lik = cscale(colk[i], invdd);
-            const int j1 = min(r + 1, (c + 1) * cw);
-            C* Li = L + i + (k + 1) * ld;
-            for (int jj = c * cw; jj < j1; ++jj)
-                Li[jj * ld] = cfmsc(lik, colk[k + 1 + jj], Li[jj * ld]);
-        }
-        __syncthreads();
-        pd = d; pinv = inv;
-    }
-    if (tid == 0) L[(n - 1) + (n - 1) * ld] = mk<R>(pd, R(0));
-    __syncthreads();
-    return 0;
-}
-
 // ============================================================================ hetrd (lower)
 // Householder reduction of the Hermitian tile A (lower triangle valid) to real
 // symmetric tridiagonal form T = Q^H A Q, Q = H_0 H_1 ... H_{n-2},
@@ -409,45 +363,6 @@ template <int RM, typename C>
 __device__ __forceinline__ void seg_set(C (&seg)[RM], int r, C v) {
 #pragma unroll
     for (int q = 0; q < RM; ++q) if (q == r) seg[q] = v;
-}
-
-// y <- L^{-1} y (forward substitution) on the column segment; L column-major in smem.
-template <int G, int RM, typename C, typename R>
-__device__ __forceinline__ void seg_trsm_lower(const C* L, int ldl, const R* invd, C (&y)[RM], int n, int g) {
-    for (int k = 0; k < n; ++k) {
-        const int owner = k % G, rk = k / G;
-        C wk = seg_get(y, rk);
-        wk = cscale(wk, invd[k]);
-        if (g == owner) seg_set(y, rk, wk);
-        wk = cshfl(wk, owner, G);
-        const C* lk = L + k * ldl;
-#pragma unroll
-        for (int r = RM - 1; r >= 0; --r) {          // active rows i > k form a suffix of r
-            const int i = g + G * r;
-            if (i <= k) break;
-            if (i < n) y[r] = cfms(lk[i], wk, y[r]);
-        }
-    }
-}
-
-// Row segment of W (columns kk = g + G r of row i) <- W L^{-H}, only kk <= i formed.
-template <int G, int RM, typename C, typename R>
-__device__ __forceinline__ void seg_trsm_right_lowerH(const C* L, int ldl, const R* invd, C (&y)[RM], int kmax,
-                                                      int i, int g) {
-    for (int k = 0; k <= kmax; ++k) {
-        const int owner = k % G, rk = k / G;
-        C ck = seg_get(y, rk);
-        ck = cscale(ck, invd[k]);
-        if (g == owner && k <= i) seg_set(y, rk, ck);
-        ck = cshfl(ck, owner, G);
-        const C* lk = L + k * ldl;
-#pragma unroll
-        for (int r = RM - 1; r >= 0; --r) {          // active columns k < kk <= i
-            const int kk = g + G * r;
-            if (kk <= k) break;
-            if (kk <= i) y[r] = cfmsc(ck, lk[kk], y[r]);
-        }
-    }
 }
 
 // ============================================================================ QL log application

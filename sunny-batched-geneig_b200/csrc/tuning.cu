@@ -45,7 +45,7 @@ bool fits(int n, int precision, const Schedule& s) {
         return big_reduce_smem_bytes(n) <= lim && ql_rows_smem_bytes(n) <= lim &&
                ql_chain_smem_bytes(n, s.chain_threads) <= lim;
     }
-    if (reduce_smem_bytes(kReduceFull, n) > lim || back_dmma_smem_bytes(n) > lim) return false;
+    if (reduce_dmma_smem_bytes(n) > lim || back_dmma_smem_bytes(n) > lim) return false;
     if (ql_chain_smem_bytes(n, s.chain_threads) > lim) return false;
     if (ql_apply_smem_bytes(n, s.ql_warps) > lim) return false;
     if (n <= 65 && pair_kernels_smem_bytes(n, s.pair_warps) > lim) return false;
@@ -270,28 +270,22 @@ bool sweep(int n, int precision, const TuneRequest& req, Schedule& best, double&
     // sweep over {16, 8, 4, 2, 1}); here at most 4 warps share a CTA
     const std::vector<int> bpb_opts = req.force_bpb && n <= 65 ? std::vector<int>{req.force_bpb}
                                       : n <= 65 ? std::vector<int>{1, 2, 4} : std::vector<int>{base.pair_warps};
-    const std::vector<int> exact_opts = (n == 32 || n == 54) ? std::vector<int>{1, 0} : std::vector<int>{base.col_exact};
-    const std::vector<int> thread_opts = req.force_threads ? std::vector<int>{req.force_threads}
-                                                           : std::vector<int>{base.hetrd_threads};
     // ql_warps shapes no kernel (the eigenvectors come from inverse iteration): kept as asked or built in
     const std::vector<int> warp_opts = req.force_bpb && n > 65 ? std::vector<int>{req.force_bpb}
                                                                : std::vector<int>{base.ql_warps};
     Schedule win = base;
+    if (req.force_threads) win.hetrd_threads = req.force_threads;
     double t_total = 0.0;
-    // reduction + tridiagonalisation together (pair_warps is shared by their warp-per-pair kernels)
+    // reduction + tridiagonalisation together
     {
         double bt = 1e30;
-        for (int pw : bpb_opts)
-            for (int ex : exact_opts)
-                for (int t : thread_opts) {
-                    Schedule s = win;
-                    s.pair_warps = pw;
-                    s.col_exact = ex;
-                    s.hetrd_threads = t;
-                    if (!fits(n, precision, s)) continue;
-                    const double ms = median_ms([&] { bench.reduce(s); bench.tridiag(s); }, 3, bench.st);
-                    if (ms < bt) { bt = ms; win.pair_warps = pw; win.col_exact = ex; win.hetrd_threads = t; }
-                }
+        for (int pw : bpb_opts) {
+            Schedule s = win;
+            s.pair_warps = pw;
+            if (!fits(n, precision, s)) continue;
+            const double ms = median_ms([&] { bench.reduce(s); bench.tridiag(s); }, 3, bench.st);
+            if (ms < bt) { bt = ms; win.pair_warps = pw; }
+        }
         t_total += bt;
         bench.reduce(win);
         bench.tridiag(win);
@@ -372,8 +366,8 @@ Schedule default_schedule(int n, int precision) {
     s.back_qpass = n > 32 ? 2 : 1;
     s.ql_warps = n <= 32 ? 8 : (n <= 64 ? 4 : 2);
     s.chain_threads = 128;
-    // above n = 56 the triangular stages on the tensor cores: the whole solve measured 1.14x (n = 58)
-    // to 1.59x (n = 192) faster than with the scalar CTA-per-pair and cluster kernels
+    // the triangular stages on the tensor cores (above n = 84 there are scalar kernels too, 4.4x slower at
+    // n = 192); the field says so above n = 56, as earlier tables do
     s.reduce_tc = n > 56 ? 1 : 0;
     while (s.chain_threads > 32 && !fits(n, precision, s)) s.chain_threads /= 2;
     while (s.ql_warps > 1 && !fits(n, precision, s)) s.ql_warps /= 2;

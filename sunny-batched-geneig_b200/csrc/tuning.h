@@ -23,9 +23,9 @@ namespace sbg {
 struct Schedule {
     int hetrd_threads = 256;    // what block_dim_x reports and force_block_dim_x sets (128 or 256); no kernel's
                                 // CTA size depends on it
-    int pair_warps = 2;         // pairs (warps) per CTA of k_potrf_warp / k_hetrd_warp_c64
+    int pair_warps = 2;         // pairs (warps) per CTA of k_hetrd_warp_c64
                                 // (n <= 65): the reference's batches per block
-    int col_exact = 1;          // the exact-n k_hegst_col where it exists
+    int col_exact = 1;          // 0 or 1, kept from earlier tables: no kernel depends on it
     int back_lanes = 1;         // 1 or 2, kept from earlier tables: no kernel depends on it
     int back_qpass = 1;         // 1 or 2, likewise
     int reduce_tc = 0;          // n > 84: the triangular stages on the tensor cores (k_reduce_tc, k_back_tc)
@@ -35,7 +35,6 @@ struct Schedule {
     LaunchShape shape() const {
         LaunchShape l;
         l.pair_warps = pair_warps;
-        l.col_exact = col_exact;
         l.reduce_tc = reduce_tc;
         return l;
     }
