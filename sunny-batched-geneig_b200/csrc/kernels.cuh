@@ -126,7 +126,7 @@ enum BackMode : int {
 //   pair_warps  pairs (one warp each) per CTA of k_hetrd_warp_c64 (the mixed form, n <= 63): 1, 2 or 4
 //               -- the reference's "batches per block"
 //   reduce_tc   n > 84: the triangular stages on the FP64 tensor cores (k_reduce_dmma or k_reduce_tc,
-//               then the Householder alone by k_hetrd_reg or k_hetrd_l2; the back-transform by
+//               then the Householder alone by k_hetrd_reg or k_hetrd_tri; the back-transform by
 //               k_back_dmma or k_back_q_tc + k_back_tc) instead of k_reduce_mid / k_reduce_big doing all
 //               three and k_back_big.  Up to n = 84 there is no other.
 struct LaunchShape {
@@ -204,7 +204,7 @@ size_t ql_rows_smem_bytes(int n);
 size_t big_stage_smem_bytes(int n, bool tc, int chain_threads);
 // mode: kBigFull (Cholesky, reduction, Householder: k_reduce_mid / k_reduce_big), kBigHegstOnly (the
 // same kernels, stopping after C = L^{-1} A L^{-H}: C's lower triangle in X, L in LV) or kBigHetrdOnly
-// (the Householder alone by k_hetrd_reg or k_hetrd_l2, from C's lower triangle in X with L already in LV, as
+// (the Householder alone by k_hetrd_reg or k_hetrd_tri, from C's lower triangle in X with L already in LV, as
 // k_reduce_tc leaves them; pairs with info != 0 are skipped).
 enum BigReduceMode : int { kBigFull = 0, kBigHegstOnly = 1, kBigHetrdOnly = 2 };
 cudaError_t launch_reduce_big(const double2* A, const double2* B, int n, int batch, const Workspace& ws, double2* X,
@@ -219,11 +219,12 @@ cudaError_t launch_reduce_big(const double2* A, const double2* B, int n, int bat
 //                          cores; ws.rstat gets each pair's outcome.
 cudaError_t launch_hetrd_c64_big(int n, int batch, const double2* C, const Workspace& ws, int* info,
                                  cudaStream_t stream);
-// The FP64 Householder alone for n > kHetrdRegMaxN after launch_reduce_tc (C's lower triangle in X),
-// one CTA per pair with the packed triangle in the pair's rotation-log region (L2-resident global
-// memory): reflectors to LV's columns, d, e, tau; pairs with info != 0 are skipped.
-cudaError_t launch_hetrd_l2(int n, int batch, const double2* C, const Workspace& ws, int* info,
-                           cudaStream_t stream);
+// The FP64 Householder alone for n > kHetrdRegMaxN (csrc/hetrd_tri.cu), one CTA per pair, C's packed
+// triangle in shared memory and, its first columns, the pair's rotation-log region: reflectors to LV's
+// columns, d, e, tau; pairs with info != 0 are skipped.  Honours the pair selection.
+cudaError_t launch_hetrd_tri(int n, int batch, const double2* C, const Workspace& ws, const int* info,
+                             cudaStream_t stream);
+size_t hetrd_tri_smem_bytes(int n);
 // Blocked FP64 Cholesky and reduction on the FP64 tensor cores (csrc/reduce_tc.cu), one CTA per
 // pair: L into LV's lower triangle, C = L^{-1} A L^{-H} (lower triangle) into X, info as the other
 // reduce kernels (n + i for a leading minor i that is not positive definite).  Uses the pair's
