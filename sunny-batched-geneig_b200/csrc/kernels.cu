@@ -667,6 +667,7 @@ cudaError_t launch_back(int mode, int n, int batch, const Workspace& ws, double2
     if (n <= kSmallMaxN || (n <= kBackDmmaMaxN && shape.reduce_tc))
         return launch_back_dmma(mode, n, batch, ws, X, info, stream);
     if (!shape.reduce_tc) return launch_back_big(mode, n, batch, ws, X, info, stream);
+    if (n <= kBackStreamMaxN) return launch_back_stream(mode, n, batch, ws, X, info, stream);
     if (mode != kBackLOnly) {                           // Q Z and L^{-H} as products through L2
         const cudaError_t err = launch_back_q_tc(n, batch, ws, X, info, stream);
         if (err != cudaSuccess || mode == kBackQOnly) return err;

@@ -189,6 +189,12 @@ constexpr int kBackDmmaMaxN = 96;
 cudaError_t launch_back_dmma(int mode, int n, int batch, const Workspace& ws, double2* X, const int* info,
                              cudaStream_t stream);
 
+// The same for kBackDmmaMaxN < n <= kBackStreamMaxN (reflectors along LV's columns), V and L streamed
+// through shared memory.  Uses the pair's rotation-log region as scratch.  Honours the pair selection.
+constexpr int kBackStreamMaxN = 192;
+cudaError_t launch_back_stream(int mode, int n, int batch, const Workspace& ws, double2* X, const int* info,
+                               cudaStream_t stream);
+
 // Pairs with n <= kSmallMaxN are solved by CTA-per-pair (or warp-per-pair) stage kernels;
 // kSmallMaxN < n <= kBigMaxN by the cluster kernels of bigsolve.cu.  For those the reduce
 // launch (kReduceFull only) also tridiagonalises, so launch_hetrd has nothing left to do,

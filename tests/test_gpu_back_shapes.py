@@ -19,8 +19,12 @@ pytestmark = pytest.mark.gpu
 EDGES = sorted({8 * t + r for t in range(0, 13) for r in (0, 1)} | set(range(49, 57)) | {7, 87, 95}) [1:]
 
 
+# the streamed form: its tile counts (two apart), a last tile of one row, one and two passes over the panels
+STREAM = (98, 104, 105, 112, 113, 127, 136, 143, 153, 168, 177, 185, 191, 192, 193)
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-@pytest.mark.parametrize("n", EDGES)
+@pytest.mark.parametrize("n", EDGES + list(STREAM))
 def test_every_tile_count(oracle_mod, n, precision):
     rng = np.random.default_rng(500 + n)
     ps = [pair(rng, n) for _ in range(3)]
