@@ -11,9 +11,10 @@
 // product form p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2} (no division: three FP64 operations and
 // one broadcast load of (d_i, e_{i-1}^2) a row), rescaled by powers of two every eight rows; its
 // count is exact for a T whose entries are perturbed by a few eps each, so the eigenvalues carry an
-// error of a few eps ||T||, as QL's.  Whole solves, QL -> bisection (FP64 form): 8 pairs of n = 54
-// 1,421 -> 628 us, 1,024 pairs 1,955 -> 944 us, 32,768 pairs 30.4 -> 28.3 ms; 2,048 pairs of n = 128
-// 30.4 -> 21.1 ms; 65,536 pairs of n = 32, which fill the GPU with either, 12.64 -> 12.63 ms.
+// error of a few eps ||T||, as QL's.  Once an eigenvalue is alone in its bracket, the recurrence's last
+// value (the characteristic polynomial) places the next shift.  Kernel time, QL -> halving only -> now: 8 pairs of n = 54
+// 846 -> 69 -> 46 us, 32,768 pairs 4.0 -> 1.95 -> 1.3 ms, 65,536 of n = 32 1.18 -> 1.2 -> 0.84 ms, 2,048 of n = 128
+// 9.9 -> 0.65 -> 0.37 ms.  Issue-bound when the GPU is full (FP64, sign and load instructions in equal parts).
 //
 // k_tridiag_ortho: pairs with many eigenvalues closer than inverse iteration can keep orthogonal by
 // itself (near a Goldstone point one huge eigenvalue makes all others a cluster) get their vectors Z
@@ -39,31 +40,42 @@ constexpr double kPadD = 8.0;               // padding rows: d - x > 0, no sign 
 constexpr double kMinE2 = 1e-40;
 
 struct ValuesSmem {
-    size_t de, lam, cnt, ql, red, total;
+    size_t de, lam, p, cnt, red, total;
     __host__ __device__ ValuesSmem(int n, int points) {
         const size_t rows = static_cast<size_t>((n + kRows - 1) / kRows * kRows);
         size_t o = 0;
         de = o;  o += 16 * rows;
         lam = o; o += 8 * ((static_cast<size_t>(n) + 1) & ~size_t(1));
-        cnt = o; o += 4 * static_cast<size_t>(points);
+        p = o;   o += 8 * static_cast<size_t>(points);
+        cnt = o; o += 8 * static_cast<size_t>(points);
         red = o; o += 16 * 8;
         total = o;
     }
 };
 
-// Number of eigenvalues of T below x[s], s < NE.
+// Number of eigenvalues of T below x[s], s < NE, and det(T - x[s] I) up to sign and one common factor as
+// p[s] 2^e[s].
 template <int NE>
-__device__ __forceinline__ void sturm(const double2* __restrict__ de, int rows, const double (&x)[NE], int (&cnt)[NE]) {
-    double p[NE], pm[NE];
+__device__ __forceinline__ void sturm(const double2* __restrict__ de, int rows, const double (&x)[NE], int (&cnt)[NE],
+                                      double (&p)[NE], int (&e)[NE]) {
+    double pm[NE];
 #pragma unroll
-    for (int s = 0; s < NE; ++s) { p[s] = 1.0; pm[s] = 0.0; cnt[s] = 0; }
+    for (int s = 0; s < NE; ++s) { p[s] = 1.0; pm[s] = 0.0; cnt[s] = 0; e[s] = 0; }
+    double2 next[kRows];
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) next[u] = de[u];
     for (int i0 = 0; i0 < rows; i0 += kRows) {
+        double2 r[kRows];
+#pragma unroll
+        for (int u = 0; u < kRows; ++u) r[u] = next[u];
+        const int i1 = i0 + kRows < rows ? i0 + kRows : 0;        // the next block, in flight meanwhile
+#pragma unroll
+        for (int u = 0; u < kRows; ++u) next[u] = de[i1 + u];
 #pragma unroll
         for (int u = 0; u < kRows; ++u) {
-            const double2 r = de[i0 + u];
 #pragma unroll
             for (int s = 0; s < NE; ++s) {
-                const double pn = fma(r.x - x[s], p[s], -(r.y * pm[s]));
+                const double pn = fma(r[u].x - x[s], p[s], -(r[u].y * pm[s]));
                 cnt[s] += static_cast<unsigned>(__double2hiint(pn) ^ __double2hiint(p[s])) >> 31;
                 pm[s] = p[s];
                 p[s] = pn;
@@ -75,8 +87,21 @@ __device__ __forceinline__ void sturm(const double2* __restrict__ de, int rows, 
             const double f = __hiloint2double(0x7fe00000 - ex, 0);
             p[s] *= f;
             pm[s] *= f;
+            e[s] += ex >> 20;
         }
     }
+}
+
+// One end of an eigenvalue's bracket: the shift, the count there, and det(T - x I) = p 2^e (none at the
+// ends of the Gershgorin interval: p is NaN).
+struct End {
+    double x, p;
+    int c, e;
+};
+
+// 2^k, for k clamped to the normal range.
+__device__ __forceinline__ double pow2_clamped(int k) {
+    return __hiloint2double((min(max(k, -1000), 1000) + 1023) << 20, 0);
 }
 
 // One pair per CTA of ceil(n / (32 NE)) warps; thread t holds the eigenvalues of index t + T s.
@@ -92,7 +117,8 @@ __global__ void __launch_bounds__(128) k_tridiag_values(int n, int batch, Worksp
     const ValuesSmem lay(n, points);
     double2* de = reinterpret_cast<double2*>(smem + lay.de);
     double* lam = reinterpret_cast<double*>(smem + lay.lam);
-    int* cnt = reinterpret_cast<int*>(smem + lay.cnt);
+    double* gp = reinterpret_cast<double*>(smem + lay.p);
+    int2* cnt = reinterpret_cast<int2*>(smem + lay.cnt);
     double* red = reinterpret_cast<double*>(smem + lay.red);
     const double* dg = ws.d + static_cast<size_t>(n) * b;
     const double* eg = ws.e + static_cast<size_t>(n) * b;
@@ -167,40 +193,85 @@ __global__ void __launch_bounds__(128) k_tridiag_values(int n, int batch, Worksp
     const double w0 = (gu - gl) / (points + 1);
     __syncthreads();
     // ---- counts on a grid of `points` shifts bracket every eigenvalue to one cell
-    double x[NE];
-    int c[NE];
+    double x[NE], px[NE];
+    int c[NE], ex[NE];
 #pragma unroll
     for (int s = 0; s < NE; ++s) x[s] = fma(static_cast<double>(tid * NE + s + 1), w0, gl);
-    sturm<NE>(de, rows, x, c);
+    sturm<NE>(de, rows, x, c, px, ex);
 #pragma unroll
-    for (int s = 0; s < NE; ++s) cnt[tid * NE + s] = c[s];
+    for (int s = 0; s < NE; ++s) {
+        gp[tid * NE + s] = px[s];
+        cnt[tid * NE + s] = make_int2(c[s], ex[s]);
+    }
     __syncthreads();
-    double lo[NE];
+    // ---- then every cell down to the spacing of the numbers at it (eps ||T|| and no less): halved while it
+    // holds more than one eigenvalue, and else by the zero of the chord through det(T - x I) at its ends
+    // (regula falsi with Anderson & Bjorck's reduction of an end that stays): 14 to 23 counts in all for the
+    // slowest eigenvalue of a warp where halving takes 49.  The counts alone decide which end moves; a step
+    // that is too close to an end is moved off it by that spacing, so that the other end follows, and a
+    // cell that three steps did not halve is halved (two: 28 to 32 counts; never: up to 60).
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    End lo[NE], hi[NE];
+    double wa[NE], wb[NE], wc[NE];                                // its width one, two and three steps ago
+    int side[NE];
+    bool open[NE];
 #pragma unroll
     for (int s = 0; s < NE; ++s) {
         const int j = tid + s * T;
         int a = 0, z = points;                                    // first grid point with count > j
         while (a < z) {
             const int m = (a + z) >> 1;
-            if (cnt[m] > j) z = m; else a = m + 1;
+            if (cnt[m].x > j) z = m; else a = m + 1;
         }
-        lo[s] = fma(static_cast<double>(a), w0, gl);
+        lo[s] = a > 0 ? End{fma(static_cast<double>(a), w0, gl), gp[a - 1], cnt[a - 1].x, cnt[a - 1].y}
+                      : End{gl, nan, 0, 0};
+        hi[s] = a < points ? End{fma(static_cast<double>(a + 1), w0, gl), gp[a], cnt[a].x, cnt[a].y}
+                           : End{gu, nan, n, 0};
+        wa[s] = wb[s] = wc[s] = 4.0 * (hi[s].x - lo[s].x);
+        side[s] = 0;
+        open[s] = j < n;
     }
-    // ---- halve every cell to below eps ||T|| / 2 (the same number of steps for all)
-    double w = w0;
-    while (w > 1.1102230246251565e-16) {
-        w *= 0.5;
+    for (int step = 0; step < 128; ++step) {
+        bool any = false;
 #pragma unroll
-        for (int s = 0; s < NE; ++s) x[s] = lo[s] + w;
-        sturm<NE>(de, rows, x, c);
+        for (int s = 0; s < NE; ++s) {
+            const int j = tid + s * T;
+            const double w = hi[s].x - lo[s].x, mid = lo[s].x + 0.5 * w;
+            const double least = 1.1102230246251565e-16 * fmax(1.0, 2.0 * fabs(mid));
+            double t = mid;
+            if (lo[s].c == j && hi[s].c == j + 1 && w <= 0.5 * wc[s]) {
+                const double r = fabs(lo[s].p) * pow2_clamped(lo[s].e - hi[s].e);
+                const double q = fma(w, r / (r + fabs(hi[s].p)), lo[s].x);
+                if (q == q) t = fmin(fmax(q, lo[s].x + least), hi[s].x - least);
+            }
+            open[s] = open[s] && w > least && t > lo[s].x && t < hi[s].x;
+            wc[s] = wb[s];
+            wb[s] = wa[s];
+            wa[s] = w;
+            x[s] = open[s] ? t : lo[s].x;
+            any = any || open[s];
+        }
+        if (!__any_sync(0xffffffffu, any)) break;
+        sturm<NE>(de, rows, x, c, px, ex);
 #pragma unroll
-        for (int s = 0; s < NE; ++s)
-            if (c[s] <= tid + s * T) lo[s] = x[s];
+        for (int s = 0; s < NE; ++s) {
+            if (!open[s]) continue;
+            const bool up = c[s] <= tid + s * T;
+            End& moved = up ? lo[s] : hi[s];
+            End& stays = up ? hi[s] : lo[s];
+            const int way = up ? -1 : 1;
+            if (side[s] == way) {
+                const double m = 1.0 - fabs(px[s] / moved.p) * pow2_clamped(ex[s] - moved.e);
+                stays.p *= m > 0.0 ? m : 0.5;                     // (also where the end had no value)
+            }
+            moved = End{x[s], px[s], c[s], ex[s]};
+            side[s] = way;
+        }
     }
 #pragma unroll
     for (int s = 0; s < NE; ++s) {
         const int j = tid + s * T;
-        if (j < n) lam[j] = (lo[s] + 0.5 * w) * us;
+        if (j < n) lam[j] = (lo[s].x + 0.5 * (hi[s].x - lo[s].x)) * us;
     }
     __syncthreads();
     // ---- ascending (close eigenvalues may come out swapped in their last bits)

@@ -68,3 +68,18 @@ def test_not_finite_pair_is_reported_alone(n):
     assert info[0] == 0 and info[3] == 0 and 0 < info[1] <= n and 0 < info[2] <= n
     for p in (0, 3):
         assert np.abs(W[p] - ref[p]).max() <= 64 * n * EPS * np.abs(ref[p]).max()
+
+
+@pytest.mark.parametrize("n", [21, 41, 63, 101, 255])
+def test_pairs_equal_to_the_last_bit(n):
+    """Wilkinson's W+: its larger eigenvalues come in pairs that agree to machine precision, so their
+    brackets are never isolated; and a T whose eigenvalues spread over ten decades."""
+    m = n // 2
+    A = np.diag(np.abs(np.arange(n) - m).astype(np.complex128)) + np.diag(np.ones(n - 1), 1) + np.diag(np.ones(n - 1), -1)
+    d = 10.0 ** np.linspace(0.0, -10.0, n)
+    G = np.diag(d).astype(np.complex128) + np.diag(0.4 * np.sqrt(d[1:] * d[:-1]), 1) + np.diag(0.4 * np.sqrt(d[1:] * d[:-1]), -1)
+    P = np.array([A, G])
+    W, _, info = run(n, Mx.from_mats(P), eye(n, 2))
+    ref = np.linalg.eigvalsh(P)
+    assert (info == 0).all() and (np.diff(W, axis=1) >= 0).all()
+    assert (np.abs(W - ref).max(axis=1) <= 64 * n * EPS * np.abs(ref).max(axis=1)).all()
