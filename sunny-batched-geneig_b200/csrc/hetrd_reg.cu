@@ -147,26 +147,57 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_hetrd_reg(int n, int batch, c
         ac[s] = in ? s * RS + lane : CR - 1;
     }
 
-    // C's lower triangle, mirrored
-    auto entry = [&](int r, int j) {
-        double2 z = zero;
-        if (r < n && j < n) {
-            z = r >= j ? Cb[r + static_cast<size_t>(j) * n] : Cb[j + static_cast<size_t>(r) * n];
-            if (r < j) z.y = -z.y;
-            if (r == j) z.y = 0.0;
-        }
-        return z;
-    };
-#pragma unroll 4
-    for (int q = 0; q < off; ++q)
+    // C's lower triangle, mirrored: the shared-memory columns' lower parts by cp.async and the register
+    // columns' by loads that are all in flight together, then the upper parts from shared memory (row j of
+    // an earlier column; only the register columns' own corner is read transposed from global memory)
+    double2* col0 = cols - warp * CR;                             // column j < off NW at col0 + j CR
+    const int jr = off * NW;                                      // first register column
+    for (int q = 0; q < off; ++q) {
+        const int j = q * NW + warp;
 #pragma unroll
-        for (int s = 0; s < R; ++s)
-            cols[q * NW * CR + ac[s]] = entry(in ? s * RS + lane : n, q * NW + warp);
+        for (int s = 0; s < R; ++s) {
+            const int r = s * RS + lane;
+            if (in && r >= j && r < n) cp_async16(col0 + j * CR + r, Cb + r + static_cast<size_t>(j) * n);
+            else if (!in || r >= n) col0[j * CR + ac[s]] = zero;
+        }
+    }
     double2 a[R][NS];
 #pragma unroll
-    for (int q = 0; q < NS; ++q)
+    for (int q = 0; q < NS; ++q) {
+        const int j = (off + q) * NW + warp;
 #pragma unroll
-        for (int s = 0; s < R; ++s) a[s][q] = entry(in ? s * RS + lane : n, (off + q) * NW + warp);
+        for (int s = 0; s < R; ++s) {
+            const int r = s * RS + lane;
+            a[s][q] = zero;
+            if (in && r < n && j < n && r >= jr)
+                a[s][q] = r >= j ? Cb[r + static_cast<size_t>(j) * n] : Cb[j + static_cast<size_t>(r) * n];
+        }
+    }
+    cp_async_wait();
+    pair_sync<NW>();
+    for (int q = 0; q < off; ++q) {
+        const int j = q * NW + warp;
+#pragma unroll
+        for (int s = 0; s < R; ++s) {
+            const int r = s * RS + lane;
+            if (in && r < j) {
+                const double2 z = col0[r * CR + j];
+                col0[j * CR + r] = make_double2(z.x, -z.y);
+            }
+            if (in && r == j) col0[j * CR + r].y = 0.0;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+        const int j = (off + q) * NW + warp;
+#pragma unroll
+        for (int s = 0; s < R; ++s) {
+            const int r = s * RS + lane;
+            if (in && r < jr && j < n) a[s][q] = col0[r * CR + j];
+            if (r < j) a[s][q].y = -a[s][q].y;
+            if (r == j) a[s][q].y = 0.0;
+        }
+    }
     for (int i = threadIdx.x; i < 2 * (RV + 1); i += 32 * NW) vbuf[i] = zero;    // rows n .. RV stay zero
     for (int i = lane; i <= RV; i += 32) wb[i] = zero;
     pair_sync<NW>();

@@ -75,15 +75,15 @@ __global__ void __launch_bounds__(kTriThreads, 1) k_hetrd_tri(int n, int batch, 
     auto col_s = [&](int j) { return Ps + (pk(j, n) - pk(j0, n)) - j; };
     auto col_g = [&](int j) { return Pg + pk(j, n) - j; };
     auto column = [&](int j) { return j >= j0 ? col_s(j) : col_g(j); };
-    for (int j = warp; j < n; j += kTriWarps) {
+    for (int j = warp; j < n; j += kTriWarps) {                   // (C's diagonal is real as the reduction left it)
         double2* cj = column(j);
+        const double2* c = Cb + static_cast<size_t>(j) * n;
         for (int i = j + lane; i < n; i += 32) {
-            double2 v = Cb[i + static_cast<size_t>(j) * n];
-            if (i == j) v.y = 0.0;
-            cj[i] = v;
+            if (j >= j0) cp_async16(cj + i, c + i);
+            else cj[i] = c[i];
         }
     }
-    __syncthreads();
+    cp_async_wait();
     // (finite before their first step: the walk multiplies them by zeros while nothing is pending)
     for (int i = tid; i < 3 * n; i += kTriThreads) (i < 2 * n ? vbuf : wb - 2 * n)[i] = zero;
     __syncthreads();
