@@ -17,10 +17,10 @@
 // The kernels it replaces walked the packed triangle in shared memory (a warp per pair, each lane
 // its own row: 47 K shared-memory wavefronts per pair at n = 54, 62 % of the load/store unit's rate),
 // a full tile in shared memory by 256 threads (66 <= n <= 84), or the triangle in L2 (n > 84).
-// Microseconds per 1,000 pairs before -> now: n = 24 48 -> 21, 32 80 -> 34, 47 191 -> 139, 54 284 -> 166,
-// 72 1,197 -> 471, 96 2,013 -> 838, 128 4,600 -> 2,240.  It is bound by the latency of a step's chain
-// (column sum, norm, square root, reflector) at the few pairs an SM holds: FP64 pipe 34 % busy, a
-// third of the stalls LDS and shuffle results, a quarter the wait for the warp that forms the reflector.
+// Microseconds per 1,000 pairs before -> now: n = 24 48 -> 20, 32 80 -> 31, 47 191 -> 113, 54 284 -> 141,
+// 72 1,197 -> 422, 96 2,013 -> 737, 128 4,600 -> 2,070.  It is bound by the latency of a step's chain
+// (column sum, norm, square root, reflector) at the few pairs an SM holds and by the load/store unit (55 % at
+// n = 54); FP64 pipe 37 % busy.
 #include "kernels.cuh"
 #include "stages.cuh"
 
@@ -55,8 +55,6 @@ struct RegHetrdSmem {
         total = o;
     }
 };
-
-constexpr int kBlock = 2;                    // columns between two tests for live ones
 
 template <int NW>
 __device__ __forceinline__ void pair_sync() {
@@ -114,7 +112,8 @@ __device__ __forceinline__ void form_reflector(int c, int RS, int la, const doub
 #define SBG_ASC32(C) C(0) C(1) C(2) C(3) C(4) C(5) C(6) C(7) C(8) C(9) C(10) C(11) C(12) C(13) C(14) C(15) \
     C(16) C(17) C(18) C(19) C(20) C(21) C(22) C(23) C(24) C(25) C(26) C(27) C(28) C(29) C(30) C(31)
 
-template <int R, int NW, int NS, int MINB>
+// kBlock: register columns between two tests for live ones
+template <int R, int NW, int NS, int MINB, int kBlock>
 __global__ void __launch_bounds__(32 * NW, MINB) k_hetrd_reg(int n, int batch, const double2* __restrict__ C,
                                                              Workspace ws, const int* __restrict__ info) {
     const int b = blockIdx.x;
@@ -224,19 +223,25 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_hetrd_reg(int n, int batch, c
             double2 acc[R], am[R];                                // the two products of each part apart:
 #pragma unroll
             for (int s = S0; s < R; ++s) acc[s] = am[s] = zero;   // half as long a dependent chain
+            {
+                double2* c = cols + q0 * (NW * CR);
+                const double2 *pv = v + q0 * NW + warp, *pp = vp + q0 * NW + warp, *pw = wb + q0 * NW + warp;
 #pragma unroll 2
-            for (int q = q0; q < off; ++q) {
-                const int j = q * NW + warp;
-                const double2 pj = vp[j], wj = wb[j], vj = v[j];
+                for (int left = off - q0; left > 0; --left) {
+                    const double2 pj = *pp, wj = *pw, vj = *pv;
 #pragma unroll
-                for (int s = S0; s < R; ++s) {
-                    double2* c = cols + q * NW * CR + ac[s];
-                    const double2 t = cfmsc(wr[s], pj, cfmsc(vr[s], wj, *c));
-                    *c = t;
-                    acc[s].x = fma(t.x, vj.x, acc[s].x);
-                    acc[s].y = fma(t.x, vj.y, acc[s].y);
-                    am[s].x = fma(t.y, vj.y, am[s].x);
-                    am[s].y = fma(t.y, vj.x, am[s].y);
+                    for (int s = S0; s < R; ++s) {
+                        const double2 t = cfmsc(wr[s], pj, cfmsc(vr[s], wj, c[ac[s]]));
+                        c[ac[s]] = t;
+                        acc[s].x = fma(t.x, vj.x, acc[s].x);
+                        acc[s].y = fma(t.x, vj.y, acc[s].y);
+                        am[s].x = fma(t.y, vj.y, am[s].x);
+                        am[s].y = fma(t.y, vj.x, am[s].y);
+                    }
+                    c += NW * CR;
+                    pv += NW;
+                    pp += NW;
+                    pw += NW;
                 }
             }
 #pragma unroll
@@ -350,31 +355,33 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_hetrd_reg(int n, int batch, c
     if (threadIdx.x == 0) { eg[n - 1] = 0.0; taug[n - 1] = zero; }
 }
 
-// (rows per lane, warps per pair, column slots in registers, pairs per SM) by n.  Measured over the
-// neighbouring shapes, microseconds per 1,000 pairs: few warps and many pairs per SM win (at n = 54
-// 1 warp 198, 2 warps 166, 3 warps 185, 4 warps 227, 8 warps 327) until a pair's columns no longer fit beside
-// others in shared memory; fewer register slots than these make the shared-memory part the bound.
+// (rows per lane, warps per pair, column slots in registers, pairs per SM, block) by n.  Measured over the
+// neighbouring shapes, microseconds per 1,000 pairs: few warps and many pairs per SM win (n = 48: 1 warp 113, 2
+// 122; n = 54: 2 warps 141, 1 warp 170, and in an earlier form 3 warps 185, 4 227, 8 327) until a
+// pair's columns no longer fit beside others in shared memory; fewer register slots than these make the
+// shared-memory part the bound (n = 54: 8 slots 162, 10 147, 12 141).
 #define SBG_HETRD_REG_BY_N(n, F)                                                       \
     do {                                                                               \
-        if ((n) <= 24) F(1, 1, 8, 24);                                                 \
-        if ((n) <= 32) F(1, 1, 16, 16);                                                \
-        if ((n) <= 40) F(2, 1, 10, 10);                                                \
-        if ((n) <= 56) F(2, 2, 10, 6);                                                 \
-        if ((n) <= 64) F(2, 2, 16, 4);                                                 \
-        if ((n) <= 76) F(3, 4, 7, 3);                                                  \
-        if ((n) <= 96) F(3, 4, 8, 2);                                                  \
-        if ((n) <= 128) F(4, 8, 8, 1);                                                 \
-        F(5, 8, 9, 1);                                                                 \
+        if ((n) <= 24) F(1, 1, 8, 24, 2);                                              \
+        if ((n) <= 32) F(1, 1, 16, 16, 4);                                             \
+        if ((n) <= 40) F(2, 1, 10, 10, 2);                                             \
+        if ((n) <= 48) F(2, 1, 16, 8, 2);                                              \
+        if ((n) <= 56) F(2, 2, 12, 5, 4);                                              \
+        if ((n) <= 64) F(2, 2, 16, 4, 2);                                              \
+        if ((n) <= 76) F(3, 4, 7, 3, 2);                                               \
+        if ((n) <= 96) F(3, 4, 8, 2, 2);                                               \
+        if ((n) <= 128) F(4, 8, 8, 1, 2);                                              \
+        F(5, 8, 9, 1, 2);                                                              \
     } while (0)
 
-template <int R, int NW, int NS, int MINB>
+template <int R, int NW, int NS, int MINB, int kBlock>
 cudaError_t run_hetrd_reg(int n, int batch, const double2* C, const Workspace& ws, const int* info,
                           cudaStream_t stream) {
     const size_t smem = RegHetrdSmem<R, NW>(n, NS).total;
     if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
     static SmemOptIn f;
-    set_smem_limit(reinterpret_cast<const void*>(k_hetrd_reg<R, NW, NS, MINB>), f, static_cast<int>(smem));
-    k_hetrd_reg<R, NW, NS, MINB><<<batch, 32 * NW, smem, stream>>>(n, batch, C, ws, info);
+    set_smem_limit(reinterpret_cast<const void*>(k_hetrd_reg<R, NW, NS, MINB, kBlock>), f, static_cast<int>(smem));
+    k_hetrd_reg<R, NW, NS, MINB, kBlock><<<batch, 32 * NW, smem, stream>>>(n, batch, C, ws, info);
     return cudaGetLastError();
 }
 
@@ -384,13 +391,13 @@ cudaError_t launch_hetrd_reg(int n, int batch, const double2* C, const Workspace
                              cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (n < 1 || n > kHetrdRegMaxN || !C || !info || !ws.LV || !ws.d || !ws.e || !ws.tau) return cudaErrorInvalidValue;
-#define SBG_RUN(R, NW, NS, MINB) return run_hetrd_reg<R, NW, NS, MINB>(n, batch, C, ws, info, stream)
+#define SBG_RUN(R, NW, NS, MINB, KB) return run_hetrd_reg<R, NW, NS, MINB, KB>(n, batch, C, ws, info, stream)
     SBG_HETRD_REG_BY_N(n, SBG_RUN);
 #undef SBG_RUN
 }
 
 size_t hetrd_reg_smem_bytes(int n) {
-#define SBG_SIZE(R, NW, NS, MINB) return RegHetrdSmem<R, NW>(n, NS).total
+#define SBG_SIZE(R, NW, NS, MINB, KB) return RegHetrdSmem<R, NW>(n, NS).total
     SBG_HETRD_REG_BY_N(n, SBG_SIZE);
 #undef SBG_SIZE
 }
