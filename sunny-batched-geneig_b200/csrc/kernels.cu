@@ -145,29 +145,38 @@ __global__ void k_ql_chain(int n, int batch, Workspace ws, double* __restrict__ 
 // Eigenvectors of the tridiagonal T (d, e) from its FP64 eigenvalues (k_tridiag_values) by inverse
 // iteration, one warp per pair, one lane per eigenvector at a time (LAPACK dstein's method):
 // T - lambda_j I = L U without pivoting, a pivot below eps ||T|| replaced by that size, two
-// solves from a fixed pseudo-random start, each followed by normalisation.  That is O(n) work
-// per vector against the O(n^2) of applying every QL rotation to it.  The vectors of
-// eigenvalues closer than kInvitOrtol ||T|| (a cluster) are computed in order, one lane per
-// cluster, with three solves each orthogonalised against the cluster's earlier vectors
-// (modified Gram-Schmidt); the other vectors' orthogonality is ~eps ||T|| / gap.  A pair with a
+// solves, each followed by normalisation.  That is O(n) work
+// per vector against the O(n^2) of applying every QL rotation to it.  Vectors of
+// eigenvalues closer than kInvitOrtol ||T|| (a cluster) are then orthogonalised in order (Gram-Schmidt);
+// where two of them overlap too much for that, the cluster's members are computed again, one lane per
+// member, with three solves each orthogonalised against the cluster's earlier vectors.  The other
+// vectors' orthogonality is ~eps ||T|| / gap.  A pair with a
 // cluster of more than kInvitMaxCluster eigenvalues (a spectrum dominated by one huge eigenvalue) or
-// more than 32 cluster members gets every vector as if it stood alone, and k_tridiag_ortho
+// more cluster members than lanes gets every vector as if it stood alone, and k_tridiag_ortho
 // orthonormalises them.  Every vector must pass ||T z - lambda z|| <= kInvitTol ||T||; a pair with a
 // failed vector or a T that is not finite is recomputed by the QL instead.
-// Per-lane scratch (1/u and the vector) is interleaved [i * 33 + lane]: lane-parallel
+// Bound by the latency of the lanes' recurrences with the 6-9 pairs per SM that the lane scratch leaves room
+// for (FP64 pipe 10 % busy at 1.95 ms).  32,768 pairs at n = 54: 1.95 -> 1.12 ms with the backward-only first solve,
+// the lane count below, running pointers, and cluster members in the main batches instead of three rounds of
+// their own for one close pair of eigenvalues in a spectrum.
+// Per-lane scratch (1/u and the vector) is interleaved [i * ld + lane]: lane-parallel
 // recurrences read consecutive words, and the warp's column-by-column copy to the caller's X
 // buffer (Z, column k = vector k) reads it across lanes without bank conflicts.
 constexpr double kInvitOrtol = 3e-4;
 constexpr int kInvitMaxCluster = 8;
 constexpr double kInvitTol = 256.0 * 1.1102230246251565e-16;
-constexpr int kInvitLd = 33;            // lane scratch [i * 33 + lane]: rows also read across lanes
+// Vectors (lanes) at a time, the same for every batch, and the odd stride of the lane scratch
+// [i * ld + lane], which both the lanes' recurrences and the reads across lanes take without conflicts:
+// 27 and 27 at n = 54 instead of 32 and 33, 22 % less scratch and two more pairs per SM.
+__host__ __device__ constexpr int invit_lanes(int n) { return (n + (n + 31) / 32 - 1) / ((n + 31) / 32); }
+__host__ __device__ constexpr int invit_ld(int n) { return invit_lanes(n) | 1; }
 
 struct InvitSmem {
     size_t scr, dd, ee, lam, cls, mem, flag, per_warp;
     // with_tile: the scratch also holds the in-kernel fallback QL's Z tile
     __host__ __device__ explicit InvitSmem(int n, bool with_tile = true) {
         size_t o = 0;
-        const size_t lanes = 2 * kInvitLd * static_cast<size_t>(n), tile = static_cast<size_t>(n) * tile_ld(n);
+        const size_t lanes = 2 * static_cast<size_t>(invit_ld(n)) * n, tile = static_cast<size_t>(n) * tile_ld(n);
         scr = o;  o += 8 * (with_tile && tile > lanes ? tile : lanes);
         dd = o;   o += 8 * static_cast<size_t>(n);
         ee = o;   o += 8 * static_cast<size_t>(n);
@@ -187,78 +196,91 @@ __device__ __forceinline__ double invit_start(int j, int i) {
     return static_cast<double>(h & 0xFFFFFu) * (2.0 / 1048575.0) - 1.0;
 }
 
-// Per-lane pieces of inverse iteration on T - lam I; invu and z are the lane's columns of the
-// interleaved scratch ([i * kInvitLd + lane]).
-#define SBG_IU(i) invu[(i) * kInvitLd + lane]
-#define SBG_ZV(i) z[(i) * kInvitLd + lane]
-// T - lam I = L U without pivoting (pivots below `tiny` raised to it): keeps 1/u_i.  Each step's
-// operands are loaded one step ahead, so the dependent chain is only the recurrence itself.
-__device__ __forceinline__ void invit_factor(int n, double lam, const double* __restrict__ dd,
-                                             const double* __restrict__ ee, double tiny, double* __restrict__ invu) {
-    const int lane = threadIdx.x & 31;
+// Per-lane pieces of inverse iteration on T - lam I; iu and z are the lane's columns of the interleaved
+// scratch (element i at i * ld).  Operands are loaded a step ahead, so each dependent chain is only the
+// recurrence itself.
+// T - lam I = L U without pivoting (pivots below `tiny` raised to it): keeps 1/u_i.
+__device__ __forceinline__ void invit_factor(int n, int ld, double lam, const double* __restrict__ dd,
+                                             const double* __restrict__ ee, double tiny, double* __restrict__ iu) {
     double u = dd[0] - lam;
     if (fabs(u) < tiny) u = copysign(tiny, u);
-    double iu = recip_nr(u);
-    SBG_IU(0) = iu;
+    double r = recip_nr(u);
+    *iu = r;
     double dn = n > 1 ? dd[1] - lam : 0.0, en = n > 1 ? ee[0] * ee[0] : 0.0;
     for (int i = 1; i < n; ++i) {
         const double di = dn, e2 = en;
         if (i + 1 < n) { dn = dd[i + 1] - lam; en = ee[i] * ee[i]; }
-        u = fma(-e2, iu, di);
+        u = fma(-e2, r, di);
         if (fabs(u) < tiny) u = copysign(tiny, u);
-        iu = recip_nr(u);
-        SBG_IU(i) = iu;
+        r = recip_nr(u);
+        iu += ld;
+        *iu = r;
     }
 }
-// z <- (T - lam I)^{-1} x with the factors above, x = sc z, or (GEN) the start vector of eigenvalue
-// j; returns ||z||^2 (summed in the backward pass).  Operands are loaded one step ahead.
-template <bool GEN>
-__device__ __forceinline__ double invit_solve(int n, const double* __restrict__ ee, const double* __restrict__ invu,
-                                              double* __restrict__ z, double sc, int j) {
-    const int lane = threadIdx.x & 31;
-    auto xin = [&](int i) { if constexpr (GEN) return invit_start(j, i); else return sc * SBG_ZV(i); };
-    double y = xin(0);
-    SBG_ZV(0) = y;
-    double xn = n > 1 ? xin(1) : 0.0, cn = n > 1 ? ee[0] * SBG_IU(0) : 0.0;
-    for (int i = 1; i < n; ++i) {                      // L y = x  (L(i, i-1) = e_{i-1} / u_{i-1})
-        const double x = xn, c = cn;
-        if (i + 1 < n) { xn = xin(i + 1); cn = ee[i] * SBG_IU(i); }
-        y = fma(-c, y, x);
-        SBG_ZV(i) = y;
-    }
-    double zn = y * SBG_IU(n - 1);                     // U z = y  (U(i, i+1) = e_i)
-    SBG_ZV(n - 1) = zn;
+// z <- U^{-1} y, y in z (ONES: y = 1, whatever z holds); returns ||z||^2.
+template <bool ONES>
+__device__ __forceinline__ double invit_back(int n, int ld, const double* __restrict__ ee, const double* __restrict__ iu,
+                                             double* __restrict__ z) {
+    z += static_cast<size_t>(n - 1) * ld;
+    iu += static_cast<size_t>(n - 1) * ld;
+    double zn = (ONES ? 1.0 : *z) * *iu;                   // U z = y  (U(i, i+1) = e_i)
+    *z = zn;
     double s2 = zn * zn;
-    double yp = n > 1 ? SBG_ZV(n - 2) : 0.0, ep = n > 1 ? ee[n - 2] : 0.0, ip = n > 1 ? SBG_IU(n - 2) : 0.0;
+    double yp = 1.0, ep = 0.0, ip = 0.0;
+    if (n > 1) {
+        if (!ONES) yp = z[-ld];
+        ep = ee[n - 2];
+        ip = iu[-ld];
+    }
     for (int i = n - 2; i >= 0; --i) {
+        z -= ld;
+        iu -= ld;
         const double yi = yp, ei = ep, ii = ip;
-        if (i > 0) { yp = SBG_ZV(i - 1); ep = ee[i - 1]; ip = SBG_IU(i - 1); }
+        if (i > 0) { if (!ONES) yp = z[-ld]; ep = ee[i - 1]; ip = iu[-ld]; }
         zn = fma(-ei, zn, yi) * ii;
-        SBG_ZV(i) = zn;
+        *z = zn;
         s2 = fma(zn, zn, s2);
     }
     return s2;
 }
+// z <- (T - lam I)^{-1} x with the factors above, x = sc z, or (GEN) the start vector of eigenvalue
+// j; returns ||z||^2 (summed in the backward pass).
+template <bool GEN>
+__device__ __forceinline__ double invit_solve(int n, int ld, const double* __restrict__ ee,
+                                              const double* __restrict__ iu, double* __restrict__ z, double sc, int j) {
+    double* zi = z;
+    const double* ui = iu;
+    double y = GEN ? invit_start(j, 0) : sc * *zi;
+    *zi = y;
+    double xn = 0.0, cn = 0.0;
+    if (n > 1) { xn = GEN ? invit_start(j, 1) : sc * zi[ld]; cn = ee[0] * *ui; }
+    for (int i = 1; i < n; ++i) {                      // L y = x  (L(i, i-1) = e_{i-1} / u_{i-1})
+        zi += ld;
+        ui += ld;
+        const double x = xn, c = cn;
+        if (i + 1 < n) { xn = GEN ? invit_start(j, i + 1) : sc * zi[ld]; cn = ee[i] * *ui; }
+        y = fma(-c, y, x);
+        *zi = y;
+    }
+    return invit_back<false>(n, ld, ee, iu, z);
+}
 // z <- sc z in place; returns ||T z - lam z||^2 of the scaled vector (one pass).
-__device__ __forceinline__ double invit_scale_residual(int n, double lam, const double* __restrict__ dd,
+__device__ __forceinline__ double invit_scale_residual(int n, int ld, double lam, const double* __restrict__ dd,
                                                        const double* __restrict__ ee, double* __restrict__ z,
                                                        double sc) {
-    const int lane = threadIdx.x & 31;
-    double zp = 0.0, zc = SBG_ZV(0), r2 = 0.0;
+    double zp = 0.0, zc = *z, r2 = 0.0, el = 0.0;
     for (int i = 0; i < n; ++i) {
-        const double zx = i + 1 < n ? SBG_ZV(i + 1) : 0.0;
-        double v = (dd[i] - lam) * zc;
-        if (i > 0) v = fma(ee[i - 1], zp, v);
-        if (i + 1 < n) v = fma(ee[i], zx, v);
+        const double zx = i + 1 < n ? z[ld] : 0.0, er = i + 1 < n ? ee[i] : 0.0;
+        const double v = fma(er, zx, fma(el, zp, (dd[i] - lam) * zc));
         r2 = fma(v, v, r2);
-        SBG_ZV(i) = zc * sc;
+        *z = zc * sc;
+        z += ld;
         zp = zc;
         zc = zx;
+        el = er;
     }
     return r2 * sc * sc;
 }
-#undef SBG_IU
-#undef SBG_ZV
 
 // flag_redo: a pair the kernel cannot take gets ws.flag = 2 and no output (the rotation-log QL is
 // then run for the flagged pairs); otherwise the warp QL runs here, on a Z tile in the scratch.
@@ -310,79 +332,105 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
         sflag[1] = cnt;
     }
     __syncwarp();
-    const int cnt = sflag[1];
+    const int cnt = sflag[1], nl = invit_lanes(n), ld = invit_ld(n);
     bool fallback = inf != 0;
-    const bool together = sflag[0] > kInvitMaxCluster || cnt > 32;    // all vectors here, then k_tridiag_ortho
+    const bool together = sflag[0] > kInvitMaxCluster || cnt > nl;    // all vectors here, then k_tridiag_ortho
     if (!fallback) {
         bool ok = true;
         double* invu = scr;
-        double* zs = scr + kInvitLd * n;
-        // (1) each cluster's first vector and every singleton: factor, two solves from a fixed
-        // pseudo-random start, residual test; 32 at a time, then copied out column by column
-        for (int base = 0; base < n; base += 32) {
+        double* zs = scr + ld * n;
+        double *iu = invu + lane, *z = zs + lane;     // (lanes >= nl have no column and never touch them)
+        // (1) every vector as if it stood alone: factor, two solves, residual test; nl at a time, then
+        // copied out column by column.  The first solve starts from L 1, so that only its backward half is
+        // left (EISPACK tinvit's start); for k_tridiag_ortho from a pseudo-random vector of its own
+        // (L times one saves its forward half too, but the vectors come out closer to one another: n = 96 with
+        // a dominating eigenvalue, k_tridiag_ortho 833 -> 915 us against 629 -> 581 us here).
+        for (int base = 0; base < n; base += nl) {
             const int j = base + lane;
-            if (j < n && (together || cls[j] == j)) {
-                invit_factor(n, lam[j], dd, ee, tiny, invu);
-                double s2 = invit_solve<true>(n, ee, invu, zs, 1.0, j);
+            if (lane < nl && j < n) {
+                invit_factor(n, ld, lam[j], dd, ee, tiny, iu);
+                double s2 = together ? invit_solve<true>(n, ld, ee, iu, z, 1.0, j) : invit_back<true>(n, ld, ee, iu, z);
                 const bool f1 = s2 > 0.0 && isfinite(s2);
-                s2 = invit_solve<false>(n, ee, invu, zs, f1 ? 1.0 / sqrt(s2) : 1.0, j);
+                s2 = invit_solve<false>(n, ld, ee, iu, z, f1 ? 1.0 / sqrt(s2) : 1.0, j);
                 const bool f2 = s2 > 0.0 && isfinite(s2);
-                const double r2 = invit_scale_residual(n, lam[j], dd, ee, zs, f2 ? 1.0 / sqrt(s2) : 1.0);
+                const double r2 = invit_scale_residual(n, ld, lam[j], dd, ee, z, f2 ? 1.0 / sqrt(s2) : 1.0);
                 ok &= f1 && f2 && sqrt(r2) <= kInvitTol * tnorm;
             }
             __syncwarp();
-            const int top = min(32, n - base);
+            const int top = min(nl, n - base);
             for (int L = 0; L < top; ++L) {
                 const int jj = base + L;
-                if (!together && cls[jj] != jj) continue;     // uniform
                 double* zc = Zg + static_cast<size_t>(jj) * n;
-                for (int i = lane; i < n; i += 32) zc[i] = zs[i * kInvitLd + L];
+                for (int i = lane; i < n; i += 32) zc[i] = zs[i * ld + L];
             }
             __syncwarp();
         }
         ok = __all_sync(0xffffffffu, ok);              // from here on `ok` is the same on every lane
-        // (2) the other cluster members, one lane each, all at once: three rounds of a solve
+        // (2) cluster members, in index order: Gram-Schmidt against the cluster's earlier vectors.  Vectors
+        // of eigenvalues a gap apart overlap by eps ||T|| / gap only, and taking that out moves the residual
+        // by eps ||T||; if an overlap is larger than 1e-6, the eigenvalues are too close for vectors
+        // computed alone and (3) computes the members again.  (Each lane reads and writes its own rows.)
+        bool again = false;
+        if (ok && !together) {
+            for (int m = 0; m < cnt && !again; ++m) {
+                const int j = members[m];
+                double* zj = Zg + static_cast<size_t>(j) * n;
+                for (int q = cls[j]; q < j && !again; ++q) {
+                    const double* zq = Zg + static_cast<size_t>(q) * n;
+                    double c = 0.0;
+                    for (int i = lane; i < n; i += 32) c = fma(zq[i], zj[i], c);
+                    c = warp_sum(c);
+                    again = !(fabs(c) <= 1e-6);                   // uniform
+                    for (int i = lane; i < n; i += 32) zj[i] = fma(-c, zq[i], zj[i]);
+                }
+                double s2 = 0.0;
+                for (int i = lane; i < n; i += 32) s2 = fma(zj[i], zj[i], s2);
+                const double inv = 1.0 / sqrt(warp_sum(s2));
+                for (int i = lane; i < n; i += 32) zj[i] *= inv;
+            }
+        }
+        // (3) such clusters' members, one lane each, all at once: three rounds of a solve
         // (every lane its own member) and modified Gram-Schmidt in index order (the whole warp,
         // lanes over rows) against the cluster's first vector and its earlier members
-        if (ok && cnt > 0 && !together) {
+        if (again) {
             const int jm = lane < cnt ? members[lane] : -1;
             if (jm >= 0) {
-                invit_factor(n, lam[jm], dd, ee, tiny, invu);
+                invit_factor(n, ld, lam[jm], dd, ee, tiny, iu);
             }
             for (int it = 0; it < 3 && ok; ++it) {        // each round's input is unit (Gram-Schmidt below)
                 if (jm >= 0) {
-                    if (it == 0) invit_solve<true>(n, ee, invu, zs, 1.0, jm);
-                    else invit_solve<false>(n, ee, invu, zs, 1.0, jm);
+                    if (it == 0) invit_solve<true>(n, ld, ee, iu, z, 1.0, jm);
+                    else invit_solve<false>(n, ld, ee, iu, z, 1.0, jm);
                 }
                 __syncwarp();
                 for (int m = 0; m < cnt && ok; ++m) {
                     const int j = members[m], s0 = cls[j];
                     const double* q0 = Zg + static_cast<size_t>(s0) * n;
                     double c = 0.0;
-                    for (int i = lane; i < n; i += 32) c = fma(q0[i], zs[i * kInvitLd + m], c);
+                    for (int i = lane; i < n; i += 32) c = fma(q0[i], zs[i * ld + m], c);
                     c = warp_sum(c);
-                    for (int i = lane; i < n; i += 32) zs[i * kInvitLd + m] = fma(-c, q0[i], zs[i * kInvitLd + m]);
+                    for (int i = lane; i < n; i += 32) zs[i * ld + m] = fma(-c, q0[i], zs[i * ld + m]);
                     for (int m2 = 0; m2 < m; ++m2) {
                         if (cls[members[m2]] != s0) continue;     // uniform
                         double c2 = 0.0;
-                        for (int i = lane; i < n; i += 32) c2 = fma(zs[i * kInvitLd + m2], zs[i * kInvitLd + m], c2);
+                        for (int i = lane; i < n; i += 32) c2 = fma(zs[i * ld + m2], zs[i * ld + m], c2);
                         c2 = warp_sum(c2);
                         for (int i = lane; i < n; i += 32)
-                            zs[i * kInvitLd + m] = fma(-c2, zs[i * kInvitLd + m2], zs[i * kInvitLd + m]);
+                            zs[i * ld + m] = fma(-c2, zs[i * ld + m2], zs[i * ld + m]);
                     }
                     double s2 = 0.0;
-                    for (int i = lane; i < n; i += 32) s2 = fma(zs[i * kInvitLd + m], zs[i * kInvitLd + m], s2);
+                    for (int i = lane; i < n; i += 32) s2 = fma(zs[i * ld + m], zs[i * ld + m], s2);
                     s2 = warp_sum(s2);
                     if (!(s2 > 0.0) || !isfinite(s2)) { ok = false; break; }     // uniform
                     const double inv = 1.0 / sqrt(s2);
-                    for (int i = lane; i < n; i += 32) zs[i * kInvitLd + m] *= inv;
+                    for (int i = lane; i < n; i += 32) zs[i * ld + m] *= inv;
                 }
                 __syncwarp();
             }
-            if (jm >= 0 && ok) ok &= sqrt(invit_scale_residual(n, lam[jm], dd, ee, zs, 1.0)) <= kInvitTol * tnorm;
+            if (jm >= 0 && ok) ok &= sqrt(invit_scale_residual(n, ld, lam[jm], dd, ee, z, 1.0)) <= kInvitTol * tnorm;
             for (int m = 0; m < cnt; ++m) {
                 double* zc = Zg + static_cast<size_t>(members[m]) * n;
-                for (int i = lane; i < n; i += 32) zc[i] = zs[i * kInvitLd + m];
+                for (int i = lane; i < n; i += 32) zc[i] = zs[i * ld + m];
             }
         }
         fallback = !__all_sync(0xffffffffu, ok);
