@@ -2,10 +2,10 @@
 // C = L^{-1} A L^{-H} (Ogita-Aishima iteration) with every matrix product on the FP64 tensor
 // cores (mma.sync m8n8k4 f64), and the FP64 fallback for pairs the refinement cannot take.
 //
-//   k_refine_c<NP>       one CTA per pair, NP / 8 warps; C (from the pair's stash) and the
-//                        eigenvector matrix Y = Q Z (from the X buffer) held in shared memory as
-//                        planar FP64 tiles (re and im planes, column-major, ld = NP + 4, zero
-//                        padded to NP = n rounded up to 8).  Warp w owns rows 8w..8w+7 of every
+//   k_refine_c<NP>       one CTA per pair, NP / 8 warps; the eigenvector matrix Y = Q Z (from the X
+//                        buffer) and P held in shared memory as planar FP64 tiles (re and im planes,
+//                        column-major, ld = NP + 4, zero padded to NP = n rounded up to 8), C read as
+//                        MMA fragments from the pair's stash of the same layout.  Warp w owns rows 8w..8w+7 of every
 //                        strip product (all NP columns): P = C Y and Y' = Y + Y E; the Hermitian
 //                        G = Y^H Y and S = Y^H P are computed as lower-triangle 8 x 8 blocks dealt
 //                        round-robin over the warps.  Writes the refined Y over X and W, or flags
@@ -65,29 +65,64 @@ struct Strip {
     }
 };
 
-// acc += A(rows row0..row0+7, :) B over k in [0, 8 NB).  A(r, k) is M(r, k) of the stored matrix,
-// or conj(M(k, r)) when CONJT; B(k, c) is the stored matrix N(k, c).  Every operand load is a
+// One k-step of a strip product: the A fragment (ar, ai) against every column block of N.
+template <int NB>
+__device__ __forceinline__ void cstep(Strip<NB>& acc, double ar, double ai, const double* __restrict__ Nre,
+                                      const double* __restrict__ Nim, int ld, int k0) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int c = 0; c < NB; ++c) {
+        const int ib = (8 * c + g) * ld + k0 + t;
+        const double br = Nre[ib], bi = Nim[ib];
+        dmma(acc.re[c][0], acc.re[c][1], ar, br);
+        dmma(acc.im[c][0], acc.im[c][1], ar, bi);
+        dmma(acc.re[c][0], acc.re[c][1], -ai, bi);
+        dmma(acc.im[c][0], acc.im[c][1], ai, br);
+    }
+}
+
+// acc += A(rows row0..row0+7, :) N over k in [0, 8 NB), both in shared memory.  Every operand load is a
 // column-major planar read with ld = NP + 4, which spreads the 16 lanes of each half-warp over 16
 // distinct 8-byte banks for both fragment shapes.
-template <int NB, bool CONJT>
+template <int NB>
 __device__ __forceinline__ void cgemm(Strip<NB>& acc, const double* __restrict__ Mre, const double* __restrict__ Mim,
                                       const double* __restrict__ Nre, const double* __restrict__ Nim, int ld, int row0) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll 2
     for (int k0 = 0; k0 < 8 * NB; k0 += 4) {
-        const int ia = CONJT ? (row0 + g) * ld + k0 + t : (k0 + t) * ld + row0 + g;
-        const double ar = Mre[ia];
-        const double ai = CONJT ? -Mim[ia] : Mim[ia];
-#pragma unroll
-        for (int c = 0; c < NB; ++c) {
-            const int ib = (8 * c + g) * ld + k0 + t;
-            const double br = Nre[ib], bi = Nim[ib];
-            dmma(acc.re[c][0], acc.re[c][1], ar, br);
-            dmma(acc.re[c][0], acc.re[c][1], -ai, bi);
-            dmma(acc.im[c][0], acc.im[c][1], ar, bi);
-            dmma(acc.im[c][0], acc.im[c][1], ai, br);
-        }
+        const int ia = (k0 + t) * ld + row0 + g;
+        cstep<NB>(acc, Mre[ia], Mim[ia], Nre, Nim, ld, k0);
     }
+}
+
+// The same with A read ahead (global memory): each element is read once per product by one lane, as 64-byte runs of
+// a column, two k-steps ahead of its use (one k-step is >= 450 cycles of MMAs).  Returns the lane's sum of
+// |A(r, k)|^2.
+template <int NB>
+__device__ __forceinline__ double cgemm_ahead(Strip<NB>& acc, const double* __restrict__ Mre,
+                                               const double* __restrict__ Mim, const double* __restrict__ Nre,
+                                               const double* __restrict__ Nim, int ld, int row0) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const double *pr = Mre + t * ld + row0 + g, *pi = Mim + t * ld + row0 + g;
+    double a0r = pr[0], a0i = pi[0], a1r = pr[4 * ld], a1i = pi[4 * ld], s2 = 0.0;
+#pragma unroll 1
+    for (int k0 = 0; k0 < 8 * NB; k0 += 8) {
+        double b0r = 0.0, b0i = 0.0, b1r = 0.0, b1i = 0.0;
+        if (k0 + 8 < 8 * NB) {
+            pr += 8 * ld;
+            pi += 8 * ld;
+            b0r = pr[0];
+            b0i = pi[0];
+            b1r = pr[4 * ld];
+            b1i = pi[4 * ld];
+        }
+        s2 = fma(a0r, a0r, fma(a0i, a0i, s2));
+        cstep<NB>(acc, a0r, a0i, Nre, Nim, ld, k0);
+        s2 = fma(a1r, a1r, fma(a1i, a1i, s2));
+        cstep<NB>(acc, a1r, a1i, Nre, Nim, ld, k0 + 4);
+        a0r = b0r; a0i = b0i; a1r = b1r; a1i = b1i;
+    }
+    return s2;
 }
 
 // The lower-triangle 8 x 8 blocks of the Hermitian products G = Y^H Y and S = Y^H P:
@@ -142,38 +177,25 @@ __device__ __forceinline__ void gram_lower(Gram<NB>& gm, const double* __restric
     }
 }
 
-// Block-wide sums of four values (one slot row per warp in red[4 * NW]); every thread gets them.
+// Block-wide sums of v[0], v[1], v[3] and max of v[2] (one slot row per warp in red[4 * NW]); every
+// thread gets them.
 template <int NW>
-__device__ __forceinline__ void block_sum4(double (&v)[4], double* red) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = warp_sum(v[q]);
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) red[4 * w + q] = v[q];
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        double s = 0.0;
-        for (int i = 0; i < NW; ++i) s += red[4 * i + q];
-        v[q] = s;
-    }
-    __syncthreads();
-}
-
-// Block-wide sums of v[0], v[1] and max of v[2] (same slots as block_sum4).
-template <int NW>
-__device__ __forceinline__ void block_sum2_max(double (&v)[4], double* red) {
+__device__ __forceinline__ void block_sum3_max(double (&v)[4], double* red) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     v[0] = warp_sum(v[0]);
     v[1] = warp_sum(v[1]);
+    v[3] = warp_sum(v[3]);
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) v[2] = fmax(v[2], shfl_xor(v[2], m));
-    if (lane == 0) { red[4 * w] = v[0]; red[4 * w + 1] = v[1]; red[4 * w + 2] = v[2]; }
+    if (lane == 0) { red[4 * w] = v[0]; red[4 * w + 1] = v[1]; red[4 * w + 2] = v[2]; red[4 * w + 3] = v[3]; }
     __syncthreads();
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int i = 0; i < NW; ++i) { a += red[4 * i]; b += red[4 * i + 1]; c = fmax(c, red[4 * i + 2]); }
-    v[0] = a; v[1] = b; v[2] = c;
+    v[0] = v[1] = v[2] = v[3] = 0.0;
+    for (int i = 0; i < NW; ++i) {
+        v[0] += red[4 * i];
+        v[1] += red[4 * i + 1];
+        v[2] = fmax(v[2], red[4 * i + 2]);
+        v[3] += red[4 * i + 3];
+    }
     __syncthreads();
 }
 
@@ -181,12 +203,10 @@ template <int NP>
 struct RefineCSmem {
     static constexpr int LD = NP + 4;
     static constexpr size_t plane = sizeof(double) * NP * LD;
-    static constexpr size_t Cre = 0, Cim = plane, Yre = 2 * plane, Yim = 3 * plane, Pre = 4 * plane,
-                            Pim = 5 * plane, lam = 6 * plane;
+    static constexpr size_t Yre = 0, Yim = plane, Pre = 2 * plane, Pim = 3 * plane, lam = 4 * plane;
     static constexpr size_t red = lam + align16(sizeof(double) * NP);
     static constexpr size_t order = red + align16(sizeof(double) * 4 * (NP / 8));
-    static constexpr size_t bar = order + align16(sizeof(int) * NP);
-    static constexpr size_t total = bar + 16;
+    static constexpr size_t total = order + align16(sizeof(int) * NP);
 };
 
 constexpr double kEps = 1.1102230246251565e-16;
@@ -205,16 +225,18 @@ constexpr double kOrthTol = 1e-13;       // max |(Y^H Y - I)_ij| accepted
 // A start from complex64 typically stops after one update (two passes of products).  Returns
 // true when it stopped converged within max_updates updates.
 template <int NP>
-__device__ bool refine(int n, const double* Cre, const double* Cim, double* Yre, double* Yim, double* Pre, double* Pim,
-                       double* lam, double* red, double cnorm, int max_updates) {
-    constexpr int NB = NP / 8, LD = NP + 4, NT = NP * 4;
+__device__ __forceinline__ bool refine(int n, const double* __restrict__ Cre, const double* __restrict__ Cim,
+                                       double* Yre, double* Yim, double* Pre, double* Pim, double* lam, double* red,
+                                       int max_updates) {
+    constexpr int NB = NP / 8, LD = NP + 4;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
     const int row0 = 8 * w;
     for (int it = 0;; ++it) {
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};  // ||S - diag lam||^2, ||R||^2, max|R_ij|, ||C||^2
         {
             Strip<NB> P;
             P.zero();
-            cgemm<NB, false>(P, Cre, Cim, Yre, Yim, LD, row0);
+            acc[3] = cgemm_ahead<NB>(P, Cre, Cim, Yre, Yim, LD, row0);
             P.store(Pre, Pim, LD, row0);      // the P tile is free: the previous E was consumed
         }
         __syncthreads();
@@ -236,7 +258,6 @@ __device__ bool refine(int n, const double* Cre, const double* Cim, double* Yre,
             }
         __syncthreads();                       // lam visible; every warp is done reading P as an operand
         // norms and the largest departure from orthonormality (lower blocks; off-diagonal blocks twice)
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};  // ||S - diag lam||^2, ||R||^2, max|R_ij|, -
 #pragma unroll
         for (int k = 0; k < Gram<NB>::KB; ++k)
 #pragma unroll
@@ -251,22 +272,32 @@ __device__ bool refine(int n, const double* Cre, const double* Cim, double* Yre,
                     acc[2] = fmax(acc[2], fabs(rr) + fabs(ri));
                 }
             }
-        // residual of every column: ||P_j - lam_j y_j||^2 against (256 eps ||C||_F)^2 ||y_j||^2
+        block_sum3_max<NB>(acc, red);
+        const double cnorm = sqrt(acc[3]);
+        // residual of every column: ||P_j - lam_j y_j||^2 against (256 eps ||C||_F)^2 ||y_j||^2; eight lanes
+        // per column (zero rows below n), four columns a warp, 2 (NP / 8) in all
         bool res_ok = true;
-        for (int j = tid; j < n; j += NT) {
+        const double tol = 256.0 * kEps * cnorm;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = 4 * (w + h * NB) + (lane >> 3);          // < NP
+            const double lj = j < n ? lam[j] : 0.0;
             double rr = 0.0, yy = 0.0;
-            const double lj = lam[j];
-            for (int i = 0; i < n; ++i) {
+#pragma unroll
+            for (int i = lane & 7; i < NP; i += 8) {
                 const double yr = Yre[j * LD + i], yi = Yim[j * LD + i];
                 const double dr = fma(-lj, yr, Pre[j * LD + i]), di = fma(-lj, yi, Pim[j * LD + i]);
                 rr = fma(dr, dr, fma(di, di, rr));
                 yy = fma(yr, yr, fma(yi, yi, yy));
             }
-            const double tol = 256.0 * kEps * cnorm;
-            if (!(rr <= tol * tol * yy)) res_ok = false;
+#pragma unroll
+            for (int m = 4; m >= 1; m >>= 1) {
+                rr += shfl_xor(rr, m);
+                yy += shfl_xor(yy, m);
+            }
+            if (j < n && !(rr <= tol * tol * yy)) res_ok = false;
         }
         res_ok = __syncthreads_and(res_ok);
-        block_sum2_max<NB>(acc, red);           // acc[0], acc[1] summed, acc[2] the block's max
         const bool orth_ok = acc[2] <= kOrthTol;
         if (res_ok && orth_ok) return true;
         if (it >= max_updates) return false;
@@ -305,18 +336,23 @@ __device__ bool refine(int n, const double* Cre, const double* Cim, double* Yre,
         __syncthreads();                       // E visible
         Strip<NB> Yn;
         Yn.load(Yre, Yim, LD, row0);
-        cgemm<NB, false>(Yn, Yre, Yim, Pre, Pim, LD, row0);
+        cgemm<NB>(Yn, Yre, Yim, Pre, Pim, LD, row0);
         __syncthreads();                       // every warp is done reading Y
         Yn.store(Yre, Yim, LD, row0);
         __syncthreads();
     }
 }
 
+// Bound by the FP64 tensor cores (three passes of products are 94 K cycles of MMAs a pair at n = 54), with
+// enough pairs on an SM that one's barriers, norms and loads run under another's MMAs: without C in
+// shared memory two pairs of n = 54 fit (108 KB and 128 registers a thread; with C one, 161 KB).
+// Microseconds for 4,096 pairs, C staged -> read as fragments: n = 8 23 -> 21, 16 89 -> 85, 24 219 -> 213, 32 476 -> 393,
+// 40 1,046 -> 845, 48 2,034 -> 1,366, 54 2,622 -> 1,937, 62 3,190 -> 2,930.
 template <int NP>
-__global__ void __launch_bounds__(NP * 4, 1) k_refine_c(int n, int batch, Workspace ws, double* __restrict__ W,
+__global__ void __launch_bounds__(NP * 4, NP <= 56 ? 128 / NP : 1) k_refine_c(int n, int batch, Workspace ws, double* __restrict__ W,
                                                       double2* __restrict__ X, int* __restrict__ info,
                                                       int max_updates) {
-    constexpr int NB = NP / 8, LD = NP + 4, NT = NP * 4;
+    constexpr int LD = NP + 4, NT = NP * 4;
     using L = RefineCSmem<NP>;
     const int b = blockIdx.x;
     if (b >= batch) return;
@@ -332,8 +368,6 @@ __global__ void __launch_bounds__(NP * 4, 1) k_refine_c(int n, int batch, Worksp
         return;
     }
     extern __shared__ __align__(16) unsigned char smem[];
-    double* Cre = reinterpret_cast<double*>(smem + L::Cre);
-    double* Cim = reinterpret_cast<double*>(smem + L::Cim);
     double* Yre = reinterpret_cast<double*>(smem + L::Yre);
     double* Yim = reinterpret_cast<double*>(smem + L::Yim);
     double* Pre = reinterpret_cast<double*>(smem + L::Pre);
@@ -341,36 +375,20 @@ __global__ void __launch_bounds__(NP * 4, 1) k_refine_c(int n, int batch, Worksp
     double* lam = reinterpret_cast<double*>(smem + L::lam);
     double* red = reinterpret_cast<double*>(smem + L::red);
     int* order = reinterpret_cast<int*>(smem + L::order);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::bar);
     const size_t mat = static_cast<size_t>(n) * n;
     double2* Xb = X + mat * b;
-    // ---- C (both planes, one bulk copy of the stash) and Y (the X buffer, complex -> planar)
-    if (tid == 0) { mbar_init(bar, 1); fence_mbar_init(); }
-    __syncthreads();
-    if (tid == 0) {
-        const uint32_t bytes = static_cast<uint32_t>(2 * L::plane);
-        mbar_arrive_expect_tx(bar, bytes);
-        bulk_g2s(Cre, static_cast<const char*>(ws.log) + 16 * static_cast<size_t>(ws.log_stride) * b, bytes, bar);
-    }
+    const double* Cg = reinterpret_cast<const double*>(static_cast<const char*>(ws.log) +
+                                                       16 * static_cast<size_t>(ws.log_stride) * b);
+    // ---- Y (the X buffer, complex -> planar)
+#pragma unroll 7
     for (int idx = tid; idx < NP * NP; idx += NT) {
         const int c = idx / NP, r = idx - c * NP;
         const double2 v = (r < n && c < n) ? Xb[r + static_cast<size_t>(c) * n] : make_double2(0.0, 0.0);
         Yre[c * LD + r] = v.x;
         Yim[c * LD + r] = v.y;
     }
-    if (!mbar_wait_bounded(bar, 0, kMaxPolls)) {
-        atomicOr(info + b, kInfoCopyTimeout);
-        mbar_wait_bounded(bar, 0, kMaxPolls);
-    }
     __syncthreads();
-    double cn[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int idx = tid; idx < NP * NP; idx += NT) {
-        const int c = idx / NP, r = idx - c * NP;
-        cn[0] = fma(Cre[c * LD + r], Cre[c * LD + r], fma(Cim[c * LD + r], Cim[c * LD + r], cn[0]));
-    }
-    block_sum4<NB>(cn, red);
-    const double cnorm = sqrt(cn[0]);
-    if (!refine<NP>(n, Cre, Cim, Yre, Yim, Pre, Pim, lam, red, cnorm, max_updates)) {
+    if (!refine<NP>(n, Cg, Cg + NP * LD, Yre, Yim, Pre, Pim, lam, red, max_updates)) {
         if (tid == 0) {                        // the FP64 fallback redoes this pair
             ws.flag[b] = 2;
             if (ws.redo_count) atomicAdd(ws.redo_count, 1ull);
@@ -380,15 +398,11 @@ __global__ void __launch_bounds__(NP * 4, 1) k_refine_c(int n, int batch, Worksp
     if (tid == 0) ws.flag[b] = 0;
     // ---- outputs: W ascending and Y's columns alike (a swap can only come from eigenvalues the
     // complex64 start ordered within its rounding; the columns follow their eigenvalues)
-    if (tid == 0) {
-        for (int j = 0; j < n; ++j) order[j] = j;
-        for (int j = 1; j < n; ++j) {                      // insertion sort by lam (stable)
-            const int o = order[j];
-            const double v = lam[o];
-            int k = j - 1;
-            while (k >= 0 && lam[order[k]] > v) { order[k + 1] = order[k]; --k; }
-            order[k + 1] = o;
-        }
+    for (int j = tid; j < n; j += NT) {                    // stable rank (every lam is finite here)
+        const double v = lam[j];
+        int k = 0;
+        for (int i = 0; i < n; ++i) k += lam[i] < v || (lam[i] == v && i < j);
+        order[k] = j;
     }
     __syncthreads();
     for (int j = tid; j < n; j += NT) W[static_cast<size_t>(n) * b + j] = lam[order[j]];
