@@ -57,11 +57,11 @@ STAGE_BYTES = {"reduce": 32 * N * N, "tridiag": 0, "eig": 16 * N, "back": 16 * N
 # DRAM bytes (read + write) per pair of each FP64 stage at n = 54: ncu's dram__bytes_read.sum +
 # dram__bytes_write.sum of each stage kernel, one capture of a 16,384-pair solve of this workload
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum --clock-control none \
-#       -k regex:"k_potrf_warp|k_hegst_col|k_hetrd_reg|k_tridiag_values|k_tridiag_invit|k_back_dmma" -s 6 -c 6 \
+#       -k regex:"k_reduce_dmma|k_hetrd_reg|k_tridiag|k_back_dmma" -s 12 -c 6 \
 #       python bench.py --pairs 16384 --steps 1 --warmup 1 --no-e2e --no-cpu --forms fp64 --sample 64
 # divided by the pairs.  Traffic grows in proportion to the pairs a launch processes, so traffic per
 # launch = this x pairs per launch.
-TRAFFIC_PER_PAIR_N54 = {"reduce": 51.4e3 + 119.8e3, "tridiag": 51.9e3, "eig": 0.9e3 + 21.1e3, "back": 157.3e3}
+TRAFFIC_PER_PAIR_N54 = {"reduce": 123.7e3, "tridiag": 52.5e3, "eig": 0.9e3 + 21.0e3, "back": 114.5e3}
 TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum per pair of a 16,384-pair solve of this "
                   "workload by the current stage kernels (one capture of all six), scaled to the launch's pairs")
 

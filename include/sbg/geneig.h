@@ -107,10 +107,11 @@ enum { SBG_CACHE_AUTO = 0, SBG_CACHE_NO_DISK = 1, SBG_CACHE_NONE = 2 }; /* Cache
 enum { SBG_PRECISION_FP64 = 0, SBG_PRECISION_MIXED = 1 };
 
 typedef struct {
-    int batches_per_block;    /* pairs per CTA; 0 = auto (ctor arg, hpp:99): of the warp-per-pair Cholesky and
-                                 Householder kernels for n <= 65 (1, 2 or 4), of the QL rotation stage above */
-    int force_block_dim_x;    /* threads per CTA of the CTA-per-pair Householder (66 <= n <= 84): 128 or 256;
-                                 0 = auto (hpp:100) */
+    int batches_per_block;    /* pairs per CTA; 0 = auto (ctor arg, hpp:99).  1, 2 or 4 for n <= 65, where it
+                                 shapes the mixed form's warp-per-pair Householder; the FP64 kernels choose
+                                 their own CTAs from n and only report it */
+    int force_block_dim_x;    /* 128 or 256; 0 = auto (hpp:100).  Checked, kept and reported; every kernel
+                                 chooses its own CTA size from n */
     int tuning_mode;          /* SBG_TUNING_*  (hpp:101) */
     int cache_mode;           /* SBG_CACHE_*   (hpp:102) */
     int precision;            /* SBG_PRECISION_FP64 (plain drop-in) or SBG_PRECISION_MIXED */
@@ -168,7 +169,7 @@ int sbg_solver_refine_redo_pairs(sbg_solver* s, long long* count, int reset);
 /* Per-stage timing: when enabled, every launch records CUDA events around each stage
  * kernel on the launch stream.  sbg_solver_read_stage_times synchronizes on them and
  * returns, per stage (0 = Cholesky + two-sided reduction, 1 = Householder
- * tridiagonalisation, 2 = tridiagonal eigensolve (QL, or QL + refinement for the mixed
+ * tridiagonalisation, 2 = tridiagonal eigensolve (with Y = Q Z and the refinement for the mixed
  * form), 3 = back-transform), the summed milliseconds and the number of kernel launches,
  * then clears the record. */
 int sbg_solver_enable_stage_timing(sbg_solver* s, int enable);
@@ -182,14 +183,13 @@ size_t sbg_workspace_bytes_per_pair(int n, int precision);
 size_t sbg_workspace_bytes(int n, int precision, int pairs);
 
 /* The solver's schedule as eight ints (no counterpart in the reference, whose schedule is its
- * (batches per block, block size) pair): [0] threads per CTA of the CTA-per-pair Householder,
- * [1] pairs per CTA of the warp-per-pair Cholesky / Householder kernels, [2] 1 = the exact-n
- * column kernels where they exist (n = 32, 54), [3] lanes per column of the column back-transform
- * (1 or 2), [4] pairs per CTA of the QL rotation stage, [5] pairs per CTA of the QL scalar
- * chain, [6] reflectors per pass of the column back-transform's Q application (1 or 2), [7] 1 = the
- * triangular stages above n = 56 (Cholesky, reduction, X = L^{-H} Y) by the blocked kernels on the
- * FP64 tensor cores, and above n = 84 the Householder by its own one-pass kernel, 0 = by the
- * one-CTA / cluster kernels that also do the Householder (0 or 1).
+ * (batches per block, block size) pair).  Three shape kernels: [1] pairs per CTA of the mixed form's
+ * complex64 Householder for n <= 63 (1, 2 or 4), [5] pairs per CTA of the QL chain that solves
+ * flagged pairs again above n = 63 (32, 64, 128 or 256), [7] above n = 84, 1 = Cholesky, reduction and
+ * X = L^{-H} Y on the FP64 tensor cores and the Householder by its own one-pass kernel, 0 = the
+ * one-CTA / cluster kernels (0 or 1).  The others are kept from earlier tables, checked against their
+ * ranges and reported, and no kernel depends on them: [0] a CTA size (128 or 256), [2] 0 or 1, [3] 1 or
+ * 2, [4] 1 .. 16, [6] 1 or 2.
  * set_schedule replaces it (values checked against their ranges and the device's shared memory;
  * SBG_ERR_INVALID_VALUE otherwise), for callers that tune outside the library. */
 int sbg_solver_schedule(const sbg_solver* s, int* out8);

@@ -19,8 +19,8 @@
 // a full tile in shared memory by 256 threads (66 <= n <= 84), or the triangle in L2 (n > 84).
 // Microseconds per 1,000 pairs before -> now: n = 24 48 -> 20, 32 80 -> 31, 47 191 -> 113, 54 284 -> 141,
 // 72 1,197 -> 422, 96 2,013 -> 737, 128 4,600 -> 2,070.  It is bound by the latency of a step's chain
-// (column sum, norm, square root, reflector) at the few pairs an SM holds and by the load/store unit (55 % at
-// n = 54); FP64 pipe 37 % busy.
+// (column sum, norm, square root, reflector) at the few pairs an SM holds and by the load/store unit (62 % at
+// n = 54); FP64 pipe 47 % busy.
 #include "kernels.cuh"
 #include "stages.cuh"
 

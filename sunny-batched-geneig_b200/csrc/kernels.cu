@@ -155,8 +155,8 @@ __global__ void k_ql_chain(int n, int batch, Workspace ws, double* __restrict__ 
 // more cluster members than lanes gets every vector as if it stood alone, and k_tridiag_ortho
 // orthonormalises them.  Every vector must pass ||T z - lambda z|| <= kInvitTol ||T||; a pair with a
 // failed vector or a T that is not finite is recomputed by the QL instead.
-// Bound by the latency of the lanes' recurrences with the 6-9 pairs per SM that the lane scratch leaves room
-// for (FP64 pipe 10 % busy at 1.95 ms).  32,768 pairs at n = 54: 1.95 -> 1.12 ms with the backward-only first solve,
+// Bound by the latency of the lanes' recurrences with the pairs that the lane scratch leaves room for (8 per
+// SM at n = 54; FP64 pipe 13 % busy).  32,768 pairs at n = 54: 1.95 -> 1.12 ms with the backward-only first solve,
 // the lane count below, running pointers, and cluster members in the main batches instead of three rounds of
 // their own for one close pair of eigenvalues in a spectrum.
 // Per-lane scratch (1/u and the vector) is interleaved [i * ld + lane]: lane-parallel

@@ -80,10 +80,11 @@ __host__ __device__ constexpr int refine_np(int n) { return (n + 7) / 8 * 8; }
 __host__ __device__ constexpr int refine_ld(int n) { return refine_np(n) + 4; }
 __host__ __device__ constexpr int refine_stash_entries(int n) { return refine_np(n) * refine_ld(n); }
 constexpr int kMixedMaxN = 63;       // inverse iteration (no rotation log, so the stash is free)
-// Entries of the rotation-log region the tensor-core kernels of n > 56 use as scratch between the
-// eigensolves (csrc/reduce_tc.cu): the inverted 32 x 32 diagonal blocks of L, and above n = 84 the
-// Q application's copy of Z (n^2 doubles), block of reflectors (n x 32), T (32 x 32) and V^H Y
-// (32 x n).  Never more than the default rotation-log capacity (3 n^2 / 2 + 8 n + 16); the region
+// Entries of the rotation-log region that csrc/reduce_tc.cu uses as scratch before and after the
+// eigensolve: the inverted 32 x 32 diagonal blocks of L (n > kReduceDmmaMaxN), and the Q application's
+// (n > kBackStreamMaxN) copy of Z (n^2 doubles), block of reflectors (n x 32), T (32 x 32) and V^H Y
+// (32 x n).  The default region also holds k_reduce_dmma's W (n x n, n > 56), k_hetrd_tri's packed triangle
+// and k_back_dmma_stream's copy of Z.  Never more than the default rotation-log capacity (3 n^2 / 2 + 8 n + 16); the region
 // is kept at least this large when a smaller log capacity is asked for.
 __host__ __device__ constexpr int tc_scratch_entries(int n) {
     return n <= 56 ? 0
@@ -127,7 +128,7 @@ enum BackMode : int {
 //               -- the reference's "batches per block"
 //   reduce_tc   n > 84: the triangular stages on the FP64 tensor cores (k_reduce_dmma or k_reduce_tc,
 //               then the Householder alone by k_hetrd_reg or k_hetrd_tri; the back-transform by
-//               k_back_dmma or k_back_q_tc + k_back_tc) instead of k_reduce_mid / k_reduce_big doing all
+//               k_back_dmma, k_back_dmma_stream or k_back_q_tc + k_back_tc) instead of k_reduce_mid / k_reduce_big doing all
 //               three and k_back_big.  Up to n = 84 there is no other.
 struct LaunchShape {
     int pair_warps = 2;
@@ -263,6 +264,8 @@ cudaError_t launch_ql_chain(int n, int batch, const Workspace& ws, double* W, in
 // Kernels one full reduce launch (kReduceFull) issues for order n: the reduction and, above kSmallMaxN
 // with the tensor-core reduction (tc), the Householder kernel.
 inline int reduce_kernel_count(int n, bool tc = false) { return n > kSmallMaxN && tc ? 2 : 1; }
+// Kernels of a kBackFull launch (Q Z and L^{-H} apart above kBackStreamMaxN).
+inline int back_kernel_count(int n, bool tc) { return n > kBackStreamMaxN && tc ? 2 : 1; }
 
 // ---- Eigensolve of the tridiagonals, FP64: eigenvalues by bisection (k_tridiag_values), eigenvectors by
 // inverse iteration (k_tridiag_invit), orthonormalised together where many eigenvalues are close

@@ -249,7 +249,9 @@ struct sbg_solver {
                    "eigensolve kernels (FP64 redo)");
         check_cuda(sbg::launch_back(sbg::kBackFull, n, cnt, sel, X, info, sched.shape(), stream),
                    "back-transform kernel (FP64 redo)");
-        stage_end(stream, ev, 3, 1 + 1 + (n > sbg::kSmallMaxN ? 0 : 1) + sbg::eig_kernel_count(n, false) + 1);
+        stage_end(stream, ev, 3, 1 + sbg::reduce_kernel_count(n, sched.reduce_tc != 0) + (n > sbg::kSmallMaxN ? 0 : 1) +
+                                     sbg::eig_kernel_count(n, false) +
+                                     sbg::back_kernel_count(n, sched.reduce_tc != 0));
     }
 
     // One chunk of at most chunk_pairs pairs through the three stages.
@@ -282,7 +284,7 @@ struct sbg_solver {
         stage_begin(stream, &ev);
         check_cuda(sbg::launch_back(mixed ? sbg::kBackLOnly : sbg::kBackFull, n, cnt, ws, X, info, sched.shape(),
                                     stream), "back-transform kernel");
-        stage_end(stream, ev, 3, !mixed && n > 56 && sched.reduce_tc ? 2 : 1);
+        stage_end(stream, ev, 3, sbg::back_kernel_count(n, !mixed && sched.reduce_tc != 0));
     }
 
     // Host buffers in, host buffers out, chunks round-robin over nstreams internal streams.  A goes

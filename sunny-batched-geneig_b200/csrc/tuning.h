@@ -23,12 +23,12 @@ namespace sbg {
 struct Schedule {
     int hetrd_threads = 256;    // what block_dim_x reports and force_block_dim_x sets (128 or 256); no kernel's
                                 // CTA size depends on it
-    int pair_warps = 2;         // pairs (warps) per CTA of k_hetrd_warp_c64
-                                // (n <= 65): the reference's batches per block
+    int pair_warps = 2;         // pairs (warps) per CTA of k_hetrd_warp_c64 (mixed form, n <= 63); what
+                                // batches_per_block reports and sets for n <= 65
     int col_exact = 1;          // 0 or 1, kept from earlier tables: no kernel depends on it
     int back_lanes = 1;         // 1 or 2, kept from earlier tables: no kernel depends on it
     int back_qpass = 1;         // 1 or 2, likewise
-    int reduce_tc = 0;          // n > 84: the triangular stages on the tensor cores (k_reduce_tc, k_back_tc)
+    int reduce_tc = 0;          // n > 84: 1 = the tensor-core stages, 0 = csrc/bigsolve.cu's
     int ql_warps = 4;           // batches_per_block above n = 65, bounded by shared memory; no kernel's shape
                                 // depends on it
     int chain_threads = 128;    // pairs (threads) per CTA of the QL scalar-chain kernel (n > 63, flagged pairs)
@@ -49,7 +49,7 @@ struct TuneRequest {
     int n = 0;
     int device = 0;
     int precision = 0;
-    int force_threads = 0;      // 0 = choose; else 128 or 256 for the CTA-per-pair Householder
+    int force_threads = 0;      // 0 = choose; else 128 or 256 (hetrd_threads)
     int force_bpb = 0;          // 0 = choose; else pairs per CTA (pair_warps for n <= 65, else ql_warps)
     bool autotune = false;
     int cache_mode = 0;         // SBG_CACHE_*
