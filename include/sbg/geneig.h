@@ -107,9 +107,8 @@ enum { SBG_CACHE_AUTO = 0, SBG_CACHE_NO_DISK = 1, SBG_CACHE_NONE = 2 }; /* Cache
 enum { SBG_PRECISION_FP64 = 0, SBG_PRECISION_MIXED = 1 };
 
 typedef struct {
-    int batches_per_block;    /* pairs per CTA; 0 = auto (ctor arg, hpp:99).  1, 2 or 4 for n <= 65, where it
-                                 shapes the mixed form's warp-per-pair Householder; the FP64 kernels choose
-                                 their own CTAs from n and only report it */
+    int batches_per_block;    /* pairs per CTA; 0 = auto (ctor arg, hpp:99).  1, 2 or 4 for n <= 65.  Checked,
+                                 kept and reported; every kernel chooses its own CTAs from n */
     int force_block_dim_x;    /* 128 or 256; 0 = auto (hpp:100).  Checked, kept and reported; every kernel
                                  chooses its own CTA size from n */
     int tuning_mode;          /* SBG_TUNING_*  (hpp:101) */
@@ -183,12 +182,12 @@ size_t sbg_workspace_bytes_per_pair(int n, int precision);
 size_t sbg_workspace_bytes(int n, int precision, int pairs);
 
 /* The solver's schedule as eight ints (no counterpart in the reference, whose schedule is its
- * (batches per block, block size) pair).  Three shape kernels: [1] pairs per CTA of the mixed form's
- * complex64 Householder for n <= 63 (1, 2 or 4), [5] pairs per CTA of the QL chain that solves
+ * (batches per block, block size) pair).  Two shape kernels: [5] pairs per CTA of the QL chain that solves
  * flagged pairs again above n = 63 (32, 64, 128 or 256), [7] above n = 84, 1 = Cholesky, reduction and
  * X = L^{-H} Y on the FP64 tensor cores and the Householder by its own one-pass kernel, 0 = the
  * one-CTA / cluster kernels (0 or 1).  The others are kept from earlier tables, checked against their
- * ranges and reported, and no kernel depends on them: [0] a CTA size (128 or 256), [2] 0 or 1, [3] 1 or
+ * ranges and reported, and no kernel depends on them: [0] a CTA size (128 or 256), [1] pairs per
+ * CTA (1, 2 or 4), [2] 0 or 1, [3] 1 or
  * 2, [4] 1 .. 16, [6] 1 or 2.
  * set_schedule replaces it (values checked against their ranges and the device's shared memory;
  * SBG_ERR_INVALID_VALUE otherwise), for callers that tune outside the library. */

@@ -4,8 +4,8 @@
 //   reduce   k_reduce_dmma (reduce_dmma.cu): B = L L^H and C = L^{-1} A L^{-H}; L into the
 //            workspace, C into the caller's X buffer.
 //   hetrd    k_hetrd_reg (hetrd_reg.cu): Householder tridiagonalisation of C, reflectors and
-//            (d, e, tau) into the workspace; the mixed form (n <= 63) runs it in complex64
-//            (k_hetrd_warp_c64).
+//            (d, e, tau) into the workspace; the mixed form (n <= 63) runs it in
+//            complex64.
 //   eig      k_tridiag_values (tridiag.cu: bisection on Sturm counts), k_tridiag_invit
 //            (eigenvectors by inverse iteration, one warp per pair) and k_tridiag_ortho
 //            (tridiag.cu: pairs with large clusters); k_ql_chain + k_ql_apply_rows (n > 63) or a
@@ -14,9 +14,8 @@
 //   back     k_back_dmma (back_dmma.cu): X = L^{-H} Q Z, written over Z (the mixed form:
 //            Y = Q Z, then X = L^{-H} Y after the refinement).
 //
-// The split follows where the work is latency bound: the QL recurrence is a
-// dependent scalar chain per pair, so it runs with many pairs per SM, while the
-// BLAS2-shaped stages run a warp or a CTA per pair.
+// Every stage gives a pair one warp or one CTA.  The redo QL's recurrence is a dependent scalar chain per
+// pair, so it runs a thread per pair.
 #include "kernels.cuh"
 #include "stages.cuh"
 
@@ -30,87 +29,6 @@ namespace sbg {
 namespace {
 
 __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-
-constexpr int kMaxPairWarps = 4;      // k_hetrd_warp_c64: 1, 2 or 4 pairs (warps) per CTA
-
-// ----------------------------------------------------------------------------- k_hetrd_warp_c64
-// Mixed form, Householder stage in complex64: one WARP per pair (n <= 65).  C's lower triangle
-// (FP64, in the X buffer) is rounded to complex64 into a packed tile (8 B per entry: 11.9 KB at
-// n = 54) and tridiagonalised by hetrd_warp_packed<float>.  Outputs go where the FP64 form's
-// Householder (k_hetrd_reg) puts them, promoted to FP64, so the
-// FP64 eigen- and back-transform kernels run on them unchanged: reflectors in LV's rows above the
-// superdiagonal, (d, e), and tau rescaled in FP64 so that each H = I - tau v v^H is unitary to
-// FP64 rounding for the promoted v (|tau|^2 ||v||^2 = 2 Re tau; the FP32 tau satisfies it only to
-// ~1e-7), which keeps the refinement's Y = Q Z orthonormal to the level of Z.  C itself (FP64) is
-// also written to the pair's stash in the refinement's tile format (refine_stash_entries), since
-// X, where the reduction left it, is overwritten before the refinement runs.
-__host__ __device__ inline size_t hetrd_c64_bytes(int n) {
-    return align_up(8 * static_cast<size_t>(n) * (n + 1) / 2, 16) + 8 * 2 * n + 2 * align_up(4 * n, 16) +
-           align_up(8 * n, 16) + 16;
-}
-
-__device__ __forceinline__ double2* refine_stash(const Workspace& ws, int b) {
-    return reinterpret_cast<double2*>(static_cast<char*>(ws.log) + 16 * static_cast<size_t>(ws.log_stride) * b);
-}
-
-__global__ void __launch_bounds__(32 * kMaxPairWarps) k_hetrd_warp_c64(int n, int batch,
-                                                                              const double2* __restrict__ C,
-                                                                              Workspace ws, int* __restrict__ info) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (b >= batch) return;
-    if (info[b] != 0) return;
-    extern __shared__ __align__(16) unsigned char smem[];
-    unsigned char* base = smem + hetrd_c64_bytes(n) * warp;
-    float2* P = reinterpret_cast<float2*>(base);
-    float2* vb = reinterpret_cast<float2*>(base + align_up(8 * static_cast<size_t>(n) * (n + 1) / 2, 16));
-    float2* wb = vb + n;
-    float* d_s = reinterpret_cast<float*>(wb + n);
-    float* e_s = d_s + align_up(4 * n, 16) / 4;
-    float2* tau_s = reinterpret_cast<float2*>(e_s + align_up(4 * n, 16) / 4);
-    const size_t mat = static_cast<size_t>(n) * n;
-    const double2* Cb = C + mat * b;
-    // stash: C full Hermitian, planar (re plane, then im plane), column-major, ld = LD, zero padded
-    const int NP = refine_np(n), LD = refine_ld(n);
-    double* sre = reinterpret_cast<double*>(refine_stash(ws, b));
-    double* sim = sre + static_cast<size_t>(NP) * LD;
-    for (int j = 0; j < NP; ++j) {
-        float2* col = P + pk(j, n) - j;
-        for (int i = j + lane; i < NP; i += 32) {
-            const bool in = i < n && j < n;
-            double2 v = in ? Cb[i + static_cast<size_t>(j) * n] : make_double2(0.0, 0.0);
-            if (i == j) v.y = 0.0;
-            if (in) col[i] = make_float2(static_cast<float>(v.x), static_cast<float>(v.y));
-            sre[j * LD + i] = v.x;
-            sim[j * LD + i] = v.y;
-            if (i != j) { sre[i * LD + j] = v.x; sim[i * LD + j] = -v.y; }
-        }
-    }
-    __syncwarp();
-    hetrd_warp_packed<float>(P, n, d_s, e_s, tau_s, vb, wb);
-    double2* LVg = ws.LV + mat * b;
-    for (int k = 0; k + 1 < n; ++k) {                    // LV(k, k+1) = v_k(k+1) = 1
-        const float2* col = P + pk(k, n) - k;            // col[i] = v_k(i), i >= k + 2
-        double s2 = 0.0;
-        for (int i = k + 1 + lane; i < n; i += 32) {
-            const double2 v = (i == k + 1) ? make_double2(1.0, 0.0)
-                                           : make_double2(static_cast<double>(col[i].x), static_cast<double>(col[i].y));
-            LVg[k + static_cast<size_t>(i) * n] = v;
-            s2 = fma(v.x, v.x, fma(v.y, v.y, s2));
-        }
-        s2 = warp_sum(s2);
-        if (lane == 0) {
-            const double tr = tau_s[k].x, ti = tau_s[k].y, t2 = tr * tr + ti * ti;
-            const double sc = t2 > 0.0 ? 2.0 * tr / (t2 * s2) : 0.0;
-            ws.tau[static_cast<size_t>(n) * b + k] = make_double2(tr * sc, ti * sc);
-        }
-    }
-    for (int i = lane; i < n; i += 32) {
-        ws.d[static_cast<size_t>(n) * b + i] = d_s[i];
-        ws.e[static_cast<size_t>(n) * b + i] = (i + 1 < n) ? static_cast<double>(e_s[i]) : 0.0;
-        if (i + 1 == n) ws.tau[static_cast<size_t>(n) * b + i] = make_double2(0.0, 0.0);
-    }
-}
 
 // ----------------------------------------------------------------------------- k_ql_chain
 // The rotation-log QL's first half, for the pairs flagged kFlagRedo only (they keep the flag, or get 3
@@ -460,10 +378,6 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
 }
 
 // Pairs (warps) per CTA of the warp-per-pair kernels: 1, 2 or 4 (anything else: the default 2).
-inline int pair_warps_of(const LaunchShape& s) {
-    return (s.pair_warps == 1 || s.pair_warps == 2 || s.pair_warps == 4) ? s.pair_warps : 2;
-}
-
 template <class K>
 void set_max_smem_once(K kernel, SmemOptIn& rec) {
     set_smem_limit(reinterpret_cast<const void*>(kernel), rec, max_smem_optin());
@@ -647,26 +561,6 @@ cudaError_t launch_eig(int n, int batch, const Workspace& ws, double* W, double2
     if (batch <= 0) return cudaSuccess;
     if (n > kInvitQlMaxN) return launch_ql_rows(n, batch, ws, W, X, info, chain_threads, stream);
     return launch_eig_invit(n, batch, ws, W, X, info, false, stream);
-}
-
-size_t hetrd_c64_smem_bytes(int n) { return hetrd_c64_bytes(n) * kMaxPairWarps; }
-
-size_t pair_kernels_smem_bytes(int n, int pair_warps) {
-    return hetrd_c64_bytes(n) * static_cast<size_t>(pair_warps);
-}
-
-cudaError_t launch_hetrd_c64(int n, int batch, const double2* C, const Workspace& ws, int* info,
-                             const LaunchShape& shape, cudaStream_t stream) {
-    if (batch <= 0) return cudaSuccess;
-    if (n < 1 || n > kMixedMaxN || !C || !info || !ws.LV || ws.log_stride < refine_stash_entries(n))
-        return cudaErrorInvalidValue;
-    const int pw = pair_warps_of(shape);
-    const size_t smem = hetrd_c64_bytes(n) * pw;
-    if (smem > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
-    static SmemOptIn f;
-    set_max_smem_once(k_hetrd_warp_c64, f);
-    k_hetrd_warp_c64<<<(batch + pw - 1) / pw, 32 * pw, smem, stream>>>(n, batch, C, ws, info);
-    return cudaGetLastError();
 }
 
 // ----------------------------------------------------------------------------- k_pull_pairs

@@ -124,14 +124,11 @@ enum BackMode : int {
 };
 
 // Launch shape of the stage kernels, the part of a schedule the autotuner varies:
-//   pair_warps  pairs (one warp each) per CTA of k_hetrd_warp_c64 (the mixed form, n <= 63): 1, 2 or 4
-//               -- the reference's "batches per block"
 //   reduce_tc   n > 84: the triangular stages on the FP64 tensor cores (k_reduce_dmma or k_reduce_tc,
 //               then the Householder alone by k_hetrd_reg or k_hetrd_tri; the back-transform by
 //               k_back_dmma, k_back_dmma_stream or k_back_q_tc + k_back_tc) instead of k_reduce_mid / k_reduce_big doing all
 //               three and k_back_big.  Up to n = 84 there is no other.
 struct LaunchShape {
-    int pair_warps = 2;
     int reduce_tc = 0;
 };
 
@@ -152,22 +149,19 @@ cudaError_t launch_hetrd_reg(int n, int batch, const double2* C, const Workspace
 cudaError_t launch_eig(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                        int chain_threads, cudaStream_t stream);
 // Mixed form (n <= kMixedMaxN), after the FP64 reduction left C in X:
-//   launch_hetrd_c64     complex64 Householder (warp per pair); FP64-promoted reflectors, tau (made
+//   launch_hetrd_c64     complex64 Householder (csrc/hetrd_reg.cu); FP64-promoted reflectors, tau (made
 //                        unitary in FP64) and T into the workspace, C into the pair's stash;
 //   launch_eig_mixed     eigenpairs of that T (launch_eig_invit), Y = Q Z
 //                        (launch_back(kBackQOnly)), then launch_refine_mixed: FP64 Ogita-Aishima
 //                        refinement of (W, Y) against the stashed C on the FP64 tensor cores, and
 //                        the FP64 fallback for pairs it cannot take;
 //   launch_back(kBackLOnly)  X = L^{-H} Y.
-cudaError_t launch_hetrd_c64(int n, int batch, const double2* C, const Workspace& ws, int* info,
-                             const LaunchShape& shape, cudaStream_t stream);
+cudaError_t launch_hetrd_c64(int n, int batch, const double2* C, const Workspace& ws, int* info, cudaStream_t stream);
 cudaError_t launch_refine_mixed(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                                 int refine_steps, cudaStream_t stream);
 cudaError_t launch_eig_mixed(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                              int refine_steps, const LaunchShape& shape, cudaStream_t stream);
 size_t hetrd_c64_smem_bytes(int n);
-// Dynamic shared memory of a CTA of k_hetrd_warp_c64 with pair_warps pairs.
-size_t pair_kernels_smem_bytes(int n, int pair_warps);
 size_t refine_c_smem_bytes(int n);
 size_t mixed_fallback_smem_bytes(int n);
 // Host-buffer path: copies `count` pairs of n x n column-major matrices from pinned host memory

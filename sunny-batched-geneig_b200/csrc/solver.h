@@ -269,7 +269,7 @@ struct sbg_solver {
         const bool mixed = precision == SBG_PRECISION_MIXED;
         stage_begin(stream, &ev);
         if (mixed)
-            check_cuda(sbg::launch_hetrd_c64(n, cnt, X, ws, info, sched.shape(), stream), "complex64 hetrd kernel");
+            check_cuda(sbg::launch_hetrd_c64(n, cnt, X, ws, info, stream), "complex64 hetrd kernel");
         else
             check_cuda(sbg::launch_hetrd(n, cnt, X, ws, info, stream), "hetrd kernel");
         stage_end(stream, ev, 1, n > sbg::kSmallMaxN ? 0 : 1);       // large n: inside the reduce kernel

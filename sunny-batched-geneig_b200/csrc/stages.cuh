@@ -417,204 +417,8 @@ __device__ __forceinline__ void ql_log_apply_row(const cplx<R>* log, int cap, cp
     }
 }
 
-// ============================================================================ hetrd, one warp, packed
+// ============================================================================ packed lower triangle
 // Column-major packed lower triangle: A(i, j), i >= j, at P[pk(j, n) + i - j].
 __host__ __device__ __forceinline__ int pk(int j, int n) { return j * n - (j * (j - 1)) / 2; }
-
-// ---- warp helpers of hetrd_warp_packed (one warp, packed lower triangle, lane rows L and m-1-L)
-
-// LAPACK zlarfg on x[0..m) (x[0] = alpha): beta, tau, and the scale that turns x[1..m) into the
-// reflector's tail (v = (1, x[1..m) * scale)).  Every lane gets the same values.
-template <typename R>
-struct WarpReflector { cplx<R> tau, scale; R beta; };
-
-template <typename R>
-__device__ __forceinline__ WarpReflector<R> warp_reflector(const cplx<R>* x, int m) {
-    const int lane = threadIdx.x & 31;
-    R s2 = R(0);
-    for (int i = 1 + lane; i < m; i += 32) s2 += cabs2(x[i]);
-    s2 = warp_sum(s2);
-    const cplx<R> alpha = x[0];
-    WarpReflector<R> f;
-    if (s2 == R(0) && alpha.y == R(0)) {
-        f.tau = mk<R>(R(0), R(0)); f.beta = alpha.x; f.scale = mk<R>(R(0), R(0));
-    } else {
-        const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + s2);
-        f.beta = alpha.x >= R(0) ? -nrm : nrm;
-        const R ib = R(1) / f.beta;                      // two reciprocals instead of four divisions
-        f.tau = mk<R>((f.beta - alpha.x) * ib, -alpha.y * ib);
-        const R ar = alpha.x - f.beta, ai = alpha.y;
-        const R id = R(1) / (ar * ar + ai * ai);
-        f.scale = mk<R>(ar * id, -ai * id);
-    }
-    return f;
-}
-
-// The reflector's vector into vb[0..m) (and its tail over x[1..m)); with tau = 0 (H = I) vb = e_0.
-template <typename R>
-__device__ __forceinline__ void warp_store_reflector(cplx<R>* x, int m, const WarpReflector<R>& f, cplx<R>* vb) {
-    const int lane = threadIdx.x & 31;
-    const bool id = f.tau.x == R(0) && f.tau.y == R(0);
-    __syncwarp();                                        // every lane has read x[0] and the norm terms
-    for (int i = lane; i < m; i += 32) {
-        if (id) { vb[i] = mk<R>(i == 0 ? R(1) : R(0), R(0)); continue; }
-        const cplx<R> v = (i == 0) ? mk<R>(R(1), R(0)) : cmul(x[i], f.scale);
-        vb[i] = v;
-        if (i > 0) x[i] = v;
-    }
-}
-
-// (A22 v)_r for the lane's rows r1 = lane and r2 = m-1-lane of the packed trailing matrix whose
-// column 0 starts at c0 (order m).  Each lane walks its two rows in ONE loop of uniform length (row
-// r1's terms, then row r2's), so no lane waits for the others' longer row: the pair has m-1 terms
-// in the lower row walk, m-1 in the mirrored column walk.  A22(r, j) sits at
-// c0 + r - j + sum_{t<j} (m - t): the address advances by (m - j - 1) from column j to j + 1.
-template <typename R>
-__device__ __forceinline__ void warp_hemv_rows(const cplx<R>* c0, int m, const cplx<R>* vb, cplx<R>& s1, cplx<R>& s2) {
-    using C = cplx<R>;
-    const int lane = threadIdx.x & 31;
-    const int h = (m + 1) >> 1;
-    const int r1 = lane, r2 = m - 1 - lane;
-    const bool own2 = lane < h && r2 != r1;
-    const C zero = mk<R>(R(0), R(0));
-    s1 = zero;
-    s2 = zero;
-    if (lane >= h) return;
-    const int tot = own2 ? r1 + r2 : r1;                 // lower walk length
-    const int sw = m - 1 - r1;
-    const int tot2 = own2 ? m - 1 : sw;                  // column walk length (== tot when own2)
-    const C* diag1 = c0 + (r1 * m - r1 * (r1 - 1) / 2); // A22(r1, r1)
-    const C* diag2 = c0 + (r2 * m - r2 * (r2 - 1) / 2); // A22(r2, r2)
-    C acc = zero, low1 = zero, u = zero, up1 = zero;
-    const C* pa = c0 + r1;
-    int jj = 0;
-    const C* cp = diag1 + 1;                             // next column-walk element
-    const C* vp = vb + r1 + 1;                           // its partner in v
-    bool lsw = false, usw = false;
-    const int both = tot < tot2 ? tot : tot2;
-    int t = 0;
-    for (; t < both; ++t) {
-        if (t == r1) { low1 = acc; acc = zero; pa = c0 + r2; jj = 0; lsw = true; }
-        if (t == sw) { up1 = u; u = zero; cp = diag2 + 1; vp = vb + r2 + 1; usw = true; }
-        acc = cfma(*pa, vb[jj], acc);
-        u = cfmac(*cp, *vp, u);
-        pa += m - jj - 1;
-        ++jj;
-        ++cp;
-        ++vp;
-    }
-    for (; t < tot; ++t) {                               // (only when the lengths differ)
-        if (t == r1) { low1 = acc; acc = zero; pa = c0 + r2; jj = 0; lsw = true; }
-        acc = cfma(*pa, vb[jj], acc);
-        pa += m - jj - 1;
-        ++jj;
-    }
-    for (; t < tot2; ++t) {
-        if (t == sw) { up1 = u; u = zero; cp = diag2 + 1; vp = vb + r2 + 1; usw = true; }
-        u = cfmac(*cp, *vp, u);
-        ++cp;
-        ++vp;
-    }
-    C low2 = zero, up2 = zero;
-    if (lsw) low2 = acc; else low1 = acc;
-    if (usw) up2 = u; else up1 = u;
-    C a1 = up1;
-    a1.x = fma(diag1[0].x, vb[r1].x, a1.x);
-    a1.y = fma(diag1[0].x, vb[r1].y, a1.y);
-    s1 = cadd(low1, a1);
-    if (own2) {
-        C a2 = up2;
-        a2.x = fma(diag2[0].x, vb[r2].x, a2.x);
-        a2.y = fma(diag2[0].x, vb[r2].y, a2.y);
-        s2 = cadd(low2, a2);
-    }
-}
-
-// A22 -= sum_q (v_q w_q^H + w_q v_q^H), q < NP, on the lane's rows r1 = lane and r2 = m-1-lane of the
-// packed trailing matrix at c0 (order m): r1 + 1 terms of row r1 (diagonal last), then r2 + 1 of row
-// r2, in one loop.  The terms of each entry are applied in q order; the diagonal entries stay real.
-template <typename R, int NP>
-__device__ __forceinline__ void warp_her2_rows(cplx<R>* c0, int m, const cplx<R>* const (&vq)[NP],
-                                               const cplx<R>* const (&wq)[NP]) {
-    using C = cplx<R>;
-    const int lane = threadIdx.x & 31;
-    const int h = (m + 1) >> 1;
-    const int r1 = lane, r2 = m - 1 - lane;
-    if (lane >= h) return;
-    const bool own2 = r2 != r1;
-    const int tot = own2 ? r1 + r2 + 2 : r1 + 1;
-    C* a = c0 + r1;
-    C vr[NP], wr[NP];
-#pragma unroll
-    for (int q = 0; q < NP; ++q) { vr[q] = vq[q][r1]; wr[q] = wq[q][r1]; }
-    int jj = 0;
-    C* dg1 = nullptr;
-    for (int t = 0; t < tot; ++t) {
-        if (t == r1 + 1) {
-            dg1 = a - (m - jj);
-            a = c0 + r2;
-#pragma unroll
-            for (int q = 0; q < NP; ++q) { vr[q] = vq[q][r2]; wr[q] = wq[q][r2]; }
-            jj = 0;
-        }
-        C tv = *a;
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-            tv = cfmsc(vr[q], wq[q][jj], tv);
-            tv = cfmsc(wr[q], vq[q][jj], tv);
-        }
-        *a = tv;
-        a += m - jj - 1;
-        ++jj;
-    }
-    // the diagonal entries (each row's last term) stay real
-    if (dg1 == nullptr) dg1 = a - (m - jj);
-    else a[-(m - jj)].y = R(0);
-    dg1->y = R(0);
-}
-
-// The Householder tridiagonalisation of hetrd_lower (LAPACK zhetd2's steps) run by ONE warp on a
-// packed lower triangle, for n <= 65.  At step k lane L owns trailing rows L and m-1-L (m = n-k-1),
-// which balances both the Hermitian matvec (m terms per row) and the rank-2 update (r+1 terms for
-// row r).  Only __syncwarp is needed.  The scaled reflector replaces A(k+2:n, k).
-// d, e, tau may be global memory (written by lane 0 as they are formed, d at the end);
-// vb, wb: n complex of shared scratch each.
-template <typename R>
-__device__ void hetrd_warp_packed(cplx<R>* P, int n, R* d, R* e, cplx<R>* tau, cplx<R>* vb, cplx<R>* wb) {
-    using C = cplx<R>;
-    const int lane = threadIdx.x & 31;
-    const C zero = mk<R>(R(0), R(0));
-    for (int k = 0; k + 1 < n; ++k) {
-        const int m = n - k - 1;
-        C* x = P + pk(k, n) + 1;                        // x[i] = A(k+1+i, k)
-        // ---- reflector, p = tau A22 v, w = p - tau/2 (p^H v) v
-        const WarpReflector<R> f = warp_reflector<R>(x, m);
-        if (lane == 0) { e[k] = f.beta; tau[k] = f.tau; }
-        warp_store_reflector<R>(x, m, f, vb);
-        __syncwarp();
-        C* c0 = P + pk(k + 1, n);
-        const int r1 = lane, r2 = m - 1 - lane, h = (m + 1) >> 1;
-        const bool own1 = lane < h, own2 = own1 && r2 != r1;
-        C s1, s2;
-        warp_hemv_rows<R>(c0, m, vb, s1, s2);
-        const C p1 = cmul(f.tau, s1), p2 = cmul(f.tau, s2);
-        C dot = zero;
-        if (own1) dot = cfmac(p1, vb[r1], dot);
-        if (own2) dot = cfmac(p2, vb[r2], dot);
-        dot.x = warp_sum(dot.x);
-        dot.y = warp_sum(dot.y);
-        const C a2 = cscale(cmul(f.tau, dot), R(-0.5));
-        if (own1) wb[r1] = cfma(a2, vb[r1], p1);        // (tau = 0: p = 0, w = 0)
-        if (own2) wb[r2] = cfma(a2, vb[r2], p2);
-        __syncwarp();
-        const C* vq[1] = {vb};
-        const C* wq[1] = {wb};
-        warp_her2_rows<R, 1>(c0, m, vq, wq);
-        __syncwarp();
-    }
-    for (int i = lane; i < n; i += 32) d[i] = P[pk(i, n)].x;
-    if (lane == 0 && n >= 1) e[n - 1] = R(0);
-    __syncwarp();
-}
 
 }  // namespace sbg

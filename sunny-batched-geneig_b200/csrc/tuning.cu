@@ -48,7 +48,6 @@ bool fits(int n, int precision, const Schedule& s) {
     if (reduce_dmma_smem_bytes(n) > lim || back_dmma_smem_bytes(n) > lim) return false;
     if (ql_chain_smem_bytes(n, s.chain_threads) > lim) return false;
     if (ql_apply_smem_bytes(n, s.ql_warps) > lim) return false;
-    if (n <= 65 && pair_kernels_smem_bytes(n, s.pair_warps) > lim) return false;
     if (precision == SBG_PRECISION_MIXED &&
         (n > kMixedMaxN || refine_c_smem_bytes(n) > lim || mixed_fallback_smem_bytes(n) > lim ||
          hetrd_c64_smem_bytes(n) > lim))
@@ -223,7 +222,7 @@ struct Bench {
     bool mixed() const { return precision == SBG_PRECISION_MIXED; }
     void reduce(const Schedule& s) { launch_reduce(kReduceFull, a(), b(), n, count, ws, x(), inf(), s.shape(), st); }
     void tridiag(const Schedule& s) {
-        if (mixed()) launch_hetrd_c64(n, count, x(), ws, inf(), s.shape(), st);
+        if (mixed()) launch_hetrd_c64(n, count, x(), ws, inf(), st);
         else launch_hetrd(n, count, x(), ws, inf(), st);
     }
     void eig(const Schedule& s) {
@@ -266,11 +265,9 @@ bool sweep(int n, int precision, const TuneRequest& req, Schedule& best, double&
     cudaMemcpy(bench.A.p, hA.data(), 16 * bench.nn * count, cudaMemcpyHostToDevice);
     cudaMemcpy(bench.B.p, hB.data(), 16 * bench.nn * count, cudaMemcpyHostToDevice);
     const Schedule base = default_schedule(n, precision);
-    // pairs per CTA of the warp-per-pair kernels (the reference's batches per block, its BPB
-    // sweep over {16, 8, 4, 2, 1}); here at most 4 warps share a CTA
+    // pair_warps (the reference's batches per block) and ql_warps shape no kernel: kept as asked or built in
     const std::vector<int> bpb_opts = req.force_bpb && n <= 65 ? std::vector<int>{req.force_bpb}
-                                      : n <= 65 ? std::vector<int>{1, 2, 4} : std::vector<int>{base.pair_warps};
-    // ql_warps shapes no kernel (the eigenvectors come from inverse iteration): kept as asked or built in
+                                                               : std::vector<int>{base.pair_warps};
     const std::vector<int> warp_opts = req.force_bpb && n > 65 ? std::vector<int>{req.force_bpb}
                                                                : std::vector<int>{base.ql_warps};
     Schedule win = base;

@@ -23,8 +23,8 @@ namespace sbg {
 struct Schedule {
     int hetrd_threads = 256;    // what block_dim_x reports and force_block_dim_x sets (128 or 256); no kernel's
                                 // CTA size depends on it
-    int pair_warps = 2;         // pairs (warps) per CTA of k_hetrd_warp_c64 (mixed form, n <= 63); what
-                                // batches_per_block reports and sets for n <= 65
+    int pair_warps = 2;         // 1, 2 or 4: what batches_per_block reports and sets for n <= 65; no kernel's
+                                // shape depends on it
     int col_exact = 1;          // 0 or 1, kept from earlier tables: no kernel depends on it
     int back_lanes = 1;         // 1 or 2, kept from earlier tables: no kernel depends on it
     int back_qpass = 1;         // 1 or 2, likewise
@@ -34,7 +34,6 @@ struct Schedule {
     int chain_threads = 128;    // pairs (threads) per CTA of the QL scalar-chain kernel (n > 63, flagged pairs)
     LaunchShape shape() const {
         LaunchShape l;
-        l.pair_warps = pair_warps;
         l.reduce_tc = reduce_tc;
         return l;
     }
