@@ -209,7 +209,11 @@ __global__ void __launch_bounds__(128) k_tridiag_values(int n, int batch, Worksp
     // (regula falsi with Anderson & Bjorck's reduction of an end that stays): 14 to 23 counts in all for the
     // slowest eigenvalue of a warp where halving takes 49.  The counts alone decide which end moves; a step
     // that is too close to an end is moved off it by that spacing, so that the other end follows, and a
-    // cell that three steps did not halve is halved (two: 28 to 32 counts; never: up to 60).
+    // cell that three steps did not halve is halved (two: 28 to 32 counts).  Where det(T - x I) nearly
+    // vanishes at an end (another eigenvalue just outside the cell), every chord lands there and that end alone
+    // creeps: the step after such a step halves (T = tridiag(1, h |i - c|, 1), n = 40 .. 128: 88 counts at most
+    // instead of 151).  Any four steps halve a cell, whatever the chords do, and the widest grid cell (n <= 2,
+    // 12 / 33 of the scaled norm) is 52 halvings from its last width: 208 steps, so the limit is never met.
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     End lo[NE], hi[NE];
     double wa[NE], wb[NE], wc[NE];                                // its width one, two and three steps ago
@@ -231,7 +235,7 @@ __global__ void __launch_bounds__(128) k_tridiag_values(int n, int batch, Worksp
         side[s] = 0;
         open[s] = j < n;
     }
-    for (int step = 0; step < 128; ++step) {
+    for (int step = 0; step < 256; ++step) {
         bool any = false;
 #pragma unroll
         for (int s = 0; s < NE; ++s) {
@@ -260,6 +264,8 @@ __global__ void __launch_bounds__(128) k_tridiag_values(int n, int batch, Worksp
             End& moved = up ? lo[s] : hi[s];
             End& stays = up ? hi[s] : lo[s];
             const int way = up ? -1 : 1;
+            // (2.3e-16: the spacing a step is held off an end by, 1.1e-16 max(1, 2 |x|), or a little more)
+            if (fabs(x[s] - moved.x) <= 2.3e-16 * fmax(1.0, fabs(x[s]))) wc[s] = 0.0;
             if (side[s] == way) {
                 const double m = 1.0 - fabs(px[s] / moved.p) * pow2_clamped(ex[s] - moved.e);
                 stays.p *= m > 0.0 ? m : 0.5;                     // (also where the end had no value)
