@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(128) k_tridiag_values(int n, int batch, Worksp
             End& moved = up ? lo[s] : hi[s];
             End& stays = up ? hi[s] : lo[s];
             const int way = up ? -1 : 1;
-            // (2.3e-16: the spacing a step is held off an end by, 1.1e-16 max(1, 2 |x|), or a little more)
-            if (fabs(x[s] - moved.x) <= 2.3e-16 * fmax(1.0, fabs(x[s]))) wc[s] = 0.0;
+            // (its own end moved by less than 2^-51: about the spacing that a step is held off an end by)
+            if ((__double2hiint(x[s] - moved.x) & 0x7fffffff) < (1023 - 51) << 20) wc[s] = 0.0;
             if (side[s] == way) {
                 const double m = 1.0 - fabs(px[s] / moved.p) * pow2_clamped(ex[s] - moved.e);
                 stays.p *= m > 0.0 ? m : 0.5;                     // (also where the end had no value)
