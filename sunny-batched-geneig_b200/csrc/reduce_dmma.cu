@@ -173,7 +173,12 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_reduce_dmma(int mode, const d
         double2* I8 = Li + K * kBlk;
         if (mode != kReduceFromLM) {
             for (int e = lane; e < 64; e += 32)
-                if ((e & 7) >= (e >> 3)) D[(e & 7) + kBlkLd * (e >> 3)] = I8[(e & 7) + kBlkLd * (e >> 3)];
+                if ((e & 7) > (e >> 3)) D[(e & 7) + kBlkLd * (e >> 3)] = I8[(e & 7) + kBlkLd * (e >> 3)];
+            if (lane < 8) {
+                // (the root of an infinite pivot came out as NaN, 0 inf; its column below is zero: the row drops out)
+                const double root = I8[10 * lane].x;
+                D[10 * lane] = make_double2(root == root ? root : __longlong_as_double(0x7ff0000000000000ll), 0.0);
+            }
             __syncwarp();
         }
         if (lane < 8) {                                           // lane j: column j of the inverse
