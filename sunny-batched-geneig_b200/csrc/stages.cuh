@@ -147,7 +147,7 @@ __device__ __forceinline__ R pow2_norm(R anorm) {
 // limits; scaling always keeps the single-precision variant safe).
 // Eigenvalues come back ascending with Z's columns permuted alike (dsteqr's
 // final selection sort).  Returns the number of off-diagonals that had not
-// converged after 30 n iterations (0 on success).
+// converged after 30 n iterations (0 on success; n - 1, with NaN in d and Z, for a T that is not finite).
 // d, e live in shared memory private to the warp; only lane 0 writes them.
 template <typename R>
 __device__ int tridiag_ql(int n, R* d, R* e, R* Z, int ldz) {
@@ -157,8 +157,18 @@ __device__ int tridiag_ql(int n, R* d, R* e, R* Z, int ldz) {
     const R safmin = sizeof(R) == 8 ? R(2.2250738585072014e-308) : R(1.17549435e-38);
     // scale to max-norm in [1/2, 1)
     R anorm = R(0);
-    for (int i = 0; i < n; ++i) anorm = fmax(anorm, fabs(d[i]));
-    for (int i = 0; i + 1 < n; ++i) anorm = fmax(anorm, fabs(e[i]));
+    bool finite = true;
+    for (int i = 0; i < n; ++i) { anorm = fmax(anorm, fabs(d[i])); finite = finite && isfinite(d[i]); }
+    for (int i = 0; i + 1 < n; ++i) { anorm = fmax(anorm, fabs(e[i])); finite = finite && isfinite(e[i]); }
+    if (!finite) {                                           // uniform: no sweep would converge
+        const R nan = static_cast<R>(__longlong_as_double(0x7ff8000000000000ll));
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) d[i] = nan;
+        for (int row = lane; row < n; row += 32)
+            for (int k = 0; k < n; ++k) Z[row * ldz + k] = nan;
+        __syncwarp();
+        return n - 1;
+    }
     anorm = pow2_norm(anorm);
     const R sc = R(1) / anorm;
     __syncwarp();
@@ -257,7 +267,8 @@ __device__ int tridiag_ql(int n, R* d, R* e, R* Z, int ldz) {
 // top = -1 ends the log.  The eigenvalues are sorted ascending and perm[k]
 // receives the pre-sort column index of eigenvalue k.
 // Returns the number of unconverged off-diagonals, or -1 if the log capacity
-// (cap entries) would be exceeded (the caller then falls back to tridiag_ql).
+// (cap entries) would be exceeded (the caller then falls back to tridiag_ql).  A T that is not finite
+// gives n - 1, NaN in W and a log that turns Z to NaN.
 // LOG = false: eigenvalues only (no log, no permutation; log, cap and perm are ignored).
 template <typename R, bool LOG = true>
 __device__ int ql_chain(int n, R* d, R* e, int stride, cplx<R>* log, int cap, int* perm, double* W) {
@@ -268,8 +279,24 @@ __device__ int ql_chain(int n, R* d, R* e, int stride, cplx<R>* log, int cap, in
 #define D(i) d[(i) * stride]
 #define E(i) e[(i) * stride]
     R anorm = R(0);
-    for (int i = 0; i < n; ++i) anorm = fmax(anorm, fabs(D(i)));
-    for (int i = 0; i + 1 < n; ++i) anorm = fmax(anorm, fabs(E(i)));
+    bool finite = true;
+    for (int i = 0; i < n; ++i) { anorm = fmax(anorm, fabs(D(i))); finite = finite && isfinite(D(i)); }
+    for (int i = 0; i + 1 < n; ++i) { anorm = fmax(anorm, fabs(E(i))); finite = finite && isfinite(E(i)); }
+    if (!finite) {                                           // no sweep would converge: one of NaN instead
+        const R nan = static_cast<R>(__longlong_as_double(0x7ff8000000000000ll));
+        for (int k = 0; k < n; ++k) W[k] = nan;
+        if constexpr (LOG) {
+            if (n + 1 > cap) return -1;
+            for (int k = 0; k < n; ++k) perm[k] = k;
+            int pos = 0;
+            if (n > 1) {
+                log[pos++] = mk<R>(R(n - 2), R(n - 1));
+                for (int k = 0; k + 1 < n; ++k) log[pos++] = mk<R>(nan, nan);
+            }
+            log[pos] = mk<R>(R(-1), R(0));
+        }
+        return n - 1;
+    }
     anorm = pow2_norm(anorm);
     const R sc = R(1) / anorm;
     for (int i = 0; i < n; ++i) D(i) *= sc;
