@@ -1136,14 +1136,14 @@ size_t big_stage_smem_bytes(int n, bool tc, int chain_threads) {
 }
 
 cudaError_t launch_ql_rows(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
-                           int chain_threads, cudaStream_t stream) {
+                           const double2* C, int chain_threads, cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (!W || !X || !info || !ws.d || !ws.e || !ws.log || !ws.perm || !ws.flag) return cudaErrorInvalidValue;
     const size_t cs = ql_chain_smem_bytes(n, chain_threads), as = ql_rows_smem_bytes(n);
     if (cs > static_cast<size_t>(max_smem_optin()) || as > static_cast<size_t>(max_smem_optin()))
         return cudaErrorInvalidValue;
     // inverse iteration for every pair it can take, then the rotation-log QL for the pairs it flagged
-    cudaError_t err = launch_eig_invit(n, batch, ws, W, X, info, true, stream);
+    cudaError_t err = launch_eig_invit(n, batch, ws, W, X, info, C, true, stream);
     if (err == cudaSuccess) err = launch_ql_chain(n, batch, ws, W, info, chain_threads, stream);
     if (err != cudaSuccess) return err;
     static SmemOptIn fd;

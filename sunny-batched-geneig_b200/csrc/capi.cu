@@ -404,7 +404,7 @@ void geneig_reduce_eig_n54_launch(const cuDoubleComplex* d_H, const cuDoubleComp
         check_cuda(sbg::launch_reduce(sbg::kReduceFull, c2(d_H), c2(d_S), 54, 1, ws, c2(d_V), d_info,
                                       s->sched.shape(), stream), "reduce kernel");
         check_cuda(sbg::launch_hetrd(54, 1, c2(d_V), ws, d_info, stream), "hetrd kernel");
-        check_cuda(sbg::launch_eig(54, 1, ws, d_W, c2(d_V), d_info, s->sched.chain_threads, stream), "eigensolve kernels");
+        check_cuda(sbg::launch_eig(54, 1, ws, d_W, c2(d_V), d_info, c2(d_V), s->sched.chain_threads, stream), "eigensolve kernels");
         check_cuda(sbg::launch_back(sbg::kBackQOnly, 54, 1, ws, c2(d_V), d_info, s->sched.shape(), stream),
                    "back kernel");
     }));
@@ -441,7 +441,7 @@ void geneig_finish_n54_launch(const cuDoubleComplex* d_L, const cuDoubleComplex*
             check_cuda(sbg::launch_hetrd(54, cnt, c2(d_M) + nn * off, ws, d_info + off, stream),
                        "hetrd kernel");
             check_cuda(sbg::launch_eig(54, cnt, ws, d_W + 54 * off, c2(d_U) + nn * off, d_info + off,
-                                       s->sched.chain_threads, stream), "eigensolve kernels");
+                                       c2(d_M) + nn * off, s->sched.chain_threads, stream), "eigensolve kernels");
             check_cuda(sbg::launch_back(sbg::kBackFull, 54, cnt, ws, c2(d_U) + nn * off, d_info + off,
                                         s->sched.shape(), stream), "back kernel");
         }

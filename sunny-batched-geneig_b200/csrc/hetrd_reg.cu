@@ -100,6 +100,8 @@ __device__ __forceinline__ void form_reflector(int c, int RS, int la, const doub
     s2 = warp_sum(s2);
     // beta = -sign(Re alpha) ||(alpha, x)||, tau = (beta - alpha) / beta, scale = 1 / (alpha - beta);
     // H = I for a zero tail and a real alpha.  The norm is n2 rsqrt(n2) after one Newton step.
+    // (An n2 or a reciprocal outside the normal range gives NaN, or a norm of 2^510 and more: k_tridiag_values sees
+    // either in d and e and has the pair formed again, scaled.)
     const bool id = s2 == 0.0 && alpha.y == 0.0;
     const double n2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, s2));
     const double rn = rsqrt(n2);

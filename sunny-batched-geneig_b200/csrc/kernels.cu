@@ -543,24 +543,24 @@ cudaError_t launch_ql_chain(int n, int batch, const Workspace& ws, double* W, in
 }
 
 cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
-                             bool flag_redo, cudaStream_t stream) {
+                             const double2* C, bool flag_redo, cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (!W || !X || !info || !ws.d || !ws.e || !ws.flag) return cudaErrorInvalidValue;
     const size_t is = InvitSmem(n, !flag_redo).per_warp;
     if (is > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
     static SmemOptIn fi;
     set_max_smem_once(k_tridiag_invit, fi);
-    const cudaError_t err = launch_tridiag_values(n, batch, ws, W, info, stream);
+    const cudaError_t err = launch_tridiag_values(n, batch, ws, W, info, C, stream);
     if (err != cudaSuccess) return err;
     k_tridiag_invit<<<batch, 32, is, stream>>>(n, batch, ws, W, X, info, flag_redo ? 1 : 0);
     return launch_tridiag_ortho(n, batch, ws, W, X, info, !flag_redo, stream);
 }
 
-cudaError_t launch_eig(int n, int batch, const Workspace& ws, double* W, double2* X, int* info, int chain_threads,
-                       cudaStream_t stream) {
+cudaError_t launch_eig(int n, int batch, const Workspace& ws, double* W, double2* X, int* info, const double2* C,
+                       int chain_threads, cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
-    if (n > kInvitQlMaxN) return launch_ql_rows(n, batch, ws, W, X, info, chain_threads, stream);
-    return launch_eig_invit(n, batch, ws, W, X, info, false, stream);
+    if (n > kInvitQlMaxN) return launch_ql_rows(n, batch, ws, W, X, info, C, chain_threads, stream);
+    return launch_eig_invit(n, batch, ws, W, X, info, C, false, stream);
 }
 
 // ----------------------------------------------------------------------------- k_pull_pairs

@@ -146,8 +146,15 @@ size_t hetrd_reg_smem_bytes(int n);      // dynamic shared memory of its CTA
 cudaError_t launch_hetrd_reg(int n, int batch, const double2* C, const Workspace& ws, const int* info,
                              cudaStream_t stream);
 // Eigenvalues W and eigenvectors Z (real, in X) of every pair's tridiagonal (see the eigensolve below).
-cudaError_t launch_eig(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
+// C: the matrix the FP64 Householder ran on (lower triangle; it may be X), for the pairs it has to be done again
+// for (csrc/tridiag.cu, hetrd_scaled; the rotation-log region is its scratch), or null.
+cudaError_t launch_eig(int n, int batch, const Workspace& ws, double* W, double2* X, int* info, const double2* C,
                        int chain_threads, cudaStream_t stream);
+// launch_eig's C after launch_reduce and launch_hetrd on X: k_reduce_mid and k_reduce_big leave none there (and
+// need none, their reflectors divide).
+inline const double2* reduced_matrix(int n, const LaunchShape& shape, const double2* X) {
+    return n <= 84 || shape.reduce_tc ? X : nullptr;
+}
 // Mixed form (n <= kMixedMaxN), after the FP64 reduction left C in X:
 //   launch_hetrd_c64     complex64 Householder (csrc/hetrd_reg.cu); FP64-promoted reflectors, tau (made
 //                        unitary in FP64) and T into the workspace, C into the pair's stash;
@@ -247,7 +254,7 @@ cudaError_t launch_refine_big(int n, int batch, const Workspace& ws, double* W, 
 size_t hetrd_c64_big_smem_bytes(int n);
 size_t refine_big_smem_bytes();
 cudaError_t launch_ql_rows(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
-                           int chain_threads, cudaStream_t stream);
+                           const double2* C, int chain_threads, cudaStream_t stream);
 cudaError_t launch_back_big(int mode, int n, int batch, const Workspace& ws, double2* X, const int* info,
                             cudaStream_t stream);
 // The QL scalar chain (thread per pair) of the pairs with ws.flag == kFlagRedo: W, the rotation log, perm;
@@ -276,7 +283,8 @@ inline int eig_kernel_count(int n, bool single) {
 }
 // Eigenvalues of every pair's tridiagonal (d, e) by bisection (csrc/tridiag.cu), ascending; NaN for
 // pairs with info != 0.  Honours the pair selection.
-cudaError_t launch_tridiag_values(int n, int batch, const Workspace& ws, double* W, int* info, cudaStream_t stream);
+cudaError_t launch_tridiag_values(int n, int batch, const Workspace& ws, double* W, int* info, const double2* C,
+                                  cudaStream_t stream);
 // Orthonormalises Z of the pairs with ws.flag == kFlagOrtho (csrc/tridiag.cu); with_ql: the warp QL for those
 // it cannot, otherwise they get kFlagRedo.  Honours the pair selection.
 cudaError_t launch_tridiag_ortho(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
@@ -285,7 +293,7 @@ size_t tridiag_ortho_smem_bytes(int n, bool with_ql);
 // The three kernels above for every pair; flag_redo: pairs they cannot take get ws.flag = kFlagRedo
 // (and no vectors) instead of the in-kernel QL.
 cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
-                             bool flag_redo, cudaStream_t stream);
+                             const double2* C, bool flag_redo, cudaStream_t stream);
 
 size_t reduce_dmma_smem_bytes(int n);
 size_t ql_chain_smem_bytes(int n, int threads);

@@ -98,7 +98,7 @@ extern "C" int sbg_geneig_full_noalloc_launch(int n, const cuDoubleComplex* d_A,
     e = sbg::launch_reduce(sbg::kReduceFull, A, B, n, batch, ws, X, d_info, sch.shape(), stream);
     if (e == cudaSuccess) e = sbg::launch_hetrd(n, batch, X, ws, d_info, stream);
     if (e == cudaSuccess)
-        e = sbg::launch_eig(n, batch, ws, d_W, X, d_info, sch.chain_threads, stream);
+        e = sbg::launch_eig(n, batch, ws, d_W, X, d_info, sbg::reduced_matrix(n, sch.shape(), X), sch.chain_threads, stream);
     if (e == cudaSuccess) e = sbg::launch_back(sbg::kBackFull, n, batch, ws, X, d_info, sch.shape(), stream);
     if (e != cudaSuccess) return fail(SBG_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     return SBG_OK;

@@ -564,7 +564,7 @@ cudaError_t launch_refine_mixed(int n, int batch, const Workspace& ws, double* W
 
 cudaError_t launch_eig_mixed(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                              int refine_steps, const LaunchShape& shape, cudaStream_t stream) {
-    cudaError_t err = launch_eig_invit(n, batch, ws, W, X, info, false, stream);
+    cudaError_t err = launch_eig_invit(n, batch, ws, W, X, info, nullptr, false, stream);
     if (err == cudaSuccess) err = launch_back(kBackQOnly, n, batch, ws, X, info, shape, stream);
     if (err == cudaSuccess) err = launch_refine_mixed(n, batch, ws, W, X, info, refine_steps, stream);
     return err;

@@ -230,7 +230,7 @@ struct sbg_solver {
         check_cuda(sbg::launch_hetrd_c64_big(n, cnt, X, ws, info, stream), "complex64 hetrd kernel");
         stage_end(stream, ev, 1, 1);
         stage_begin(stream, &ev);
-        check_cuda(sbg::launch_eig(n, cnt, ws, W, X, info, sched.chain_threads, stream),
+        check_cuda(sbg::launch_eig(n, cnt, ws, W, X, info, nullptr, sched.chain_threads, stream),
                    "eigensolve kernels");
         check_cuda(sbg::launch_back(sbg::kBackQOnly, n, cnt, ws, X, info, sched.shape(), stream), "Q-apply kernel");
         check_cuda(sbg::launch_refine_big(n, cnt, ws, W, X, info, refine_steps, stream), "refinement kernel");
@@ -245,7 +245,8 @@ struct sbg_solver {
         check_cuda(sbg::launch_reduce(sbg::kReduceFull, A, B, n, cnt, sel, X, info, sched.shape(), stream),
                    "reduce kernel (FP64 redo)");
         check_cuda(sbg::launch_hetrd(n, cnt, X, sel, info, stream), "hetrd kernel (FP64 redo)");
-        check_cuda(sbg::launch_eig(n, cnt, sel, W, X, info, sched.chain_threads, stream),
+        check_cuda(sbg::launch_eig(n, cnt, sel, W, X, info, sbg::reduced_matrix(n, sched.shape(), X), sched.chain_threads,
+                                   stream),
                    "eigensolve kernels (FP64 redo)");
         check_cuda(sbg::launch_back(sbg::kBackFull, n, cnt, sel, X, info, sched.shape(), stream),
                    "back-transform kernel (FP64 redo)");
@@ -279,7 +280,8 @@ struct sbg_solver {
                                              stream),
                        "mixed eigensolve kernels");
         else
-            check_cuda(sbg::launch_eig(n, cnt, ws, W, X, info, sched.chain_threads, stream), "eigensolve kernels");
+            check_cuda(sbg::launch_eig(n, cnt, ws, W, X, info, sbg::reduced_matrix(n, sched.shape(), X), sched.chain_threads,
+                                       stream), "eigensolve kernels");
         stage_end(stream, ev, 2, sbg::eig_kernel_count(n, mixed));
         stage_begin(stream, &ev);
         check_cuda(sbg::launch_back(mixed ? sbg::kBackLOnly : sbg::kBackFull, n, cnt, ws, X, info, sched.shape(),

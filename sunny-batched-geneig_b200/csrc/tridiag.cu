@@ -104,11 +104,115 @@ __device__ __forceinline__ double pow2_clamped(int k) {
     return __hiloint2double((min(max(k, -1000), 1000) + 1023) << 20, 0);
 }
 
+// The sum of x over the CTA, in every thread (red: a slot per warp).
+__device__ __forceinline__ double block_sum(double x, double* red) {
+    x = warp_sum(x);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+    __syncthreads();
+    x = 0.0;
+    for (int w = 0; w < static_cast<int>(blockDim.x) >> 5; ++w) x += red[w];
+    __syncthreads();
+    return x;
+}
+
+// The FP64 Householder again, by this CTA, for a pair with a column whose squared norm left the normal range: one of
+// norm below 1.5e-154 comes out of k_hetrd_reg and k_hetrd_tri as NaN, one above 3e153 can come out wrong.  LAPACK's zlarfg
+// rescales such a column as it meets it; a test for it there, never true, made every step's chain longer (the
+// kernel 3 % slower at n = 54, 10 % at 24 and 32, 20 % at 40), while here it is part of a norm that is
+// formed anyway.  C (lower triangle) times a power of two, its largest entry in [1, 2), goes to S (n x n, full); a column
+// that is below 2^-450 then is taken as zero.  zhetd2's steps, each a pass over S in L2: milliseconds at n = 128.
+// v, w: n entries of shared memory each.  Loops stay rolled, for the registers of
+// the kernel.  Nothing is written if C is not finite.
+__device__ __noinline__ void hetrd_scaled(int n, const double2* C, double2* S, double2* v, double2* w, double* red,
+                                          double* d, double* e, double2* tau, double2* LV, bool lv_cols) {
+    const int tid = threadIdx.x, T = blockDim.x;
+    int most = 0;                                                 // high word of the largest |part| of C's triangle
+#pragma unroll 1
+    for (int j = 0; j < n; ++j)
+#pragma unroll 1
+        for (int i = j + (tid & 31); i < n; i += 32) {            // (every warp all of it)
+            const double2 z = C[i + static_cast<size_t>(j) * n];
+            most = max(most, max(__double2hiint(z.x) & 0x7fffffff, i == j ? 0 : __double2hiint(z.y) & 0x7fffffff));
+        }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (most >= 0x7ff00000) return;                               // uniform
+    const int hi = min(max(0x7fe00000 - (most & 0x7ff00000), 0x00100000), 0x7fd00000);
+    const double by = __hiloint2double(hi, 0), back = __hiloint2double(0x7fe00000 - hi, 0);
+#pragma unroll 1
+    for (int idx = tid; idx < n * n; idx += T) {
+        const int j = idx / n, i = idx - j * n;
+        double2 z = cscale(C[max(i, j) + static_cast<size_t>(min(i, j)) * n], by);
+        if (i <= j) z.y = i < j ? -z.y : 0.0;
+        S[idx] = z;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k + 1 < n; ++k) {
+        const double2* ck = S + static_cast<size_t>(k) * n;
+        const double2 alpha = ck[k + 1];
+        double s2 = 0.0;
+#pragma unroll 1
+        for (int i = k + 2 + tid; i < n; i += T) s2 += cabs2(ck[i]);
+        s2 = fma(alpha.y, alpha.y, block_sum(s2, red));
+        const bool id = s2 <= 0x1p-900;                           // uniform
+        const double nrm = sqrt(fma(alpha.x, alpha.x, s2)), beta = alpha.x >= 0.0 ? -nrm : nrm;
+        const double ar = alpha.x - beta, den = fma(ar, ar, alpha.y * alpha.y);
+        const double2 zero = make_double2(0.0, 0.0);
+        const double2 tk = id ? zero : make_double2((beta - alpha.x) / beta, -alpha.y / beta);
+        const double2 scale = id ? zero : make_double2(ar / den, -alpha.y / den);
+        if (tid == 0) {
+            d[k] = ck[k].x * back;
+            e[k] = (id ? alpha.x : beta) * back;
+            tau[k] = tk;
+        }
+#pragma unroll 1
+        for (int i = k + 1 + tid; i < n; i += T) {
+            v[i] = i == k + 1 ? make_double2(1.0, 0.0) : id ? zero : cmul(ck[i], scale);
+            if (lv_cols) LV[(i - k - 1) + static_cast<size_t>(n - 1 - k) * n] = v[i];
+            else LV[k + static_cast<size_t>(i) * n] = v[i];
+        }
+        __syncthreads();
+        if (id) continue;
+        // w = p + a2 v, p = tau A22 v, a2 = -|tau|^2 / 2 (v^H A22 v); then A22 -= v w^H + w v^H
+        double vav = 0.0;
+#pragma unroll 1
+        for (int i = k + 1 + tid; i < n; i += T) {
+            double2 sum = zero;
+#pragma unroll 1
+            for (int j = k + 1; j < n; ++j) sum = cfma(S[i + static_cast<size_t>(j) * n], v[j], sum);
+            vav = fma(v[i].x, sum.x, fma(v[i].y, sum.y, vav));
+            w[i] = cmul(tk, sum);
+        }
+        const double a2 = -0.5 * cabs2(tk) * block_sum(vav, red);
+#pragma unroll 1
+        for (int i = k + 1 + tid; i < n; i += T) w[i] = make_double2(fma(a2, v[i].x, w[i].x), fma(a2, v[i].y, w[i].y));
+        __syncthreads();
+#pragma unroll 1
+        for (int i = k + 1 + tid; i < n; i += T)
+#pragma unroll 1
+            for (int j = k + 1; j < n; ++j) {
+                double2 z = cfmsc(w[i], v[j], cfmsc(v[i], w[j], S[i + static_cast<size_t>(j) * n]));
+                if (i == j) z.y = 0.0;
+                S[i + static_cast<size_t>(j) * n] = z;
+            }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        d[n - 1] = S[static_cast<size_t>(n) * n - 1].x * back;
+        e[n - 1] = 0.0;
+        tau[n - 1] = make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+}
+
 // One pair per CTA of ceil(n / (32 NE)) warps; thread t holds the eigenvalues of index t + T s.
-// A T that is not finite goes through the QL recurrence (one thread), whose info code it gets.
+// A T that is not finite, or so large that a reflector may have been wrong, is formed again from C (where there is
+// one) by hetrd_scaled and goes through the QL recurrence (one thread), whose info code it gets.
+// (At most 72 registers for NE = 1, one warp: hetrd_scaled alone would take 80, and 28 pairs fit an SM as 25.)
 template <int NE>
-__global__ void __launch_bounds__(128) k_tridiag_values(int n, int batch, Workspace ws, double* __restrict__ W,
-                                                        int* __restrict__ info) {
+__global__ void __launch_bounds__(NE == 1 ? 32 : 128, NE == 1 ? 28 : 4)
+    k_tridiag_values(int n, int batch, Workspace ws, double* __restrict__ W, int* __restrict__ info,
+                     const double2* __restrict__ C) {
     const int b = blockIdx.x;
     if (b >= batch || !pair_selected(ws, b)) return;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -157,8 +261,14 @@ __global__ void __launch_bounds__(128) k_tridiag_values(int n, int batch, Worksp
     } else {
         finite = __all_sync(0xffffffffu, finite);
     }
-    if (!finite) {                                                // uniform
+    if (!finite || amax >= 0x1p508) {                             // uniform
         double* d = reinterpret_cast<double*>(smem + lay.de);     // 2 rows doubles: d, then e
+        if (C) {
+            const size_t nn = static_cast<size_t>(n) * n, at = static_cast<size_t>(n) * b;
+            double2* v = reinterpret_cast<double2*>(smem);        // (de, lam, p, cnt: 40 n bytes)
+            hetrd_scaled(n, C + nn * b, static_cast<double2*>(ws.log) + static_cast<size_t>(ws.log_stride) * b, v, v + n,
+                         red, ws.d + at, ws.e + at, ws.tau + at, ws.LV + nn * b, n > kSmallMaxN);
+        }
         double* e = d + rows;
         for (int i = tid; i < n; i += T) { d[i] = dg[i]; e[i] = eg[i]; }
         __syncthreads();
@@ -461,18 +571,21 @@ __global__ void __launch_bounds__(kOrthoThreads) k_tridiag_ortho(int n, int batc
 }
 
 template <int NE>
-cudaError_t run_values(int n, int batch, const Workspace& ws, double* W, int* info, cudaStream_t stream) {
+cudaError_t run_values(int n, int batch, const Workspace& ws, double* W, int* info, const double2* C,
+                       cudaStream_t stream) {
     const int T = 32 * ((n + 32 * NE - 1) / (32 * NE));
-    k_tridiag_values<NE><<<batch, T, ValuesSmem(n, T * NE).total, stream>>>(n, batch, ws, W, info);
+    k_tridiag_values<NE><<<batch, T, ValuesSmem(n, T * NE).total, stream>>>(n, batch, ws, W, info, C);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_tridiag_values(int n, int batch, const Workspace& ws, double* W, int* info, cudaStream_t stream) {
+cudaError_t launch_tridiag_values(int n, int batch, const Workspace& ws, double* W, int* info, const double2* C,
+                                  cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (n < 1 || n > kBigMaxN || !W || !info || !ws.d || !ws.e) return cudaErrorInvalidValue;
-    return n <= 32 ? run_values<1>(n, batch, ws, W, info, stream) : run_values<2>(n, batch, ws, W, info, stream);
+    if (C && (!ws.LV || !ws.tau || !ws.log || ws.log_stride < n * n)) return cudaErrorInvalidValue;
+    return n <= 32 ? run_values<1>(n, batch, ws, W, info, C, stream) : run_values<2>(n, batch, ws, W, info, C, stream);
 }
 
 cudaError_t launch_tridiag_ortho(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,

@@ -229,7 +229,7 @@ struct Bench {
         if (mixed())
             launch_eig_mixed(n, count, ws, w(), x(), inf(), 5, s.shape(), st);
         else
-            launch_eig(n, count, ws, w(), x(), inf(), s.chain_threads, st);
+            launch_eig(n, count, ws, w(), x(), inf(), nullptr, s.chain_threads, st);
     }
     void back(const Schedule& s) {
         launch_back(mixed() ? kBackLOnly : kBackFull, n, count, ws, x(), inf(), s.shape(), st);
