@@ -4,12 +4,10 @@
 // and picks the block size by probing cuSolverDx or by a timing sweep
 // (src/nvrtc/nvrtc_solver.cpp:205-240, 649-925, 1021-1042), caching the cubin in
 // process and on disk (:392-597).  Here every kernel is compiled ahead of time for
-// sm_100a; a schedule is the launch shape of each stage: pairs per CTA of the warp-per-pair
-// kernels (the reference's batches per block), which column-kernel instantiation and how many
-// lanes per column, CTA sizes of the CTA-per-pair and QL kernels.  Suggested mode uses a
-// built-in table; autotune mode times each stage's candidates on a synthetic batch,
-// validates the winning combination (every pair's info, eigenvalues against the built-in
-// schedule's, host residuals of sampled columns), and memoises it in process and in a
+// sm_100a and takes its CTA from n, so that of a schedule's eight fields two shape a launch: reduce_tc, and
+// chain_threads for the pairs that inverse iteration gives up.  Suggested mode uses a built-in table;
+// autotune mode times the stages on a synthetic batch, validates the schedule (every pair's info,
+// eigenvalues against the built-in schedule's, host residuals of sampled columns), and memoises it in process and in a
 // versioned, checksummed table file (atomic write-then-rename; a corrupt or foreign file is
 // ignored and rewritten).
 #pragma once
