@@ -487,6 +487,11 @@ cudaError_t launch_back_stream(int mode, int n, int batch, const Workspace& ws, 
     return cudaErrorInvalidValue;
 }
 
+size_t back_stream_smem_bytes(int n) {
+    const size_t nt = static_cast<size_t>((n <= 112 ? 112 : (n + 15) / 16 * 16) / 8);      // as the cases above
+    return 16 * kBlk * (2 * nt + 2 * nt);
+}
+
 size_t back_dmma_smem_bytes(int n) {
     const size_t nt = static_cast<size_t>((n + 7) / 8);
     return 16 * (8 * nt * (8 * nt + 1) + 2 * kBlk * nt + 8 * nt);

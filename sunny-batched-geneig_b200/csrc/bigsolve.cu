@@ -1127,12 +1127,14 @@ cudaError_t launch_hetrd_c64_big(int n, int batch, const double2* C, const Works
 
 size_t ql_rows_smem_bytes(int n) { return ql_rows_bytes(n); }
 
-size_t big_stage_smem_bytes(int n, bool tc, int chain_threads) {
-    size_t m = std::max(ql_rows_smem_bytes(n), ql_chain_smem_bytes(n, chain_threads));
-    m = std::max(m, std::max(invit_smem_bytes(n, false), tridiag_ortho_smem_bytes(n, false)));
-    if (tc) return std::max(m, n <= kHetrdRegMaxN ? hetrd_reg_smem_bytes(n) : hetrd_tri_smem_bytes(n));
-    // k_reduce_tc / k_back_*_tc: static only
-    return std::max(m, std::max(big_reduce_smem_bytes(n), BigBackSmem(n).total));
+size_t stage_smem_bytes(int n, bool tc, int chain_threads) {
+    const size_t m = eig_smem_bytes(n, chain_threads);
+    if (n > kSmallMaxN && !tc) return std::max(m, std::max(big_reduce_smem_bytes(n), BigBackSmem(n).total));
+    // (k_reduce_tc, k_back_q_tc and k_back_tc: static only)
+    const size_t reduce = n <= kReduceDmmaMaxN ? reduce_dmma_smem_bytes(n) : 0;
+    const size_t hetrd = n <= kHetrdRegMaxN ? hetrd_reg_smem_bytes(n) : hetrd_tri_smem_bytes(n);
+    const size_t back = n <= kBackDmmaMaxN ? back_dmma_smem_bytes(n) : n <= kBackStreamMaxN ? back_stream_smem_bytes(n) : 0;
+    return std::max(std::max(m, reduce), std::max(hetrd, back));
 }
 
 cudaError_t launch_ql_rows(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,

@@ -46,7 +46,6 @@ int supported_max_n(int precision) {
         }
         size_t need = std::max(sbg::reduce_dmma_smem_bytes(n), sbg::back_dmma_smem_bytes(n));
         need = std::max(need, sbg::hetrd_reg_smem_bytes(n));
-        need = std::max(need, sbg::ql_apply_smem_bytes(n, 1));
         need = std::max(need, sbg::ql_chain_smem_bytes(n, 32));
         if (big_mixed) {
             need = std::max(need, sbg::hetrd_c64_big_smem_bytes(n));
@@ -328,11 +327,12 @@ int sbg_solver_batches_per_block(const sbg_solver* s) {
 int sbg_solver_block_dim_x(const sbg_solver* s) { return s ? s->sched.hetrd_threads : 0; }
 unsigned int sbg_solver_shared_mem_bytes(const sbg_solver* s) {
     if (!s) return 0;
-    size_t m = s->n > sbg::kSmallMaxN
-                   ? sbg::big_stage_smem_bytes(s->n, s->sched.reduce_tc != 0, s->sched.chain_threads)
-                   : std::max(sbg::reduce_dmma_smem_bytes(s->n), sbg::back_dmma_smem_bytes(s->n));
+    size_t m = sbg::stage_smem_bytes(s->n, s->sched.reduce_tc != 0, s->sched.chain_threads);
     if (sbg::mixed_big(s->n, s->precision == SBG_PRECISION_MIXED))
         m = std::max(m, std::max(sbg::hetrd_c64_big_smem_bytes(s->n), sbg::refine_big_smem_bytes()));
+    else if (s->precision == SBG_PRECISION_MIXED)
+        m = std::max(m, std::max(sbg::hetrd_c64_smem_bytes(s->n),
+                                 std::max(sbg::refine_c_smem_bytes(s->n), sbg::mixed_fallback_smem_bytes(s->n))));
     return static_cast<unsigned>(m);
 }
 int sbg_solver_was_autotuned(const sbg_solver* s) { return s ? s->autotuned : 0; }
@@ -370,7 +370,8 @@ void geneig_full_n54_batched_launch(const cuDoubleComplex* d_H, const cuDoubleCo
 }
 unsigned int geneig_full_n54_batched_block_dim_x(void) { return sbg::default_schedule(54, SBG_PRECISION_FP64).hetrd_threads; }
 unsigned int geneig_full_n54_batched_shared_mem_bytes(void) {
-    return static_cast<unsigned>(std::max(sbg::reduce_dmma_smem_bytes(54), sbg::back_dmma_smem_bytes(54)));
+    const sbg::Schedule c = sbg::default_schedule(54, SBG_PRECISION_FP64);
+    return static_cast<unsigned>(sbg::stage_smem_bytes(54, c.reduce_tc != 0, c.chain_threads));
 }
 
 void chol_n54_launch(const cuDoubleComplex* d_S, cuDoubleComplex* d_L, int* d_info, cudaStream_t stream) {
@@ -413,7 +414,7 @@ unsigned int geneig_reduce_eig_n54_block_dim_x(void) { return sbg::default_sched
 unsigned int geneig_reduce_eig_n54_shared_mem_bytes(void) { return geneig_full_n54_batched_shared_mem_bytes(); }
 unsigned int geneig_reduce_eig_n54_chol_smem_bytes(void) { return static_cast<unsigned>(sbg::reduce_dmma_smem_bytes(54)); }
 unsigned int geneig_reduce_eig_n54_heev_smem_bytes(void) {
-    return static_cast<unsigned>(sbg::ql_apply_smem_bytes(54, sbg::default_schedule(54, SBG_PRECISION_FP64).ql_warps));
+    return static_cast<unsigned>(sbg::eig_smem_bytes(54, sbg::default_schedule(54, SBG_PRECISION_FP64).chain_threads));
 }
 unsigned int geneig_reduce_eig_n54_heev_workspace(void) {
     return static_cast<unsigned>(sbg::workspace_bytes_per_pair(54) / 16);

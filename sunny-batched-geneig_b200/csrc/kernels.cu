@@ -524,10 +524,16 @@ cudaError_t launch_hetrd(int n, int batch, const double2* C, const Workspace& ws
 }
 
 size_t ql_chain_smem_bytes(int n, int threads) { return 8 * 2 * static_cast<size_t>(n) * threads; }
-size_t ql_apply_smem_bytes(int n, int pairs_per_cta) {
+size_t ql_warps_bound_bytes(int n, int pairs_per_cta) {
     const size_t rows = (static_cast<size_t>(n) + 31) / 32;
     return (align_up(8 * static_cast<size_t>(n) * tile_ld(n), 16) + rows * 2 * 32 * 16 + align_up(16 * static_cast<size_t>(n), 16)) *
            pairs_per_cta;
+}
+
+size_t eig_smem_bytes(int n, int chain_threads) {
+    const bool ql_here = n <= kInvitQlMaxN;
+    const size_t m = std::max(tridiag_values_smem_bytes(n), std::max(invit_smem_bytes(n, ql_here), tridiag_ortho_smem_bytes(n, ql_here)));
+    return ql_here ? m : std::max(m, std::max(ql_chain_smem_bytes(n, chain_threads), ql_rows_smem_bytes(n)));
 }
 
 cudaError_t launch_ql_chain(int n, int batch, const Workspace& ws, double* W, int* info, int chain_threads,

@@ -207,9 +207,10 @@ constexpr int kBigMaxN = 256;
 bool big_path(int n);
 size_t big_reduce_smem_bytes(int n);
 size_t ql_rows_smem_bytes(int n);
-// Largest dynamic shared memory per CTA among the FP64 kernels a solve of order n > kSmallMaxN
-// launches: tc = the schedule's reduce_tc, chain_threads its QL chain width.
-size_t big_stage_smem_bytes(int n, bool tc, int chain_threads);
+// Largest dynamic shared memory per CTA among the FP64 kernels that a solve of order n launches, and among its
+// eigensolve's: tc = the schedule's reduce_tc, chain_threads its QL chain width.
+size_t stage_smem_bytes(int n, bool tc, int chain_threads);
+size_t eig_smem_bytes(int n, int chain_threads);
 // mode: kBigFull (Cholesky, reduction, Householder: k_reduce_mid / k_reduce_big), kBigHegstOnly (the
 // same kernels, stopping after C = L^{-1} A L^{-H}: C's lower triangle in X, L in LV) or kBigHetrdOnly
 // (the Householder alone by k_hetrd_reg or k_hetrd_tri, from C's lower triangle in X with L already in LV, as
@@ -290,6 +291,7 @@ cudaError_t launch_tridiag_values(int n, int batch, const Workspace& ws, double*
 cudaError_t launch_tridiag_ortho(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
                                  bool with_ql, cudaStream_t stream);
 size_t tridiag_ortho_smem_bytes(int n, bool with_ql);
+size_t tridiag_values_smem_bytes(int n);
 // The three kernels above for every pair; flag_redo: pairs they cannot take get ws.flag = kFlagRedo
 // (and no vectors) instead of the in-kernel QL.
 cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
@@ -297,9 +299,11 @@ cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, d
 
 size_t reduce_dmma_smem_bytes(int n);
 size_t ql_chain_smem_bytes(int n, int threads);
-// The bound on ql_warps (pairs per CTA): each pair's Z tile, log stage and T in shared memory.
-size_t ql_apply_smem_bytes(int n, int pairs_per_cta);
+// What the schedule's ql_warps (pairs per CTA) is held against, so that a value that was refused stays refused: the Z tile,
+// log stage and T of each pair in the kernel that it used to shape.  No kernel has this size.
+size_t ql_warps_bound_bytes(int n, int pairs_per_cta);
 size_t back_dmma_smem_bytes(int n);
+size_t back_stream_smem_bytes(int n);
 size_t invit_smem_bytes(int n, bool with_tile);
 // r[i] = recip_nr(u[i]) for i < count (device self-test of the inverse iteration's reciprocal).
 cudaError_t launch_selftest_recip(const double* u, double* r, int count, cudaStream_t stream);

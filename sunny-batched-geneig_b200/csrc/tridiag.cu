@@ -600,6 +600,11 @@ cudaError_t launch_tridiag_ortho(int n, int batch, const Workspace& ws, double* 
     return cudaGetLastError();
 }
 
+size_t tridiag_values_smem_bytes(int n) {
+    const int NE = n <= 32 ? 1 : 2;
+    return ValuesSmem(n, 32 * ((n + 32 * NE - 1) / (32 * NE)) * NE).total;
+}
+
 size_t tridiag_ortho_smem_bytes(int n, bool with_ql) { return OrthoSmem(n, with_ql).total; }
 
 }  // namespace sbg

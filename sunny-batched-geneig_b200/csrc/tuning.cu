@@ -47,7 +47,7 @@ bool fits(int n, int precision, const Schedule& s) {
     }
     if (reduce_dmma_smem_bytes(n) > lim || back_dmma_smem_bytes(n) > lim) return false;
     if (ql_chain_smem_bytes(n, s.chain_threads) > lim) return false;
-    if (ql_apply_smem_bytes(n, s.ql_warps) > lim) return false;
+    if (ql_warps_bound_bytes(n, s.ql_warps) > lim) return false;
     if (precision == SBG_PRECISION_MIXED &&
         (n > kMixedMaxN || refine_c_smem_bytes(n) > lim || mixed_fallback_smem_bytes(n) > lim ||
          hetrd_c64_smem_bytes(n) > lim))
