@@ -16,8 +16,8 @@
 // Bound by the tensor pipe and its latency: the products alone take 20.4 K cycles per pair and SM at
 // n = 54 (NT = 7), the kernel 33 K.  It replaced a thread per column (n <= 56: one 16-byte broadcast per
 // complex FMA, FP64 pipe 29 % busy), 4 or 8 lanes per column (57 .. 84) and, for 85 .. 96, tile products
-// through L2.  Microseconds per 1,000 pairs before -> now: n = 24 22 -> 14, 32 29 -> 24, 47 178 -> 71, 54
-// 174 -> 113, 64 472 -> 143, 72 1,286 -> 257, 96 1,441 -> 517; 8 pairs of n = 54: 87 -> 30 us.
+// through L2.  Microseconds per 1,000 pairs before -> now: n = 24 22 -> 12, 32 29 -> 22, 47 178 -> 67, 54
+// 174 -> 108, 64 472 -> 140, 72 1,286 -> 237, 96 1,441 -> 454; 8 pairs of n = 54: 87 -> 30 us.
 #include "kernels.cuh"
 #include "stages.cuh"
 #include "tiles.cuh"
@@ -450,8 +450,9 @@ cudaError_t launch_back_dmma(int mode, int n, int batch, const Workspace& ws, do
     if (batch <= 0) return cudaSuccess;
     if (n < 1 || n > kBackDmmaMaxN || !X || !info || !ws.LV || !ws.tau) return cudaErrorInvalidValue;
 #define SBG_CASE(NT, MINB) case NT: return run_back_dmma<NT, MINB>(mode, n, batch, ws, X, info, stream)
-    // (column tiles = warps, CTAs per SM): as many CTAs as the columns' registers allow without spills that
-    // cost more (n = 72: 338 us per 1,000 pairs with one CTA, 257 with two and 176 bytes spilled)
+    // (column tiles = warps, CTAs per SM): as many CTAs as shared memory and the columns' registers allow; for nine
+    // tiles two are worth 964 bytes of spill stores a thread (n = 72: 271 us per 1,000 pairs with one CTA and none, 237
+    // with two)
     switch ((n + 7) / 8) {
         SBG_CASE(1, 16);
         SBG_CASE(2, 16);

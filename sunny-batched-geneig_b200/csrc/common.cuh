@@ -25,10 +25,6 @@ template <typename C, typename R> __device__ __forceinline__ C cscale(C a, R s) 
 template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
     C r; r.x = a.x * b.x - a.y * b.y; r.y = a.x * b.y + a.y * b.x; return r;
 }
-// conj(a) * b
-template <typename C> __device__ __forceinline__ C cmulc(C a, C b) {
-    C r; r.x = a.x * b.x + a.y * b.y; r.y = a.x * b.y - a.y * b.x; return r;
-}
 // acc + a * b
 template <typename C> __device__ __forceinline__ C cfma(C a, C b, C acc) {
     acc.x = fma(a.x, b.x, acc.x); acc.x = fma(-a.y, b.y, acc.x);
@@ -66,10 +62,6 @@ template <typename C> __device__ __forceinline__ C cshfl(C v, int src, int width
 template <typename R> __device__ __forceinline__ R warp_sum(R v) {
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) v += shfl_xor(v, m);
-    return v;
-}
-template <typename R> __device__ __forceinline__ R group_sum(R v, int width) {
-    for (int m = width >> 1; m >= 1; m >>= 1) v += shfl_xor(v, m, width);
     return v;
 }
 

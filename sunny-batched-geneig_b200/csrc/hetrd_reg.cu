@@ -174,7 +174,6 @@ __device__ __forceinline__ void form_reflector(int c, int RS, int la, const floa
 
 // One case per column slot: a sweep over the live slots q0 .. NS - 1 jumps into the sequence once
 // and falls through.  The columns of slot q0 that are dead already meet v = w = 0.
-#define SBG_ASC16(C) C(0) C(1) C(2) C(3) C(4) C(5) C(6) C(7) C(8) C(9) C(10) C(11) C(12) C(13) C(14) C(15)
 #define SBG_ASC32(C) C(0) C(1) C(2) C(3) C(4) C(5) C(6) C(7) C(8) C(9) C(10) C(11) C(12) C(13) C(14) C(15) \
     C(16) C(17) C(18) C(19) C(20) C(21) C(22) C(23) C(24) C(25) C(26) C(27) C(28) C(29) C(30) C(31)
 
@@ -453,7 +452,8 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_hetrd_reg(int n, int batch, c
 // neighbouring shapes, microseconds per 1,000 pairs: few warps and many pairs per SM win (n = 48: 1 warp 113, 2
 // 122; n = 54: 2 warps 141, 1 warp 170, and in an earlier form 3 warps 185, 4 227, 8 327) until a
 // pair's columns no longer fit beside others in shared memory; fewer register slots than these make the
-// shared-memory part the bound (n = 54: 8 slots 162, 10 147, 12 141).
+// shared-memory part the bound (n = 54: 8 slots 162, 10 147, 12 141).  A block of 4 where it measured better (n = 32: 33.2
+// with 2, 30.6 with 4), 2 elsewhere.  Above n = 128 nine slots of five rows spill 740 bytes a thread (stores).
 #define SBG_HETRD_REG_BY_N(n, F)                                                       \
     do {                                                                               \
         if ((n) <= 24) F(1, 1, 8, 24, 2);                                              \

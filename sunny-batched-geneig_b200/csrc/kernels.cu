@@ -377,7 +377,6 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(int n, int batch, Workspac
     }
 }
 
-// Pairs (warps) per CTA of the warp-per-pair kernels: 1, 2 or 4 (anything else: the default 2).
 template <class K>
 void set_max_smem_once(K kernel, SmemOptIn& rec) {
     set_smem_limit(reinterpret_cast<const void*>(kernel), rec, max_smem_optin());

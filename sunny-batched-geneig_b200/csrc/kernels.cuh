@@ -18,8 +18,8 @@ namespace sbg {
 // which the back-transform kernel then overwrites with X in place.
 //   log  cap entries (16 B)  the QL rotation log of the pair (ql_chain)
 //   perm n int               sort permutation of the QL eigenvalues
-//   flag 1 int               1 if the log overflowed (the apply kernel then runs the
-//                            warp-per-pair QL for that pair)
+//   flag 1 int               what k_tridiag_invit made of the pair (kFlagDone, kFlagRedo, kFlagOrtho), or 3: the
+//                            log overflowed, and the apply kernel runs the warp QL for the pair
 struct Workspace {
     double2* LV = nullptr;
     double2* tau = nullptr;
@@ -275,7 +275,7 @@ inline int back_kernel_count(int n, bool tc) { return n > kBackStreamMaxN && tc 
 // through the QL: in those kernels, one warp, for n <= kInvitQlMaxN; above it by the rotation-log QL
 // (k_ql_chain + k_ql_apply_rows), which runs for the flagged pairs alone.
 constexpr int kInvitQlMaxN = 63;
-// Workspace::flag of a pair after k_tridiag_invit (1 and 3 are the rotation log's overflow marks).
+// Workspace::flag of a pair after k_tridiag_invit (k_ql_chain sets 3 where the rotation log overflows).
 constexpr int kFlagDone = 0, kFlagRedo = 2, kFlagOrtho = 4;
 // Kernels one eigensolve stage launches for order n.
 inline int eig_kernel_count(int n, bool single) {

@@ -35,7 +35,9 @@ struct ReduceDmmaSmem {
     static constexpr size_t l = 0;
     static constexpr size_t linv = l + 16 * static_cast<size_t>(kBlk) * (NT * (NT + 1) / 2);
     static constexpr size_t flag = linv + 16 * static_cast<size_t>(kBlk) * NT;
-    // W, (r, c) at r + kLdw c, where two CTAs still fit an SM with it
+    // W, (r, c) at r + kLdw c, where as many CTAs fit an SM with it as without (MINB below).  n = 49 .. 56, two CTAs
+    // either way: 104 us per 1,000 pairs at n = 49 against 128 through the output buffer; 41 .. 48, three instead
+    // of four: 76 against 71 at n = 47.
     static constexpr int kLdw = 8 * NT + 1;
     static constexpr bool kW = NT <= 7 && NT != 6;
     static constexpr size_t wt = flag + 16;
@@ -295,7 +297,8 @@ cudaError_t launch_reduce_dmma(int mode, const double2* A, const double2* B, int
     if (n > 56 && mode != kReduceChol && mode != kReduceFromLM &&
         (!ws.log || static_cast<size_t>(ws.log_stride) < static_cast<size_t>(n) * n))
         return cudaErrorInvalidValue;
-    // (column tiles, warps, CTAs per SM): a warp per tile up to 56; above, fewer warps with two or more tiles
+    // (column tiles, warps, CTAs per SM): as many CTAs as shared memory leaves room for, some registers spilled for it
+    // (stores up to 224 bytes a thread, 692 for 18 tiles).  A warp per tile up to 56; above, fewer warps with two or more tiles
     // each and more CTAs, so that other pairs' solves run beside a pair's Cholesky (n = 64: 8 warps x 2 CTAs
     // 161 us per 1,000 pairs, 4 x 4 136; n = 72: 5 x 2 255, 5 x 3 215, 9 x 1 343)
 #define SBG_CASE(NT, NW, MINB) case NT: return run_reduce_dmma<NT, NW, MINB>(mode, A, B, n, batch, ws, out, info, stream)

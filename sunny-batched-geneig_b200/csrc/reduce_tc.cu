@@ -1,6 +1,7 @@
-// Blocked FP64 Cholesky and two-sided reduction on the FP64 tensor cores, one CTA (4 warps) per
-// pair, for n > kSmallMaxN, where the scalar kernels that hold a pair's triangle in shared memory
-// (k_reduce_mid) or spread it over a cluster (k_reduce_big) run at a few percent of the FP64 peak.
+// Blocked FP64 Cholesky and two-sided reduction on the FP64 tensor cores, one CTA (4 warps) per pair, for
+// n > kReduceDmmaMaxN, and the back-transform for n > kBackStreamMaxN, where a pair's matrices no longer
+// fit an SM; the scalar kernels for such n (k_reduce_big, k_back_big, a cluster per pair) run at a few percent of the
+// FP64 peak.
 //
 //   k_reduce_tc   B = L L^H, W = L^{-1} A, C = L^{-1} W^H (= L^{-1} A L^{-H}), in 32 x 32 blocks:
 //                   Cholesky, left-looking: T(:, K) = B(:, K) - L(:, <K) L(K, <K)^H (tile products),
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_reduce_tc(const double2* A,
     if (tid == 0) info[b] = 0;
 }
 
-// X = L^{-H} Y in place over the X buffer (Y complex there), one CTA per pair, for n > kSmallMaxN:
+// X = L^{-H} Y in place over the X buffer (Y complex there), one CTA per pair:
 // the backward substitution by blocks of 32, from the last block row up,
 //   T(I, :) = Y(I, :) - L(>I, I)^H X(>I, :),   X(I, :) = L(I, I)^{-H} T(I, :),
 // every product a tile product on the FP64 tensor cores; the diagonal blocks of L (LV's lower
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_back_tc(int n, int batch, W
     }
 }
 
-// Y = Q Z for n > kSmallMaxN (Z real in the X buffer, Y complex over it), Q = H_0 H_1 ... H_{n-2}
+// Y = Q Z (Z real in the X buffer, Y complex over it), Q = H_0 H_1 ... H_{n-2}
 // from the reflectors the big-n Householder stores (v_k(k+1+s) = LV(s, n-1-k), v_k(k+1) = 1) and
 // tau: blocks of 32 reflectors in compact WY form, Q_blk = I - V T V^H with T upper triangular
 // (LAPACK zlarft, forward, columnwise: T(i, i) = tau_i, T(0:i, i) = -tau_i T(0:i, 0:i) V^H v_i),

@@ -90,8 +90,8 @@ def _check_pair_buffers(n, A, B, W, X, info):
 class Solver:
     """Runtime-n solver handle (mirrors NvrtcGeneigSolver, src/nvrtc/nvrtc_solver.hpp:81-217).
 
-    batches_per_block: pairs per CTA of the QL stage (0 = auto).
-    block_dim: threads per CTA of the CTA-per-pair stages, 128 or 256 (0 = auto).
+    batches_per_block: 1, 2 or 4 up to n = 65, 1 .. 16 above (0 = auto); checked, kept and reported, no kernel's shape.
+    block_dim: 128 or 256 (0 = auto); likewise.
     tuning: "suggested" (built-in schedule) or "autotune" (measured, persisted).
     cache: "auto" | "no_disk" | "none" (the autotune table's layers).
     precision: "fp64" (the plain drop-in) or "mixed" (complex64 tridiagonalisation and FP64
