@@ -9,7 +9,8 @@
 //   eig      k_tridiag_values (tridiag.cu: bisection on Sturm counts), k_tridiag_invit
 //            (eigenvectors by inverse iteration, one warp per pair) and k_tridiag_ortho
 //            (tridiag.cu: pairs with large clusters); k_ql_chain + k_ql_apply_rows (n > 63) or a
-//            warp QL inside those kernels for the pairs they cannot take.  The mixed form refines
+//            warp QL inside those kernels for the pairs they cannot take; n <= 4 k_tridiag_tiny, the
+//            warp QL alone.  The mixed form refines
 //            Y = Q Z against C afterwards (refine.cu).
 //   back     k_back_dmma (back_dmma.cu): X = L^{-H} Q Z, written over Z (the mixed form:
 //            Y = Q Z, then X = L^{-H} Y after the refinement).
@@ -551,6 +552,7 @@ cudaError_t launch_eig_invit(int n, int batch, const Workspace& ws, double* W, d
                              const double2* C, bool flag_redo, cudaStream_t stream) {
     if (batch <= 0) return cudaSuccess;
     if (!W || !X || !info || !ws.d || !ws.e || !ws.flag) return cudaErrorInvalidValue;
+    if (n <= kTridiagTinyMaxN) return launch_tridiag_tiny(n, batch, ws, W, X, info, C, stream);
     const size_t is = InvitSmem(n, !flag_redo).per_warp;
     if (is > static_cast<size_t>(max_smem_optin())) return cudaErrorInvalidValue;
     static SmemOptIn fi;

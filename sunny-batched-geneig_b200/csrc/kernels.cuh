@@ -277,10 +277,15 @@ inline int back_kernel_count(int n, bool tc) { return n > kBackStreamMaxN && tc 
 constexpr int kInvitQlMaxN = 63;
 // Workspace::flag of a pair after k_tridiag_invit (k_ql_chain sets 3 where the rotation log overflows).
 constexpr int kFlagDone = 0, kFlagRedo = 2, kFlagOrtho = 4;
+// The whole eigensolve of so small an n is one kernel (csrc/tridiag.cu); honours the pair selection.
+constexpr int kTridiagTinyMaxN = 4;
+cudaError_t launch_tridiag_tiny(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
+                                const double2* C, cudaStream_t stream);
 // Kernels one eigensolve stage launches for order n.
 inline int eig_kernel_count(int n, bool single) {
-    if (single) return 6;          // k_tridiag_values, _invit, _ortho, Q-apply, refinement, fallback
-    return n <= kInvitQlMaxN ? 3 : 5;
+    const int t = n <= kTridiagTinyMaxN ? 1 : 3;       // k_tridiag_tiny, or k_tridiag_values, _invit, _ortho
+    if (single) return t + 3;                          // Q-apply, refinement, fallback
+    return n <= kInvitQlMaxN ? t : t + 2;
 }
 // Eigenvalues of every pair's tridiagonal (d, e) by bisection (csrc/tridiag.cu), ascending; NaN for
 // pairs with info != 0.  Honours the pair selection.

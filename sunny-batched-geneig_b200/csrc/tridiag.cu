@@ -570,6 +570,48 @@ __global__ void __launch_bounds__(kOrthoThreads) k_tridiag_ortho(int n, int batc
     if (lane == 0) info[b] = unconv;
 }
 
+// ----------------------------------------------------------------------------- k_tridiag_tiny
+// n <= kTridiagTinyMaxN: eigenvalues and eigenvectors by the warp QL, Z row-major in shared memory; one launch,
+// where bisection, inverse iteration and k_tridiag_ortho are three that cost more than their work.  The
+// eigensolve of 65,536 pairs, those three -> this, in us: n = 1 145 -> 41, 2 281 -> 76, 3 298 -> 154, 4 315 -> 240, 5
+// 338 -> 344, 6 355 -> 463; of one pair 13 -> 6, 19 -> 8, 19 -> 10, 19 -> 14, 19 -> 18, 19 -> 23.
+__global__ void __launch_bounds__(32) k_tridiag_tiny(int n, int batch, Workspace ws, double* __restrict__ W,
+                                                     double2* __restrict__ X, int* __restrict__ info,
+                                                     const double2* __restrict__ C) {
+    const int b = blockIdx.x, lane = threadIdx.x;
+    if (b >= batch || !pair_selected(ws, b)) return;
+    __shared__ __align__(16) double2 vw[2 * kTridiagTinyMaxN];
+    __shared__ double z[kTridiagTinyMaxN * (kTridiagTinyMaxN + 1)], d[kTridiagTinyMaxN], e[kTridiagTinyMaxN], red[1];
+    const size_t nn = static_cast<size_t>(n) * n, at = static_cast<size_t>(n) * b;
+    if (lane == 0) ws.flag[b] = kFlagDone;
+    if (info[b] != 0) {                                           // uniform
+        if (lane < n) W[at + lane] = __longlong_as_double(0x7ff8000000000000ll);
+        return;
+    }
+    double x = lane < n ? ws.d[at + lane] : 0.0, y = lane + 1 < n ? ws.e[at + lane] : 0.0;
+    if (C && __any_sync(0xffffffffu, !(fabs(x) < 0x1p508 && fabs(y) < 0x1p508))) {
+        hetrd_scaled(n, C + nn * b, static_cast<double2*>(ws.log) + static_cast<size_t>(ws.log_stride) * b, vw, vw + n, red,
+                     ws.d + at, ws.e + at, ws.tau + at, ws.LV + nn * b, false);
+        x = lane < n ? ws.d[at + lane] : 0.0;
+        y = lane + 1 < n ? ws.e[at + lane] : 0.0;
+    }
+    const int ld = n + 1;
+    if (lane < n) {
+        d[lane] = x;
+        e[lane] = y;
+        for (int c = 0; c < n; ++c) z[lane * ld + c] = lane == c ? 1.0 : 0.0;
+    }
+    __syncwarp();
+    const int unconv = tridiag_ql<double>(n, d, e, z, ld);
+    __syncwarp();
+    if (lane < n) {
+        double* Z = reinterpret_cast<double*>(X + nn * b);
+        W[at + lane] = d[lane];
+        for (int k = 0; k < n; ++k) Z[lane + k * n] = z[lane * ld + k];
+    }
+    if (lane == 0 && unconv) info[b] = unconv;
+}
+
 template <int NE>
 cudaError_t run_values(int n, int batch, const Workspace& ws, double* W, int* info, const double2* C,
                        cudaStream_t stream) {
@@ -586,6 +628,15 @@ cudaError_t launch_tridiag_values(int n, int batch, const Workspace& ws, double*
     if (n < 1 || n > kBigMaxN || !W || !info || !ws.d || !ws.e) return cudaErrorInvalidValue;
     if (C && (!ws.LV || !ws.tau || !ws.log || ws.log_stride < n * n)) return cudaErrorInvalidValue;
     return n <= 32 ? run_values<1>(n, batch, ws, W, info, C, stream) : run_values<2>(n, batch, ws, W, info, C, stream);
+}
+
+cudaError_t launch_tridiag_tiny(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
+                                const double2* C, cudaStream_t stream) {
+    if (batch <= 0) return cudaSuccess;
+    if (n < 1 || n > kTridiagTinyMaxN || !W || !X || !info || !ws.d || !ws.e || !ws.flag) return cudaErrorInvalidValue;
+    if (C && (!ws.LV || !ws.tau || !ws.log || ws.log_stride < n * n)) return cudaErrorInvalidValue;
+    k_tridiag_tiny<<<batch, 32, 0, stream>>>(n, batch, ws, W, X, info, C);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_tridiag_ortho(int n, int batch, const Workspace& ws, double* W, double2* X, int* info,
