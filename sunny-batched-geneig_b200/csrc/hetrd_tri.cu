@@ -12,8 +12,8 @@
 // With the whole triangle in L2 (3 CTAs per SM, 444 triangles of 295 KB at n = 192: more than L2 holds)
 // the walks were bound by that traffic, 2.6 TB/s: 14.4 us per pair at n = 192.  The last 154
 // columns of n = 192 take part in all but 2 % of it.  Now 8.6 us per pair; 83 % of a step is the walk,
-// ~1,450 cycles per two columns where the FP64 pipe needs 440: issue and the latency of two columns' chains
-// with two warps per scheduler.  us per 1,000 pairs before -> now: n = 160 7,500 -> 5,600, 192 14,400 -> 8,600.
+// ~1,450 cycles per two columns where the FP64 pipe needs 440: the latency of two columns' chains, of the step's
+// barriers and of shared memory with two warps per scheduler (issue slots 30 % used, FP64 pipe 18 %).  us per 1,000 pairs before -> now: n = 160 7,500 -> 5,600, 192 14,400 -> 8,600.
 #include "kernels.cuh"
 #include "stages.cuh"
 
