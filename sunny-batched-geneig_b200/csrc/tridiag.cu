@@ -321,8 +321,8 @@ __global__ void __launch_bounds__(NE == 1 ? 32 : 128, NE == 1 ? 28 : 4)
     // that is too close to an end is moved off it by that spacing, so that the other end follows, and a
     // cell that three steps did not halve is halved (two: 28 to 32 counts).  Where det(T - x I) nearly
     // vanishes at an end (another eigenvalue just outside the cell), every chord lands there and that end alone
-    // creeps: the step after such a step halves (T = tridiag(1, h |i - c|, 1), n = 40 .. 128: 88 counts at most
-    // instead of 151).  Any four steps halve a cell, whatever the chords do, and the widest grid cell (n <= 2,
+    // creeps: the step after such a step halves (T = tridiag(1, h |i - c|, 1), n = 40 .. 128: 87 counts at most
+    // instead of 151).  Any four steps halve a cell, whatever the chords do, and the widest grid cell (n <= 32,
     // 12 / 33 of the scaled norm) is 52 halvings from its last width: 208 steps, so the limit is never met.
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     End lo[NE], hi[NE];
